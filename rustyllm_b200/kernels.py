@@ -68,6 +68,9 @@ _SIGNATURES = {
                                _c_void_p, _c_void_p],
     "rl_rope_kv_write": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p,
                          _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
+    "rl_attention_f32_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "rl_attention_f32": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
+                         _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_int, _c_float, _c_int, _c_void_p, _c_int, _c_void_p],
     "rl_attention_simt": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p,
                           _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
                           _c_void_p],
@@ -632,7 +635,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
                    num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
                    value_dim: Optional[int] = None, sink: bool = False, gate: Optional[torch.Tensor] = None,
                    softcap: float = 0.0, keep_first: int = 0, chunk: int = 0, values_in_keys: bool = False,
-                   gate_per_head: bool = False, sinks: Optional[torch.Tensor] = None) -> None:
+                   gate_per_head: bool = False, sinks: Optional[torch.Tensor] = None, single_tokens: bool = False) -> None:
     """q: [M, >= H*hd] (a view into the qkv buffer is fine), out: [M, H*vd] where vd is
     ``value_dim`` (default: head_dim), the width of a value head.  ``sink``: the softmax's
     denominator has one more term of score 0 (and no value).  ``gate`` [M, H*vd] (a view is
@@ -641,7 +644,8 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     [0, keep_first) stay visible after the window has passed them.  ``chunk`` > 0 (instead of a window): a query at
     position p sees positions [p - p % chunk, p].  ``values_in_keys``: the values are the first ``value_dim`` elements
     of the key rows (``v_pool`` is not read).  ``gate_per_head``: ``gate`` is [M, H], one number a head.  ``sinks`` (float32
-    [H]): the extra term of the denominator has the score sinks[h] instead of 0."""
+    [H]): the extra term of the denominator has the score sinks[h] instead of 0.  ``single_tokens``: every sequence of the
+    step brings one token (a 32-bit step's launch shape follows it, not its result)."""
     vd = head_dim if value_dim is None else value_dim
     if values_in_keys:
         assert vd <= head_dim
@@ -657,6 +661,17 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
         _need(gate, "gate", q.dtype, contiguous=False)
         assert gate.shape == (M, num_heads if gate_per_head else num_heads * vd) and gate.stride(1) == 1
         ldg = gate.stride(0) if M > 1 else gate.shape[1]
+    if (q.dtype == torch.float32 and vd == head_dim and not (window or chunk or values_in_keys)
+            and library().rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, out.stride(0), q.data_ptr(), out.data_ptr())):
+        # 32-bit heads of 64 or 128 that see every position: tiles of rows that share a key (csrc/attention_f32.cu; 500 tokens of
+        # 32 heads of 64: 101 us against 914 with the any-shape kernel; four single tokens behind 96 to 700: 15.6 against 151)
+        _check(library().rl_attention_f32(
+            q.data_ptr(), ldq, k_pool.data_ptr(), v_pool.data_ptr(), page_table.data_ptr(), page_table.shape[1],
+            slot_of_token.data_ptr(), positions.data_ptr(), out.data_ptr(), out.stride(0), M, num_heads, num_kv_heads, head_dim,
+            float(scale), int(bool(sink)), _ptr(gate), ldg, float(softcap or 0.0), int(bool(gate_per_head)), _sinks(sinks, num_heads),
+            int(bool(single_tokens)), _stream()), "rl_attention_f32")
+        _count()
+        return
     _check(library().rl_attention_simt_shaped(
         q.data_ptr(), ldq, k_pool.data_ptr(), v_pool.data_ptr(), _dt(q), page_table.data_ptr(),
         page_table.shape[1], slot_of_token.data_ptr(), positions.data_ptr(), out.data_ptr(), out.stride(0),
@@ -1918,7 +1933,7 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_
         attention_simt(q, k_pool, v_pool, page_table, step.slot_of_token, step.positions, out,
                        num_heads, num_kv_heads, head_dim, scale, window, value_dim=value_dim, sink=sink, gate=gate,
                        softcap=softcap, keep_first=keep_first, chunk=chunk, values_in_keys=values_in_keys,
-                       gate_per_head=gate_per_head, sinks=sinks)
+                       gate_per_head=gate_per_head, sinks=sinks, single_tokens=step.is_decode)
         return
     # the decode kernel and its plans take a chunked mask as a negative window
     dec_window = -int(chunk) if chunk else int(window)
@@ -1931,7 +1946,7 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_
         # any-shape kernel, the decode kernel and the tcgen05 prompt kernel have them (the mma.sync prompt kernel does not)
         attention_simt(q, k_pool, v_pool, page_table, step.slot_of_token, step.positions, out,
                        num_heads, num_kv_heads, head_dim, scale, window, value_dim=value_dim, sink=sink, gate=gate,
-                       softcap=softcap, keep_first=keep_first, chunk=chunk, sinks=sinks)
+                       softcap=softcap, keep_first=keep_first, chunk=chunk, sinks=sinks, single_tokens=step.is_decode)
         return
     if decode_ok:
         splits = decode_splits(q.shape[0], num_kv_heads)
@@ -1980,7 +1995,7 @@ def attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_
                           step.q_lens, out, num_heads, num_kv_heads, head_dim, scale, window, sink=sink, gate=gate)
         return
     attention_simt(q, k_pool, v_pool, page_table, step.slot_of_token, step.positions, out,
-                   num_heads, num_kv_heads, head_dim, scale, window, sink=sink, gate=gate, chunk=chunk)
+                   num_heads, num_kv_heads, head_dim, scale, window, sink=sink, gate=gate, chunk=chunk, single_tokens=step.is_decode)
 
 
 from .sampling.config import MAX_TOP_K  # noqa: E402  (one definition, host side)

@@ -1172,3 +1172,50 @@ def test_kernels_refuse_what_they_cannot_do():
                          torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, 2200, device=DEV), 2, 2, 1100, 1.0)
     with pytest.raises(k.KernelError, match="not handled"):
         k.swiglu(torch.zeros(2, 4, dtype=torch.float16, device=DEV), torch.zeros(2, 2, dtype=torch.float16, device=DEV))
+
+
+# ----------------------------------------------------------------------------- 32-bit attention by tiles of rows
+@pytest.mark.parametrize("H,G,hd", [(4, 4, 64), (8, 2, 64), (15, 3, 64), (16, 1, 64), (3, 3, 128), (6, 1, 128), (28, 2, 128)])
+def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
+    """Sequences whose ends fall beside the edges of 32-key chunks and 64-key pages, tiles of rows that several sequences share,
+    and the same rows as single tokens: the float64 result, and bit for bit the same rows whatever shares their tile."""
+    k = K()
+    lens = [1, 31, 32, 33, 3, 64, 65, 300]
+    q, kp, vp, pt, sot, pos, ref = _attention_case(torch.float32, H, G, hd, lens, lens, seed=H + hd)
+    scale = 1.0 / math.sqrt(hd)
+    wide = torch.zeros(q.shape[0], H * hd + 4, device=DEV)          # rows of a wider buffer
+    wide[:, :H * hd] = q
+    out = torch.empty_like(q)
+    k.attention_simt(wide[:, :H * hd], kp, vp, pt, sot, pos, out, H, G, hd, scale)
+    torch.testing.assert_close(out.double().cpu(), ref, rtol=2e-5, atol=2e-5)
+    ends = [sum(lens[:b + 1]) - 1 for b in range(len(lens))]
+    for rows in (ends, [ends[-1] - 7], list(range(ends[-2] + 5, ends[-1] - 50))):
+        some = torch.empty(len(rows), H * hd, device=DEV)
+        k.attention_simt(q[rows].contiguous(), kp, vp, pt, sot[rows].contiguous(), pos[rows].contiguous(), some, H, G, hd, scale,
+                         single_tokens=len(rows) < 20)
+        assert torch.equal(some, out[rows])
+    # what a row may not see cannot reach it: infinities behind position 290 of the longest sequence
+    slot = int(sot[-1])
+    page, at = int(pt[slot, 290 // PAGE]), 290 % PAGE
+    kp[page, :, at:], vp[page, :, at:] = math.inf, math.nan
+    again = torch.empty_like(q)
+    k.attention_simt(q, kp, vp, pt, sot, pos, again, H, G, hd, scale)
+    keep = ends[-1] - (299 - 290)
+    assert torch.equal(again[:keep], out[:keep]) and not torch.isfinite(again[keep:]).any()
+
+
+@pytest.mark.parametrize("H,G,hd", [(8, 2, 64), (6, 1, 128)])
+@pytest.mark.parametrize("options", ["sink", "sinks", "gate", "head gate", "softcap"])
+def test_attention_f32_options_follow_the_any_shape_kernel(H, G, hd, options):
+    """The same call through the any-shape kernel (a chunked mask longer than every sequence is no mask): both are sums of
+    float products, a few units in the last place of values of size 1 apart."""
+    k = K()
+    lens = [40, 1, 130]
+    q, kp, vp, pt, sot, pos, _ = _attention_case(torch.float32, H, G, hd, lens, lens, seed=5)
+    M = q.shape[0]
+    kw = {"sink": dict(sink=True), "sinks": dict(sinks=_rand(H, seed=1)), "gate": dict(gate=_rand(M, H * hd + 3, seed=2)[:, :H * hd]),
+          "head gate": dict(gate=_rand(M, H, seed=3), gate_per_head=True), "softcap": dict(softcap=2.0)}[options]
+    out, plain = torch.empty_like(q), torch.empty_like(q)
+    k.attention_simt(q, kp, vp, pt, sot, pos, out, H, G, hd, 1.0 / math.sqrt(hd), **kw)
+    k.attention_simt(q, kp, vp, pt, sot, pos, plain, H, G, hd, 1.0 / math.sqrt(hd), chunk=1 << 20, **kw)
+    torch.testing.assert_close(out, plain, rtol=1e-5, atol=4e-6)
