@@ -1,10 +1,9 @@
 // out[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) on the CUDA cores, for any M, N, K.
 //
-// This is the matrix product of the true 32-bit path (float inputs, FFMA, float
-// accumulation, no tensor cores and no reduced-precision mode) and the fallback of
-// the bf16 path for shapes the tensor-core kernel refuses (bf16 inputs widened to
-// float, float accumulation).  Both operands are K-major, as every weight of the
-// model is stored ([out x in], out = W x; SimonWaldherr/RustyLLM src/model.rs:185-186).
+// The products of 32-bit runs that gemm_f32_split.cu (many tokens) and the kernel for few tokens do not take - sums
+// shorter than K = 256, few outputs - and the fallback of the bf16 path for shapes the tensor-core kernel refuses (bf16
+// inputs widened to float, float accumulation).  Both operands are K-major, as every weight of the model is stored
+// ([out x in], out = W x; SimonWaldherr/RustyLLM src/model.rs:185-186).
 //
 // Each output element is accumulated over k = 0..K-1 in order, whatever the tile
 // it falls in: the result for one row does not depend on the other rows of the

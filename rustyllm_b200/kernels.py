@@ -42,6 +42,9 @@ _SIGNATURES = {
     "rl_random_fill": [_c_void_p, _c_int, _c_ll, ctypes.c_ulonglong, _c_float, _c_float, _c_void_p],
     "rl_gemm_simt": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                      _c_int, _c_int, _c_void_p],
+    "rl_gemm_f32_split_supported": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int],
+    "rl_gemm_f32_split": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int,
+                          _c_void_p],
     "rl_layer_norm": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_float, _c_void_p],
     "rl_branch_join": [_c_void_p, _c_float, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p, _c_void_p, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_void_p],
@@ -572,8 +575,9 @@ def random_fill(out: torch.Tensor, seed: int, mean: float, std: float) -> None:
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int,
               bias: Optional[torch.Tensor] = None) -> None:
-    """out = a @ w.T (+ bias) on the CUDA cores.  a: [M, K] (rows may be strided),
-    w: [N, K] contiguous, same dtype.  out_mode: OUT_SAME / OUT_F32 / OUT_ADD_F32."""
+    """out = a @ w.T (+ bias) of float or bf16 operands of any shape, float sums, on the CUDA cores; float operands of more
+    than 8 rows by ``gemm_f32_split`` where that takes them.  a: [M, K] (rows may be strided), w: [N, K] contiguous, same
+    dtype.  out_mode: OUT_SAME / OUT_F32 / OUT_ADD_F32."""
     _need(a, "a", contiguous=False); _need(w, "w", a.dtype); _need(out, "out", contiguous=False)
     M, K = a.shape
     N = w.shape[0]
@@ -588,8 +592,26 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int
         assert bias.numel() == N
     lda = a.stride(0) if M > 1 else K
     ldo = out.stride(0) if M > 1 else N
+    if a.dtype == torch.float32 and library().rl_gemm_f32_split_supported(a.data_ptr(), w.data_ptr(), M, N, K, lda):
+        gemm_f32_split(a, w, out, out_mode == OUT_ADD_F32, bias)
+        return
     _check(library().rl_gemm_simt(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _dt(a), out_mode,
                                   M, N, K, lda, ldo, _stream()), "rl_gemm_simt")
+    _count()
+
+
+def gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, add: bool, bias: Optional[torch.Tensor] = None,
+                   parts: int = 0) -> None:
+    """out = a @ w.T (+ bias), or added into out: float operands cut into three bf16 terms each, products on the tensor
+    cores, sums of 64 values of k added up in float registers (csrc/gemm_f32_split.cu).  ``parts``: CTAs that share a tile's
+    K range (0: by the shapes)."""
+    _need(a, "a", torch.float32, contiguous=False); _need(w, "w", torch.float32); _need(out, "out", torch.float32, contiguous=False)
+    M, K = a.shape
+    N = w.shape[0]
+    assert w.shape[1] == K and out.shape == (M, N) and a.stride(1) == 1 and out.stride(1) == 1
+    _check(library().rl_gemm_f32_split(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), int(bool(add)), M, N, K,
+                                       a.stride(0) if M > 1 else K, out.stride(0) if M > 1 else N,
+                                       _tc_error_word(a.device).data_ptr(), parts, _stream()), "rl_gemm_f32_split")
     _count()
 
 
@@ -1429,7 +1451,8 @@ def check_device_errors() -> None:
             t.zero_()
             raise KernelError(f"a tensor-core kernel on cuda:{key} gave up waiting (code {code}; matrix product: "
                               "1 = for a free stage, 2 = for a TMA load, 3 = for the accumulator, 4 = for a free "
-                              "accumulator; prefill attention: 11 = producer, 12/13 = MMA issuer, 14 = softmax)")
+                              "accumulator; prefill attention: 11 = producer, 12/13 = MMA issuer, 14 = softmax; 32-bit "
+                              "product: 21 = for a free stage, 22 = for sums, 23 / 24 = MMA issuer)")
 
 
 def gemm_tc_supported(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:

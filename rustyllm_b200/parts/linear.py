@@ -2,9 +2,9 @@
 
 Every weight is ``[out x in]`` with ``in`` contiguous and is used as ``y = W x``
 (SimonWaldherr/RustyLLM src/model.rs:185-186), so both operands are K-major.
-float32 weights run on the CUDA cores with float32 accumulation (the true 32-bit
-path).  bfloat16 weights run on the tensor cores where the tensor-core kernel takes
-the shape, else on the CUDA cores with float32 accumulation.
+float32 weights run with float32 accuracy (``K.gemm_simt`` picks the kernel: on the CUDA cores,
+or on the tensor cores from exact bf16 cuts of both operands).  bfloat16 weights run on the tensor
+cores where the tensor-core kernel takes the shape, else on the CUDA cores with float32 accumulation.
 """
 from __future__ import annotations
 

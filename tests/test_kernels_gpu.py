@@ -1219,3 +1219,76 @@ def test_attention_f32_options_follow_the_any_shape_kernel(H, G, hd, options):
     k.attention_simt(q, kp, vp, pt, sot, pos, out, H, G, hd, 1.0 / math.sqrt(hd), **kw)
     k.attention_simt(q, kp, vp, pt, sot, pos, plain, H, G, hd, 1.0 / math.sqrt(hd), chunk=1 << 20, **kw)
     torch.testing.assert_close(out, plain, rtol=1e-5, atol=4e-6)
+
+
+# ----------------------------------------------------------------------------- 32-bit products from bf16 cuts
+def _f32_split(k, a, w, bias=None, parts=0):
+    out = torch.empty(a.shape[0], w.shape[0], device=DEV)
+    k.gemm_f32_split(a, w, out, False, bias, parts)
+    return out
+
+
+def _f32_ordered(k, a, w, bias=None):
+    """The sum in the order of k, on the CUDA cores."""
+    out = torch.empty(a.shape[0], w.shape[0], device=DEV)
+    k._check(k.library().rl_gemm_simt(a.data_ptr(), w.data_ptr(), k._ptr(bias), out.data_ptr(), k.F32, k.OUT_F32, a.shape[0], w.shape[0],
+                                      a.shape[1], a.stride(0), w.shape[0], k._stream()), "rl_gemm_simt")
+    return out
+
+
+@pytest.mark.parametrize("M,N,K_", [(1, 1, 4), (17, 256, 256), (33, 384, 516), (65, 256, 256), (127, 300, 260), (128, 128, 64), (129, 129, 1028), (200, 500, 2048),
+                                    (300, 257, 8192)])
+@pytest.mark.parametrize("parts", [0, 1, 2, 4, 8])
+def test_gemm_f32_split_is_as_exact_as_the_ordered_sum(M, N, K_, parts):
+    """Error against 64 bits, relative to the result's rms, no larger than that of the sum in the order of k from K = 256 on, where
+    the product is taken (both are seen to be 1e-7 to 1e-6; 3e-8 is a rounding of the result itself); bias, strided rows and
+    addition into the output.  Shorter sums have fewer roundings to save: up to four units in the last place of a sum of 64 values
+    that the tensor core cuts off (4 x 2^-24) against the ordered sum's 64 roundings to nearest (8 x 2^-25 in the mean)."""
+    k = K()
+    a, w, bias = _rand(M, K_ + 4, seed=1)[:, :K_], _rand(N, K_, seed=2), _rand(N, seed=3)
+    a = a * torch.exp(2.0 * _rand(M, K_, seed=6))          # values of very different sizes
+    wide = torch.zeros(M, K_ + 4, device=DEV)
+    wide[:, :K_] = a
+    a = wide[:, :K_]
+    ref = a.double() @ w.double().T + bias.double()
+    out = _f32_split(k, a, w, bias, parts)
+    plain = _f32_ordered(k, a, w, bias)
+    rms = ref.square().mean().sqrt()
+    err = lambda x: ((x.double() - ref).square().mean().sqrt() / rms).item()
+    print(f"split {err(out):.3g}, ordered {err(plain):.3g}")
+    assert err(out) <= err(plain) * (1.0 if K_ >= 256 else 1.5) + 3e-8
+    res = _rand(M, N + 4, seed=4)[:, :N]
+    into = res.clone()
+    k.gemm_f32_split(a, w, into, True, bias, parts)
+    assert torch.equal(into, res + out)
+    again = _f32_split(k, a, w, bias, parts)
+    assert torch.equal(again, out)
+
+
+def test_gemm_f32_split_keeps_what_is_no_finite_number_and_the_largest_floats():
+    k = K()
+    M, N, K_ = 70, 256, 256
+    a, w = _rand(M, K_, seed=1), _rand(N, K_, seed=2)
+    a[3, 5], a[4, 7], a[5, 9] = math.inf, math.nan, 3.4e38
+    w[6] *= 0.0
+    w[6, 9] = 1.0
+    w[8, 5] = 0.0
+    out = _f32_split(k, a, w)
+    plain = _f32_ordered(k, a, w)
+    assert torch.equal(torch.isnan(out), torch.isnan(plain)) and torch.equal(torch.isinf(out), torch.isinf(plain))
+    assert out[5, 6] == plain[5, 6] == a[5, 9]
+    fine = torch.isfinite(plain)
+    torch.testing.assert_close(out[fine], plain[fine], rtol=1e-5, atol=1e-4)
+
+
+def test_products_of_many_float_rows_take_the_split_kernel():
+    k = K()
+    lib = k.library()
+    a, w = _rand(100, 512, seed=1), _rand(256, 512, seed=2)
+    out = torch.empty(100, 256, device=DEV)
+    k.gemm_simt(a, w, out, k.OUT_SAME)
+    assert torch.equal(out, _f32_split(k, a, w))
+    p = a.data_ptr()
+    for bad in ((8, 256, 512, 512), (100, 127, 512, 512), (100, 256, 252, 252), (100, 256, 510, 510), (100, 256, 512, 514)):
+        assert not lib.rl_gemm_f32_split_supported(p, w.data_ptr(), *bad)
+    assert not lib.rl_gemm_f32_split_supported(p + 4, w.data_ptr(), 100, 256, 512, 512)
