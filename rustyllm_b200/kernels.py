@@ -45,6 +45,11 @@ _SIGNATURES = {
     "rl_gemm_f32_split_supported": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int],
     "rl_gemm_f32_split": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int,
                           _c_void_p],
+    "rl_linear_scan_chunks": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_int, _c_int, _c_int,
+                              _c_int, _c_int],
+    "rl_linear_scan_chunked": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p,
+                               _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_void_p, _c_int, _c_int,
+                               _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_layer_norm": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_float, _c_void_p],
     "rl_branch_join": [_c_void_p, _c_float, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p, _c_void_p, _c_float, _c_void_p, _c_int, _c_int, _c_int, _c_void_p],
@@ -1146,6 +1151,16 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Te
         assert skip.numel() == num_heads
     sp, ss = _state_args(state)
     assert state.shape[1] >= 4 * num_heads * dk * dv
+    chunks = library().rl_linear_scan_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _dt(q), sp, ss,
+                                             M, seq_slots.numel(), num_heads, dk, dv)
+    if chunks:      # many tokens: products a chunk of 64 instead of a walk (csrc/linear_scan_chunked.cu)
+        work = torch.empty(chunks * num_heads * (dk * dv + 1), dtype=torch.float32, device=out.device)
+        _check(library().rl_linear_scan_chunked(
+            q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _ptr(dt_raw), lddt, _dt(q), _ptr(dt_bias),
+            rate.data_ptr(), _ptr(skip), mode, int(bool(silu)), cu_seqlens.data_ptr(), seq_slots.data_ptr(), seq_slots.numel(), sp, ss,
+            out.data_ptr(), out.stride(0), M, num_heads, heads_per_group, dk, dv, work.data_ptr(), _stream()), "rl_linear_scan_chunked")
+        _count(3)
+        return
     _check(library().rl_linear_scan(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _ptr(dt_raw), lddt,
                                     _dt(q), _ptr(dt_bias), rate.data_ptr(), _ptr(skip), mode, int(bool(silu)), cu_seqlens.data_ptr(),
                                     seq_slots.data_ptr(), seq_slots.numel(), sp, ss, out.data_ptr(), out.stride(0), num_heads,

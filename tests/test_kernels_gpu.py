@@ -1292,3 +1292,98 @@ def test_products_of_many_float_rows_take_the_split_kernel():
     for bad in ((8, 256, 512, 512), (100, 127, 512, 512), (100, 256, 252, 252), (100, 256, 510, 510), (100, 256, 512, 514)):
         assert not lib.rl_gemm_f32_split_supported(p, w.data_ptr(), *bad)
     assert not lib.rl_gemm_f32_split_supported(p + 4, w.data_ptr(), 100, 256, 512, 512)
+
+
+# ----------------------------------------------------------------------------- linear recurrences by chunks
+def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed):
+    """Inputs as views of one wide buffer, states that are not zero, and the recurrence in float64 on what the kernel reads."""
+    M, G = sum(lens), H // hpg
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    buf = rand(M, 2 * G * dk + H * dv + H + 4 - H % 4).to(dtype)
+    k, q, v = buf[:, :G * dk], buf[:, G * dk:2 * G * dk], buf[:, 2 * G * dk:2 * G * dk + H * dv]
+    dt = buf[:, 2 * G * dk + H * dv:2 * G * dk + H * dv + H]
+    dt_bias, skip = rand(H), rand(H)
+    rate = torch.tensor([0.9, 0.5, 0.999, 1.0, 0.0][:H] * H, device=DEV)[:H].contiguous() if mode == 0 else rand(H) * 2.0
+    slots = list(range(len(lens) - 1, -1, -1))
+    state = torch.zeros(len(lens) + 1, 4 * H * dk * dv + 256, dtype=torch.uint8, device=DEV)
+    state.view(torch.float32).copy_(rand(len(lens) + 1, H * dk * dv + 64))
+    act = mode == 0
+    f = lambda x: (torch.nn.functional.silu(x.double()) if act else x.double())
+    Q, K_, V = (f(x).view(M, -1, w).repeat_interleave(r, dim=1) for x, w, r in ((q, dk, hpg), (k, dk, hpg), (v, dv, 1)))
+    if mode:
+        b = torch.nn.functional.softplus(dt.double() + dt_bias.double(), threshold=40.0)
+        a = torch.exp(-torch.exp(rate.double()) * b)
+    else:
+        b, a = torch.ones(M, H, dtype=torch.float64, device=DEV), rate.double().expand(M, H)
+    ref, last, at = torch.empty(M, H, dv, dtype=torch.float64, device=DEV), {}, 0
+    for s, n in zip(slots, lens):
+        S = state[s, :4 * H * dk * dv].view(torch.float32).view(H, dv, dk).transpose(1, 2).double()
+        for t in range(at, at + n):
+            S = a[t][:, None, None] * S + (b[t][:, None] * K_[t])[:, :, None] * V[t][:, None, :]
+            ref[t] = (Q[t][:, None, :] @ S)[:, 0] + (skip.double()[:, None] * V[t] if mode else 0.0)
+        last[s] = S.transpose(1, 2)
+        at += n
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    kw = dict(dt_raw=dt, dt_bias=dt_bias, skip=skip) if mode else dict(silu=True)
+    return (q, k, v), state, cu, torch.tensor(slots, dtype=torch.int32, device=DEV), rate, kw, ref.flatten(1), last
+
+
+def _scan_walk(k, qkv, state, cu, slots, rate, kw, H, hpg, dk, dv):
+    """The walk from token to token, whatever the number of tokens."""
+    q, kk, v = qkv
+    out = torch.empty(q.shape[0], H * dv, device=DEV)
+    sp, ss = k._state_args(state)
+    dt = kw.get("dt_raw")
+    k._check(k.library().rl_linear_scan(q.data_ptr(), q.stride(0), kk.data_ptr(), kk.stride(0), v.data_ptr(), v.stride(0), k._ptr(dt),
+                                        dt.stride(0) if dt is not None else 0, k._dt(q), k._ptr(kw.get("dt_bias")), rate.data_ptr(),
+                                        k._ptr(kw.get("skip")), int(dt is not None), int(kw.get("silu", False)), cu.data_ptr(),
+                                        slots.data_ptr(), slots.numel(), sp, ss, out.data_ptr(), out.stride(0), H, hpg, dk, dv, 1,
+                                        k._stream()), "rl_linear_scan")
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("H,hpg,dk,dv", [(5, 1, 128, 128), (4, 2, 64, 128), (4, 4, 128, 64), (3, 1, 64, 64)])
+def test_linear_scan_by_chunks_is_as_exact_as_the_walk(dtype, mode, H, hpg, dk, dv):
+    """Sequences that end beside the edges of chunks of 64, from states that are not zero, decays from 1 to 0: outputs and states
+    against float64, as exact as the walk's (1e-7 of the rms: sums of up to 128 values in float)."""
+    k = K()
+    lens = [130, 1, 64, 65, 63, 128, 200]
+    qkv, state, cu, slots, rate, kw, ref, last = _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed=dk + dv + mode)
+    before = state.clone()
+    walked_state = state.clone()
+    walk = _scan_walk(k, qkv, walked_state, cu, slots, rate, kw, H, hpg, dk, dv)
+    out = torch.empty_like(walk)
+    launches = k.launch_count
+    k.linear_scan(*qkv, out, state, cu, slots, H, hpg, dk, dv, rate, **kw)
+    assert k.launch_count - launches == 3, "the chunked form"
+    rel = lambda x, y: ((x.double() - y).square().mean().sqrt() / y.square().mean().sqrt()).item()
+    print(f"chunks {rel(out, ref):.3g}, walk {rel(walk, ref):.3g}")
+    assert rel(out, ref) <= rel(walk, ref) + 1e-7
+    n = 4 * H * dk * dv
+    for s, S in last.items():
+        got, other = (x[s, :n].view(torch.float32).view(H, dv, dk) for x in (state, walked_state))
+        assert rel(got, S) <= rel(other, S) + 1e-7
+    assert torch.equal(state[:, n:], before[:, n:]) and torch.equal(state[len(lens)], before[len(lens)])
+
+
+def test_linear_scan_by_chunks_keeps_later_tokens_out_of_earlier_outputs_and_takes_what_it_can():
+    k = K()
+    H, dk, dv = 2, 128, 64
+    qkv, state, cu, slots, rate, kw, ref, _ = _scan_case(torch.float32, 1, H, 1, dk, dv, [260], seed=3)
+    out = torch.empty(260, H * dv, device=DEV)
+    first = state.clone()
+    k.linear_scan(*qkv, out, first, cu, slots, H, 1, dk, dv, rate, **kw)
+    qkv[2][85], qkv[1][100] = math.inf, math.nan
+    again = torch.empty_like(out)
+    k.linear_scan(*qkv, again, state, cu, slots, H, 1, dk, dv, rate, **kw)
+    assert torch.equal(again[:85], out[:85]) and not torch.isfinite(again[85:]).any()
+    lib, q = k.library(), qkv[0]
+    ask = lambda ptr=q.data_ptr(), ld=128, dt=0, st=0, M=256, B=1, a=128, b=128: lib.rl_linear_scan_chunks(
+        ptr, ld, q.data_ptr() & ~15, 128, q.data_ptr() & ~15, 128, dt, st, 128, M, B, 16, a, b)
+    ok = q.data_ptr() & ~15
+    assert ask(ok) == 5
+    for bad in (dict(ptr=ok + 4), dict(ld=126), dict(st=4), dict(M=255), dict(M=319, B=10), dict(a=96), dict(b=32), dict(M=100_000)):
+        assert ask(**{"ptr": ok, **bad}) == 0, bad
