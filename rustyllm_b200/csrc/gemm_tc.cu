@@ -406,6 +406,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // there are about as many of them as CTAs: the last wave then takes bt / BT of a full
 // wave's time instead of a whole one with most CTAs idle.  No partial sums, no fix-up:
 // a narrow tile is a whole tile of its own.
+// Eight epilogue warps, two a quarter of the weight rows: with four, a tile of K = 2,048 (11 us of products) whose epilogue has more to do than
+// store took longer to drain than to multiply (2,048 -> 16,384 with SwiGLU, 5,514 tokens: 348 us, with a plain store 282; with eight 281 and
+// 280; 2,048 -> 2,048 added into the residual 52.2 -> 44.9 us).
+static constexpr int TC_PERSISTENT_THREADS = 320;
 struct TcTail {
   int first;         // index of the first narrow tile = number of tiles of full width
   int bt;            // tokens a narrow tile (a multiple of 16, <= BT)
@@ -428,7 +432,7 @@ __device__ __forceinline__ TcTileAt tc_tile_at(int tile, int tiles_m, int BT, co
 
 
 template <int BT>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                           const __grid_constant__ CUtensorMap map_a_tail, const float* __restrict__ bias,
                           void* __restrict__ out, int out_mode, int M, int N, int K,
@@ -459,7 +463,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&acc_full[i]), 1);
-      mbar_init(smem_u32(&acc_empty[i]), 4);       // one arrival per epilogue warp
+      mbar_init(smem_u32(&acc_empty[i]), 8);       // one arrival per epilogue warp
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -551,7 +555,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
   } else {
     // ---------------- epilogue warps ----------------
     rl_pdl_wait();
-    const int quarter = warp & 3;
+    // two warps a quarter of the weight rows: the first takes the first half of the tile's tokens, in whole 32s (what the
+    // add-into-residual form takes at a time), the second the rest
+    const int quarter = warp & 3, second = (warp - 2) >> 2;
     int t = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const TcTileAt at = tc_tile_at(tile, tiles_m, BT, tail);
@@ -566,7 +572,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       TcFuse fuse = {};
       fuse.act_limit = act_limit;
       fuse.act_alpha = act_alpha;
-      tile_epilogue<BT>(tmem_base + (uint32_t)(buf * BT), quarter, lane, at.n0, at.m0, min(at.bt, M - at.m0), M, N, ldo, bias, out,
+      const int cols = min(at.bt, M - at.m0), half = min(cols, (at.bt / 2 + 31) & ~31), c0 = second ? half : 0;
+      tile_epilogue<BT>(tmem_base + (uint32_t)(buf * BT + c0), quarter, lane, at.n0, at.m0 + c0, second ? cols - half : half, M, N, ldo, bias, out,
                         out_mode, fuse, nullptr);
       tc_fence_before();
       __syncwarp();
@@ -620,7 +627,7 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
     if (rc != RL_OK) return rc;
   }
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
-  cudaError_t e = rl_launch_pdl(gemm_tc_persistent_kernel<BT>, dim3(grid), dim3(TC_THREADS), (size_t)Cfg::SMEM_BYTES, stream,
+  cudaError_t e = rl_launch_pdl(gemm_tc_persistent_kernel<BT>, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)Cfg::SMEM_BYTES, stream,
                                 mw, ma, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tiles_m, num_tiles, tail, tile_group, group_rows,
                                 fuse.act_limit, fuse.act_alpha);
   if (e != cudaSuccess) {
