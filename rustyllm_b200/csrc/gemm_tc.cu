@@ -199,7 +199,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_splits = (int)cluster_size(), split = (int)cluster_rank();
   const int n0 = (blockIdx.x / num_splits) * BLOCK_N_OUT;   // first weight row (output feature) of this CTA
-  const int m0 = blockIdx.y * BT;                           // first token of this CTA
+  const int tile_m = BT > 64 && fuse.tile_m > 0 ? fuse.tile_m : BT;      // tokens of a tile
+  const int m0 = blockIdx.y * tile_m;                       // first token of this CTA
   int w_row0 = n0;                                          // first row of the weight tile in the weight's tensor map
   if (fuse.tile_group != nullptr) {
     // grouped: which of the stacked matrices this token tile meets is written by a kernel in front,
@@ -239,7 +240,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int pre = min(num_kb, Cfg::STAGES);
       for (int kb = 0; kb < pre; ++kb) {
         const uint32_t fb = smem_u32(&full_bar[kb]);
-        mbar_expect_tx(fb, Cfg::STAGE_BYTES);
+        mbar_expect_tx(fb, (BLOCK_N_OUT + tile_m) * BLOCK_K * 2);
         tma_load_2d(smem_u32(tiles + (size_t)kb * Cfg::STAGE_BYTES), &map_w, fb, (kb0 + kb) * BLOCK_K, w_row0);
       }
       rl_pdl_wait();
@@ -254,7 +255,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           break;
         }
         const uint32_t fb = smem_u32(&full_bar[s]);
-        mbar_expect_tx(fb, Cfg::STAGE_BYTES);
+        mbar_expect_tx(fb, (BLOCK_N_OUT + tile_m) * BLOCK_K * 2);
         uint8_t* st = tiles + (size_t)s * Cfg::STAGE_BYTES;
         tma_load_2d(smem_u32(st), &map_w, fb, (kb0 + kb) * BLOCK_K, w_row0);
         tma_load_2d(smem_u32(st + BLOCK_N_OUT * BLOCK_K * 2), &map_a, fb, (kb0 + kb) * BLOCK_K, m0);
@@ -263,7 +264,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- MMA issuer ----------------
-      constexpr uint32_t idesc = make_idesc(BLOCK_N_OUT, BT);
+      const uint32_t idesc = make_idesc(BLOCK_N_OUT, tile_m);
       bool ok = true;
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         const int s = kb % Cfg::STAGES;
@@ -317,12 +318,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int quarter = warp & 3;                    // lanes this warp may read
     const int row = quarter * 32 + lane;             // accumulator row = weight row of the tile
     if (ok && num_splits == 1) {
-      tile_epilogue<BT>(tmem_base, quarter, lane, n0, m0, min(BT, M - m0), M, N, ldo, bias, out, out_mode, fuse, fuse_smem);
+      tile_epilogue<BT>(tmem_base, quarter, lane, n0, m0, min(tile_m, M - m0), M, N, ldo, bias, out, out_mode, fuse, fuse_smem);
     } else if (num_splits > 1 && ok) {
       // this part's partial tile -> own shared memory (the ring is free: every MMA has
       // completed), as [token column][weight row] floats
       float* red = reinterpret_cast<float*>(tiles);
-      const int cols = min(BT, M - m0);
+      const int cols = min(tile_m, M - m0);
 #pragma unroll 1
       for (int c = 0; c < BT / 16; ++c) {
         if (c * 16 >= cols) break;
@@ -346,7 +347,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int et = threadIdx.x - 64;
       const int r4 = (et & 31) * 4, cg = et >> 5;
       const int nn = n0 + r4;
-      const int cols = min(BT, M - m0);
+      const int cols = min(tile_m, M - m0);
       const uint32_t red_local = smem_u32(tiles);
       const bool vec_ok = (nn + 3 < N) && ((ldo & 3) == 0) && (((uintptr_t)out & 15) == 0);
       float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                           const __grid_constant__ CUtensorMap map_a_tail, const float* __restrict__ bias,
                           void* __restrict__ out, int out_mode, int M, int N, int K,
-                          int ldo, int* __restrict__ err, int tiles_m, int num_tiles, const TcTail tail,
+                          int ldo, int* __restrict__ err, int tile_m, int tiles_m, int num_tiles, const TcTail tail,
                           const int* __restrict__ tile_group, int group_rows, float act_limit, float act_alpha) {
   // tile_group (null: none): the weight is stacked matrices of group_rows rows, and the token tile of BT rows at
   // m0 multiplies with matrix tile_group[m0 / BT]; negative: the tile is skipped by every role alike.  The table
@@ -485,7 +486,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       bool waited = false, ok = true;
       if (tile_group != nullptr) { rl_pdl_wait(); waited = true; }
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TcTileAt at = tc_tile_at(tile, tiles_m, BT, tail);
+        const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
         int n0 = at.n0;
         const int m0 = at.m0;
         if (tile_group != nullptr) {
@@ -508,7 +509,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
           // weights may be requested before the preceding kernels have finished, activations not
           if (!waited) { rl_pdl_wait(); waited = true; }
           uint8_t* sa = st + BLOCK_N_OUT * BLOCK_K * 2;
-          tma_load_2d(smem_u32(sa), at.bt == BT ? &map_a : &map_a_tail, fb, kb * BLOCK_K, m0);
+          tma_load_2d(smem_u32(sa), at.bt == tile_m ? &map_a : &map_a_tail, fb, kb * BLOCK_K, m0);
         }
       }
     }
@@ -519,7 +520,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       bool ok = true;
       if (tile_group != nullptr) rl_pdl_wait();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TcTileAt mat = tc_tile_at(tile, tiles_m, BT, tail);
+        const TcTileAt mat = tc_tile_at(tile, tiles_m, tile_m, tail);
         if (tile_group != nullptr && tile_group[mat.m0 / BT] < 0) continue;
         const uint32_t idesc = make_idesc(BLOCK_N_OUT, mat.bt);
         const int buf = t & 1;
@@ -560,7 +561,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     const int quarter = warp & 3, second = (warp - 2) >> 2;
     int t = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const TcTileAt at = tc_tile_at(tile, tiles_m, BT, tail);
+      const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
       if (tile_group != nullptr && tile_group[at.m0 / BT] < 0) continue;
       const int buf = t & 1;
       const uint32_t acc_phase = (t >> 1) & 1;
@@ -587,6 +588,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 }
 
 
+// The height of equal tiles that cover M tokens with as many of them as tiles of BT do, in the instruction's steps of 16: 293 tokens are two
+// tiles of 160, not 256 and a mostly empty 256 (a product instruction of 160 columns takes 100 clocks, of 256 columns 128).  8B shape,
+// 293 tokens: gate-up 99.6 -> 93.0 us, QKV 26.4 -> 25.2 us, O 28.6 -> 23.7 us, down 61.5 -> 52.1 us.
+static int balanced_tile(int M, int BT) {
+  const int tiles = (M + BT - 1) / BT, each = (M + tiles - 1) / tiles;
+  return (each + 15) / 16 * 16;
+}
+
 template <int BT>
 static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, const void* A, int lda, const float* bias,
                                 void* out, int out_mode, int M, int N, int K, int ldo, int* err, cudaStream_t stream,
@@ -601,17 +610,18 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
     configured = true;
   }
   const int num_sms = rl_num_sms();
-  const int tiles_m = (M + BT - 1) / BT, tiles_n = (N + BLOCK_N_OUT - 1) / BLOCK_N_OUT;
+  const int tile_m = tile_group != nullptr ? BT : balanced_tile(M, BT);
+  const int tiles_m = (M + tile_m - 1) / tile_m, tiles_n = (N + BLOCK_N_OUT - 1) / BLOCK_N_OUT;
   const int total = tiles_m * tiles_n;
   // the tiles behind the last full wave: the narrowest token tile (from 64 tokens: below, the
   // weight tile's trip through shared memory takes longer than the products) that leaves no
   // more of them than there are CTAs
-  TcTail tail = {total, BT, 0, 0, 0, 1, tile_group != nullptr ? tiles_n : 0};
+  TcTail tail = {total, tile_m, 0, 0, 0, 1, tile_group != nullptr ? tiles_n : 0};
   int num_tiles = total;
   const int full = (total / num_sms) * num_sms;
   if (full < total && tile_group == nullptr) {      // grouped: a narrow tile could lie across two groups' rows
-    const int n_first = full / tiles_m, t0_first = (full % tiles_m) * BT;
-    for (int bt = 64; bt < BT; bt += 16) {
+    const int n_first = full / tiles_m, t0_first = (full % tiles_m) * tile_m;
+    for (int bt = 64; bt < tile_m; bt += 16) {
       const int count_first = (M - t0_first + bt - 1) / bt, per_n = (M + bt - 1) / bt;
       const int cnt = count_first + (tiles_n - n_first - 1) * per_n;
       if (cnt <= num_sms) {
@@ -621,14 +631,18 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
       }
     }
   }
-  CUtensorMap ma_tail = ma;      // the same activations in boxes as tall as a narrow tile
+  CUtensorMap ma_tile = ma, ma_tail = ma;      // the same activations in boxes as tall as a tile, and as a narrow tile
+  if (tile_m != BT) {
+    const int rc = tc_make_map(&ma_tile, A, M, K, lda, tile_m);
+    if (rc != RL_OK) return rc;
+  }
   if (tail.bt != BT) {
     const int rc = tc_make_map(&ma_tail, A, M, K, lda, tail.bt);
     if (rc != RL_OK) return rc;
   }
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
   cudaError_t e = rl_launch_pdl(gemm_tc_persistent_kernel<BT>, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)Cfg::SMEM_BYTES, stream,
-                                mw, ma, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tiles_m, num_tiles, tail, tile_group, group_rows,
+                                mw, ma_tile, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, tail, tile_group, group_rows,
                                 fuse.act_limit, fuse.act_alpha);
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_tc: launch of the persistent kernel failed: %s", cudaGetErrorString(e));
@@ -831,6 +845,11 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
     default: break;
   }
   if (splits > 1) {       // few tiles of many tokens: the parts of a tile as a cluster, as for few tokens
+    fuse.tile_m = balanced_tile(M, bt);
+    if (fuse.tile_m != bt) {
+      rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
+      if (rc != RL_OK) return rc;
+    }
     if (bt == 128) return launch_tc<128>(mw, ma, bias, out, out_mode, M, N, K, ldo, err, splits, kb_per, fuse, stream);
     return launch_tc<256>(mw, ma, bias, out, out_mode, M, N, K, ldo, err, splits, kb_per, fuse, stream);
   }

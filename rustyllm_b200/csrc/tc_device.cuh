@@ -65,6 +65,8 @@ struct TcFuse {
   int group_rows;
   // constants of the clamped gate (out_mode TC_OUT_CLAMPED only)
   float act_limit, act_alpha;
+  // tokens of a tile of the cluster kernel for more than 64 tokens (0: all that the kernel's form holds)
+  int tile_m;
 };
 
 static constexpr int BLOCK_N_OUT = 128;   // weight rows per CTA (MMA M)

@@ -1174,6 +1174,39 @@ def test_kernels_refuse_what_they_cannot_do():
         k.swiglu(torch.zeros(2, 4, dtype=torch.float16, device=DEV), torch.zeros(2, 2, dtype=torch.float16, device=DEV))
 
 
+# ----------------------------------------------------------------------------- token tiles of equal height
+@pytest.mark.parametrize("M", [65, 79, 81, 129, 143, 145, 256, 257, 271, 289, 293, 513, 530, 769])
+@pytest.mark.parametrize("splits", [1, 2, 4])
+def test_gemm_tc_token_tiles_of_every_height(M, splits):
+    """Numbers of tokens whose equal tiles are and are not multiples of 16 and of 32 (the epilogue's halves), in one part (the persistent
+    kernel) and as clusters, in every form of output; rows behind the last stay as they are.  Tolerances as above: K = 520 float sums,
+    one rounding to bf16."""
+    k = K()
+    N, K_ = 390, 520
+    a, w, bias = _rand(M, K_, dtype=torch.bfloat16, seed=1), _rand(N, K_, dtype=torch.bfloat16, seed=2), _rand(N, seed=3)
+    ref = a.double() @ w.double().T
+    f32 = dict(rtol=1e-4, atol=8e-5 * math.sqrt(K_))
+    res = _rand(M + 5, N, seed=4)
+    out = res.clone()
+    k.gemm_tc(a, w, out[:M], k.OUT_ADD_F32, bias, force_splits=splits)
+    torch.testing.assert_close(out[:M].double(), ref + bias.double() + res[:M].double(), **f32)
+    assert torch.equal(out[M:], res[M:])
+    out = res.clone()
+    k.gemm_tc(a, w, out[:M], k.OUT_F32, force_splits=splits)
+    torch.testing.assert_close(out[:M].double(), ref, **f32)
+    assert torch.equal(out[M:], res[M:])
+    same = res.to(torch.bfloat16)
+    k.gemm_tc(a, w, same[:M], k.OUT_SAME, force_splits=splits)
+    torch.testing.assert_close(same[:M].double(), ref, rtol=1e-2, atol=1e-2 * math.sqrt(K_))
+    assert torch.equal(same[M:], res[M:].to(torch.bfloat16))
+    act = res[:, :N // 2].to(torch.bfloat16).contiguous()
+    k.gemm_tc(a, w * 0.05, act[:M], k.OUT_SWIGLU, force_splits=splits)
+    small = a.double() @ (w * 0.05).double().T
+    torch.testing.assert_close(act[:M].double(), torch.nn.functional.silu(small[:, 0::2]) * small[:, 1::2], rtol=2e-2, atol=2e-2)
+    assert torch.equal(act[M:], res[M:, :N // 2].to(torch.bfloat16))
+    k.check_device_errors()
+
+
 # ----------------------------------------------------------------------------- 32-bit attention by tiles of rows
 @pytest.mark.parametrize("H,G,hd", [(4, 4, 64), (8, 2, 64), (15, 3, 64), (16, 1, 64), (3, 3, 128), (6, 1, 128), (28, 2, 128)])
 def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
