@@ -352,7 +352,7 @@ int sp_launch(const float* A, const float* W, const float* bias, float* out, int
 
 // 1 where the split product is taken instead of the CUDA cores: rows that 16-byte pieces can fetch, a tile's width of outputs, sums from
 // K = 256 on (shorter ones it does not make more exactly than the ordered sum: K = 64 1.7e-7 against 1.4e-7 of the result's rms, K = 256
-// 2.1e-7 against 2.3e-7), and more than 8 tokens (up to there gemm_simt.cu streams the weight).
+// 2.1e-7 against 2.3e-7), and more than 8 tokens (up to there gemm_f32_few.cu: see there).
 extern "C" int rl_gemm_f32_split_supported(const void* A, const void* W, int M, int N, int K, int lda) {
   return M > 8 && N >= 128 && K >= 256 && K % 4 == 0 && lda % 4 == 0 && lda >= K && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 &&
          (N + 127) / 128 <= 65535;

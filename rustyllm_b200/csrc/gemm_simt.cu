@@ -1,6 +1,6 @@
 // out[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) on the CUDA cores, for any M, N, K.
 //
-// The products of 32-bit runs that gemm_f32_split.cu (many tokens) and the kernel for few tokens do not take - sums
+// The products of 32-bit runs that gemm_f32_split.cu (many tokens) and gemm_f32_few.cu (few) do not take - sums
 // shorter than K = 256, few outputs - and the fallback of the bf16 path for shapes the tensor-core kernel refuses (bf16
 // inputs widened to float, float accumulation).  Both operands are K-major, as every weight of the model is stored
 // ([out x in], out = W x; SimonWaldherr/RustyLLM src/model.rs:185-186).

@@ -1327,6 +1327,34 @@ def test_products_of_many_float_rows_take_the_split_kernel():
     assert not lib.rl_gemm_f32_split_supported(p + 4, w.data_ptr(), 100, 256, 512, 512)
 
 
+@pytest.mark.parametrize("N,K_", [(1, 256), (5, 260), (130, 2048), (4736, 512), (4737, 1028), (257, 8192)])
+def test_gemm_f32_few_is_more_exact_than_the_ordered_sum_and_rows_do_not_depend_on_the_batch(N, K_):
+    """Every number of rows of the kernel's shapes, rows of a wider buffer, bias, addition into the output; a row's bits are the same in
+    every one of them.  Error against 64 bits no larger than that of the sum in the order of k (3e-8: the result's own rounding)."""
+    k = K()
+    wide = _rand(8, K_ + 8, seed=1)
+    w, bias = _rand(N, K_, seed=2), _rand(N, seed=3)
+    a = wide[:, 4:4 + K_]
+    full = torch.empty(8, N, device=DEV)
+    k.gemm_simt(a, w, full, k.OUT_F32, bias)
+    ref = a.double() @ w.double().T + bias.double()
+    err = lambda x: (x.double() - ref).square().mean().sqrt() / ref.square().mean().sqrt()
+    plain = _f32_ordered(k, a, w, bias)
+    print(f"few {err(full):.3g}, ordered {err(plain):.3g}")
+    assert err(full) <= err(plain) + 3e-8
+    for rows in ([7], [0, 6], [3, 4, 5], list(range(5)), list(range(1, 8))):
+        some = torch.empty(len(rows), N + 3, device=DEV)[:, :N]
+        k.gemm_simt(a[rows].contiguous(), w, some, k.OUT_SAME, bias)
+        assert torch.equal(some, full[rows])
+    res = _rand(8, N, seed=4)
+    into = res.clone()
+    k.gemm_simt(a, w, into, k.OUT_ADD_F32, bias)
+    assert torch.equal(into, res + full)
+    lib = k.library()
+    for M, kk, lda in ((0, 256, 256), (9, 256, 256), (4, 252, 256), (4, 258, 260), (4, 256, 258)):
+        assert not lib.rl_gemm_f32_few_supported(w.data_ptr(), w.data_ptr(), M, N, kk, lda)
+
+
 # ----------------------------------------------------------------------------- linear recurrences by chunks
 def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed):
     """Inputs as views of one wide buffer, states that are not zero, and the recurrence in float64 on what the kernel reads."""
