@@ -85,11 +85,15 @@ rope_kv_write_kernel(T* __restrict__ qkv, int ld, const int* __restrict__ positi
 // 16-byte aligned rows.  A thread rotates eight pairs (two 16-byte loads, two 16-byte
 // stores) or copies sixteen value elements.  The token's sines and cosines are the same
 // for all its heads: the CTA computes them once into shared memory.
+// Sixteen heads a CTA: at head size 128 they are a thread's work each.  At 64 they are half of the threads', and with more CTAs than the GPU
+// holds at once a token's CTAs repeat the chain position - page - cosines that bounds them: up to 64 heads a CTA then (32 heads over 8
+// KV heads of 64: 5,514 tokens 18.4 -> 11.4 us, 2,048 7.6 -> 6.2; of 128: 1,200 tokens 7.2 -> 9.5, not taken).
 #define ROPE_FAST_HEADS_PER_CTA 16
+#define ROPE_FAST_MANY_HEADS 64
 __global__ void __launch_bounds__(ROPE_THREADS)
 rope_kv_write_bf16_half_kernel(__nv_bfloat16* __restrict__ qkv, int ld, const int* __restrict__ positions,
                                const int* __restrict__ slot_of_token, const int* __restrict__ page_table, int max_pages,
-                               const float* __restrict__ inv_freq, int H, int G, int hd,
+                               const float* __restrict__ inv_freq, int H, int G, int hd, int heads_per_cta,
                                __nv_bfloat16* __restrict__ k_pool, __nv_bfloat16* __restrict__ v_pool) {
   __shared__ float2 cs[128];                              // (cos, sin) of the token's hd / 2 <= 128 angles
   rl_pdl_trigger();
@@ -101,8 +105,8 @@ rope_kv_write_bf16_half_kernel(__nv_bfloat16* __restrict__ qkv, int ld, const in
   const int page = page_table[(size_t)slot * max_pages + pos / RL_PAGE];
   const size_t dst = ((size_t)page * G) * RL_PAGE * hd + (size_t)(pos % RL_PAGE) * hd;
   const int half = hd / 2, per_head = half / 8;          // groups of eight pairs a head
-  const int slot0 = blockIdx.y * ROPE_FAST_HEADS_PER_CTA;
-  const int nslots = min(ROPE_FAST_HEADS_PER_CTA, H + 2 * G - slot0);
+  const int slot0 = blockIdx.y * heads_per_cta;
+  const int nslots = min(heads_per_cta, H + 2 * G - slot0);
   for (int i = threadIdx.x; i < half; i += ROPE_THREADS) {
     float sn, c;
     sincosf((float)pos * inv_freq[i], &sn, &c);
@@ -320,13 +324,15 @@ extern "C" int rl_rope_kv_write_mixed(void* qkv, int dtype, int ld, const int* p
                   slot_of_token, page_table, max_pages, num_heads * head_dim * esz / 16, num_kv_heads, head_dim * esz / 16,
                   value_dim * esz / 16, (uint4*)k_pool, (uint4*)v_pool);
   else if (v_other == nullptr && dtype == RL_BF16 && write_cache && !interleaved && rotary_dim == head_dim && value_dim == head_dim && head_dim % 16 == 0 && ld % 8 == 0 &&
-      ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)k_pool & 15) == 0 && ((uintptr_t)v_pool & 15) == 0)
-    rl_launch_pdl(rope_kv_write_bf16_half_kernel,
-                  dim3(num_tokens, (num_heads + 2 * num_kv_heads + ROPE_FAST_HEADS_PER_CTA - 1) / ROPE_FAST_HEADS_PER_CTA),
+      ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)k_pool & 15) == 0 && ((uintptr_t)v_pool & 15) == 0) {
+    const int heads = num_heads + 2 * num_kv_heads, at_once = rl_num_sms() * (2048 / ROPE_THREADS);
+    const int per_cta = (long long)num_tokens * ((heads + ROPE_FAST_HEADS_PER_CTA - 1) / ROPE_FAST_HEADS_PER_CTA) > at_once && head_dim <= 64 ? ROPE_FAST_MANY_HEADS
+                                                                                                                                           : ROPE_FAST_HEADS_PER_CTA;
+    rl_launch_pdl(rope_kv_write_bf16_half_kernel, dim3(num_tokens, (heads + per_cta - 1) / per_cta),
                   threads, 0, stream, (__nv_bfloat16*)qkv, ld, positions,
-                  slot_of_token, page_table, max_pages, inv_freq, num_heads, num_kv_heads, head_dim,
+                  slot_of_token, page_table, max_pages, inv_freq, num_heads, num_kv_heads, head_dim, per_cta,
                   (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool);
-  else if (dtype == RL_BF16 && write_cache && interleaved && rotary_dim > 0 && rotary_dim % 8 == 0 && head_dim % 8 == 0 && value_dim % 8 == 0 &&
+  } else if (dtype == RL_BF16 && write_cache && interleaved && rotary_dim > 0 && rotary_dim % 8 == 0 && head_dim % 8 == 0 && value_dim % 8 == 0 &&
            ld % 8 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)k_pool & 15) == 0 && ((uintptr_t)v_pool & 15) == 0 &&
            (v_other == nullptr || (ld_other % 8 == 0 && ((uintptr_t)v_other & 15) == 0)))
     rl_launch_pdl(rope_kv_write_bf16_pairs_kernel, dim3(num_tokens), threads, 0, stream, (__nv_bfloat16*)qkv, ld, positions, slot_of_token,
