@@ -9,7 +9,7 @@
 // once, and only the small second kernel walks from chunk to chunk.
 //
 // What bounds it: multiply-adds on the CUDA cores (about 2.7 M a chunk and head of 128 x 128), where the token-by-token walk is
-// bound by the latency of its chain: 2,048 tokens of 16 heads of 128 x 128: 141 us against 638; 32 heads of 128 x 64: 159 against 606.  Everything
+// bound by the latency of its chain: 2,048 tokens of 16 heads of 128 x 128: 128 us against 637; 32 heads of 128 x 64: 129 against 606.  Everything
 // behind the loads is 32-bit as there; sums of logarithms are 64-bit, so that exp(L_i - L_j) is as exact for late tokens of a chunk as for early
 // ones.  Outputs of a position depend on where chunks begin, that is on how a sequence was cut into steps, to rounding.  Error against 64 bits
 // relative to the outputs' rms: 0.8e-7 to 1.8e-7, the walk's 0.7e-7 to 6.7e-7 (tests/test_kernels_gpu.py).
@@ -44,11 +44,24 @@ __device__ __forceinline__ float4 ch_ld4(const __nv_bfloat16* p) {
   return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
 }
 template <typename T>
-__device__ __forceinline__ float4 ch_value(const T* p, int act) {
-  float4 x = ch_ld4(p);
+__device__ __forceinline__ float4 ch_value(float4 x, int act) {
   if (act) x = make_float4(ch_silu(x.x, T()), ch_silu(x.y, T()), ch_silu(x.z, T()), ch_silu(x.w, T()));
   return x;
 }
+// Rows t0 .. t0 + nt of [., ld] (zeros behind) as 64 rows of W values in registers, four neighbouring ones a piece, all pieces of a thread
+// on their way at once; piece p is row `row(p)`, values `col(p)` .. + 3.
+template <typename T, int W>
+struct ChRows {
+  static constexpr int PIECES = CH * W / 4 / CH_THREADS;
+  float4 x[PIECES];
+  static __device__ __forceinline__ int row(int p) { return (int)(threadIdx.x + p * CH_THREADS) / (W / 4); }
+  static __device__ __forceinline__ int col(int p) { return (int)(threadIdx.x + p * CH_THREADS) % (W / 4) * 4; }
+  __device__ __forceinline__ void load(const T* base, int ld, int t0, int nt) {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+      x[p] = row(p) < nt ? ch_ld4(base + (size_t)(t0 + row(p)) * ld + col(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+};
 
 // chunk `index` of the step: its sequence, first token and number of tokens; false: there is none
 __device__ __forceinline__ bool ch_find(const ChunkArgs& a, int index, int& t0, int& nt) {
@@ -112,26 +125,25 @@ __global__ void __launch_bounds__(CH_THREADS) chunk_add_kernel(const ChunkArgs a
   const int h = blockIdx.x, tid = threadIdx.x;
   int t0, nt;
   if (!ch_find(a, blockIdx.y, t0, nt)) return;
+  const T *k = (const T*)a.k + (size_t)(h / a.hpg) * DK, *v = (const T*)a.v + (size_t)h * DV;
+  ChRows<T, DK> kr;
+  ChRows<T, DV> vr;
+  kr.load(k, a.ldk, t0, nt);                 // on their way while the decays are summed
+  vr.load(v, a.ldv, t0, nt);
   ch_decays<T>(a, h, t0, nt, L, bsize);
   __syncthreads();
   if (tid < CH) weight[tid] = tid < nt ? expf((float)(L[nt - 1] - L[tid])) * bsize[tid] : 0.f;
   if (tid == 0) a.decay[(size_t)blockIdx.y * a.H + h] = expf((float)L[nt - 1]);
   __syncthreads();
-  const T *k = (const T*)a.k + (size_t)(h / a.hpg) * DK, *v = (const T*)a.v + (size_t)h * DV;
-  for (int i = tid; i < CH * DK / 4; i += CH_THREADS) {
-    const int j = i / (DK / 4), n = 4 * (i % (DK / 4));
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < nt) {
-      x = ch_value(k + (size_t)(t0 + j) * a.ldk + n, a.act);
-      const float w = weight[j];
-      x = make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
-    }
-    *reinterpret_cast<float4*>(Ks + j * DK + n) = x;
+#pragma unroll
+  for (int p = 0; p < ChRows<T, DK>::PIECES; ++p) {
+    const float4 x = ch_value<T>(kr.x[p], a.act);
+    const float w = weight[kr.row(p)];
+    *reinterpret_cast<float4*>(Ks + kr.row(p) * DK + kr.col(p)) = make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
   }
-  for (int i = tid; i < CH * DV / 4; i += CH_THREADS) {
-    const int j = i / (DV / 4), c = 4 * (i % (DV / 4));
-    *reinterpret_cast<float4*>(Vs + j * DV + c) = j < nt ? ch_value(v + (size_t)(t0 + j) * a.ldv + c, a.act) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+#pragma unroll
+  for (int p = 0; p < ChRows<T, DV>::PIECES; ++p)
+    *reinterpret_cast<float4*>(Vs + vr.row(p) * DV + vr.col(p)) = ch_value<T>(vr.x[p], a.act);
   __syncthreads();
   constexpr int NN = DK / 64, NCc = DV / 64;           // runs of four n and of four c a thread, 64 apart
   const int tx = tid & 15, ty = tid >> 4;
@@ -262,13 +274,17 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const ChunkArg
   const int h = blockIdx.x, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   int t0, nt;
   if (!ch_find(a, blockIdx.y, t0, nt)) return;
-  ch_decays<T>(a, h, t0, nt, L, bsize);
   const T *q = (const T*)a.q + (size_t)(h / a.hpg) * DK, *k = (const T*)a.k + (size_t)(h / a.hpg) * DK, *v = (const T*)a.v + (size_t)h * DV;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = tid; i < CH * DK / 4; i += CH_THREADS) {
-    const int j = i / (DK / 4), n = 4 * (i % (DK / 4));
-    *reinterpret_cast<float4*>(Qs + j * LQ + n) = j < nt ? ch_value(q + (size_t)(t0 + j) * a.ldq + n, a.act) : zero;
-    *reinterpret_cast<float4*>(X + j * LQ + n) = j < nt ? ch_value(k + (size_t)(t0 + j) * a.ldk + n, a.act) : zero;
+  {
+    ChRows<T, DK> qr, kr;
+    qr.load(q, a.ldq, t0, nt);               // on their way while the decays are summed
+    kr.load(k, a.ldk, t0, nt);
+    ch_decays<T>(a, h, t0, nt, L, bsize);
+#pragma unroll
+    for (int p = 0; p < ChRows<T, DK>::PIECES; ++p) {
+      *reinterpret_cast<float4*>(Qs + qr.row(p) * LQ + qr.col(p)) = ch_value<T>(qr.x[p], a.act);
+      *reinterpret_cast<float4*>(X + kr.row(p) * LQ + kr.col(p)) = ch_value<T>(kr.x[p], a.act);
+    }
   }
   __syncthreads();
   {
@@ -283,9 +299,12 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const ChunkArg
       }
   }
   __syncthreads();
-  for (int i = tid; i < CH * DV / 4; i += CH_THREADS) {
-    const int j = i / (DV / 4), c = 4 * (i % (DV / 4));
-    *reinterpret_cast<float4*>(X + j * DV + c) = j < nt ? ch_value(v + (size_t)(t0 + j) * a.ldv + c, a.act) : zero;
+  {
+    ChRows<T, DV> vr;
+    vr.load(v, a.ldv, t0, nt);
+#pragma unroll
+    for (int p = 0; p < ChRows<T, DV>::PIECES; ++p)
+      *reinterpret_cast<float4*>(X + vr.row(p) * DV + vr.col(p)) = ch_value<T>(vr.x[p], a.act);
   }
   __syncthreads();
   // rows ty + 16 r, columns 64 * half + tx + 16 u: what the chunk's own tokens contribute.  Tokens behind a row's are left out, not
@@ -338,11 +357,11 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const ChunkArg
   const float* S = a.work + ((size_t)blockIdx.y * a.H + h) * DK * DV;
 #pragma unroll
   for (int f = 0; f < HALVES; ++f) {
+    ChRows<float, DK> sr;
+    sr.load(S + (size_t)(64 * f) * DK, DK, 0, 64);
     __syncthreads();                                              // the values, or the columns in front, have been read
-    for (int i = tid; i < 64 * DK / 4; i += CH_THREADS) {
-      const int c = i / (DK / 4), n = 4 * (i % (DK / 4));
-      *reinterpret_cast<float4*>(X + c * LQ + n) = *reinterpret_cast<const float4*>(S + (size_t)(64 * f + c) * DK + n);
-    }
+#pragma unroll
+    for (int p = 0; p < ChRows<float, DK>::PIECES; ++p) *reinterpret_cast<float4*>(X + sr.row(p) * LQ + sr.col(p)) = sr.x[p];
     __syncthreads();
     float s[4][4];
     ch_dots<DK, 4, 4>(Qs, X, tx, ty, s);
@@ -383,7 +402,7 @@ constexpr long long CH_WORK_LIMIT = 768LL << 20;       // bytes of work a call m
 // Chunks that the chunked form of a step of num_tokens tokens is launched for (its work: chunks * heads * (dk * dv + 1) floats), or 0 where the
 // walk of rl_linear_scan is the way: state widths other than 64 and 128, rows that pieces of four elements cannot fetch, fewer than
 // 256 tokens or 32 a sequence (three kernels take some 60 us however little there is: 16 heads of 128 x 128, 128 tokens of one sequence 59
-// us against 43, 256 tokens 59 against 83; 4 sequences of 32 tokens 53 against 45, 8 of 32 tokens 61 against 76, 4 of 64 tokens 65 against
+// us against 43, 256 tokens 56 against 83; 4 sequences of 32 tokens 53 against 45, 8 of 32 tokens 61 against 76, 4 of 64 tokens 65 against
 // 84), or more work than 768 MiB (some 24,000 tokens of 32 such heads).
 extern "C" int rl_linear_scan_chunks(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, int dtype, const void* state,
                                      long long state_stride, int num_tokens, int num_seqs, int num_heads, int dk, int dv) {
