@@ -1174,6 +1174,30 @@ def test_kernels_refuse_what_they_cannot_do():
         k.swiglu(torch.zeros(2, 4, dtype=torch.float16, device=DEV), torch.zeros(2, 2, dtype=torch.float16, device=DEV))
 
 
+@pytest.mark.parametrize("H,G,hd", [(32, 8, 64), (70, 5, 64), (24, 6, 32), (32, 8, 128)])
+def test_rope_of_many_tokens_gives_the_bits_of_few(H, G, hd):
+    """As many tokens as make a CTA take up to 64 heads (head sizes up to 64; 80 heads are two such CTAs), against the same tokens a
+    hundred at a time, whose CTAs take sixteen heads each: rows, keys and values bit for bit."""
+    k = K()
+    M, P_ = 1300, 1300 // 64 + 1
+    qkv = _rand(M, (H + 2 * G) * hd, dtype=torch.bfloat16, seed=1)
+    inv = torch.tensor([500000.0 ** (-2.0 * i / hd) for i in range(hd // 2)], dtype=torch.float32, device=DEV)
+    pos = torch.arange(M, dtype=torch.int32, device=DEV)
+    slot = torch.zeros(M, dtype=torch.int32, device=DEV)
+    table = torch.randperm(P_, generator=torch.Generator().manual_seed(2)).to(torch.int32).to(DEV).view(1, P_)
+    got = []
+    for step in (M, 100):
+        x, kp = qkv.clone(), torch.zeros(P_, G, 64, hd, dtype=torch.bfloat16, device=DEV)
+        vp = torch.zeros_like(kp)
+        for m in range(0, M, step):
+            s = slice(m, min(M, m + step))
+            k.rope_kv_write(x[s], pos[s], slot[s], table, inv, H, G, hd, hd, False, kp, vp)
+        got.append((x, kp, vp))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    assert got[0][1].abs().sum() > 0 and not torch.equal(got[0][0], qkv)
+
+
 # ----------------------------------------------------------------------------- token tiles of equal height
 @pytest.mark.parametrize("M", [65, 79, 81, 129, 143, 145, 256, 257, 271, 289, 293, 513, 530, 769])
 @pytest.mark.parametrize("splits", [1, 2, 4])
