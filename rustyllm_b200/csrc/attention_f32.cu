@@ -4,7 +4,7 @@
 // What bounds it: multiply-adds for a prompt (4 * width a visible pair and head), the cache's bytes and the length of
 // a warp's chain for single tokens.  The any-shape kernel (attention_simt.cu) gives a CTA to a token and head and reads
 // every key's row once for it, one warp-wide sum a score: 914 us for 500 tokens of 32 heads of 64 over 8 KV heads and
-// 151 us for four single tokens behind 96 to 700 (one B200); this kernel: 101 us (10 TFLOP/s: a tile's eight warps have
+// 151 us for four single tokens behind 96 to 700 (one B200); this kernel: 80 us (13 TFLOP/s: a tile's eight warps have
 // one or two chunks each, so its ends weigh) and 15.6 us.  Here the ROWS rows of a CTA are the query heads of a KV head,
 // of one token or of several neighbouring ones, so that a key is read once for all of them, and scores and sums are
 // register tiles: a lane holds four rows by ROWS / 4 keys of a score tile, and four rows by HD * ROWS / 128 dimensions
@@ -12,7 +12,8 @@
 //
 // Keys are taken 32 at a time in position order, chunk c of a sequence by warp c % WARPS, which brings the keys and the values
 // of its chunk into a shared-memory area of its own (16-byte asynchronous copies: the next chunk's keys arrive under
-// this chunk's P V, its values under the next chunk's scores).  At the end the warps' (max, denominator, output)
+// this chunk's P V, its values under the next chunk's scores; or, with more CTAs than SMs, one area for both and two CTAs an SM:
+// see rl_attention_f32).  At the end the warps' (max, denominator, output)
 // are merged in the order of the warps.  Chunks, their warps and the order of every sum are functions of a row's position
 // alone - neither ROWS nor what shares the tile changes a bit - so a position's result does not depend on the
 // batch or on how the tokens were cut into steps.  A dot product is summed in runs of 16 dimensions.
@@ -47,24 +48,29 @@ struct AfArgs {
 
 // a warp's area in floats: keys (rows 16 bytes further apart than they are long: lanes that read one column of eight neighbouring
 // rows meet in no bank), values, probabilities
-template <int HD, int ROWS> constexpr int af_warp_floats() { return AF_CHUNK * (HD + 4) + AF_CHUNK * HD + ROWS * (AF_CHUNK + 4); }
-template <int HD, int ROWS, int WARPS> constexpr int af_smem() { return (ROWS * (HD + 4) + WARPS * af_warp_floats<HD, ROWS>()) * 4; }
+// SHARED: the values take the place of the chunk's keys, so that two CTAs fit an SM
+template <int HD, int ROWS, bool SHARED> constexpr int af_warp_floats() {
+  return AF_CHUNK * (HD + 4) + (SHARED ? 0 : AF_CHUNK * HD) + ROWS * (AF_CHUNK + 4);
+}
+template <int HD, int ROWS, int WARPS, bool SHARED> constexpr int af_smem() {
+  return (ROWS * (HD + 4) + WARPS * af_warp_floats<HD, ROWS, SHARED>()) * 4;
+}
 
-template <int HD, int ROWS, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs a) {
+template <int HD, int ROWS, int WARPS, bool SHARED>
+__global__ void __launch_bounds__(WARPS * 32, SHARED ? 2 : 1) attention_f32_kernel(const AfArgs a) {
   constexpr int RG = ROWS / 4, KG = 32 / RG;              // lanes: RG groups of rows (row = i * RG + rg) by KG groups of keys
   constexpr int NK = AF_CHUNK / KG;                       // keys a lane: kg + KG * j
   constexpr int DPL = HD / KG, VW = DPL < 4 ? DPL : 4, NV = DPL / VW;      // dimensions a lane: NV runs of VW
   static_assert(VW == 2 || VW == 4, "a lane's run of dimensions is a vector");
-  constexpr int KS = HD + 4, PS = AF_CHUNK + 4;
+  constexpr int KS = HD + 4, VS = SHARED ? KS : HD, PS = AF_CHUNK + 4;
   extern __shared__ __align__(16) float af_smem_area[];
   float* Qs = af_smem_area;                               // [ROWS][KS], scaled
   __shared__ float s_max[WARPS][ROWS], s_sum[WARPS][ROWS];
   __shared__ int s_pos[ROWS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rg = lane / KG, kg = lane % KG;
-  float* Ks = af_smem_area + ROWS * KS + warp * af_warp_floats<HD, ROWS>();
-  float* Vs = Ks + AF_CHUNK * KS;
-  float* Ps = Vs + AF_CHUNK * HD;
+  float* Ks = af_smem_area + ROWS * KS + warp * af_warp_floats<HD, ROWS, SHARED>();
+  float* Vs = SHARED ? Ks : Ks + AF_CHUNK * KS;
+  float* Ps = Vs + AF_CHUNK * VS;
   const int g = blockIdx.y, hpg = a.H / a.G;
   const int tile = gridDim.x - 1 - blockIdx.x;            // a prompt's last tokens have the most keys: they start first
   const int m0 = tile * a.tokens, tokens = min(a.tokens, a.M - m0), rows = tokens * hpg;
@@ -121,8 +127,12 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
     };
     fetch(Ks, KS, a.k_pool, warp);
     for (int c = warp; c < chunks; c += WARPS) {
-      fetch(Vs, HD, a.v_pool, c);
-      af_wait<1>();                                       // this chunk's keys
+      if constexpr (SHARED) {
+        af_wait<0>();                                     // this chunk's keys
+      } else {
+        fetch(Vs, VS, a.v_pool, c);
+        af_wait<1>();
+      }
       __syncwarp();
       float s[4][NK];
 #pragma unroll
@@ -155,7 +165,8 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
           for (int j = 0; j < NK; ++j) s[i][j] += part[i][j];
       }
       __syncwarp();                                       // every lane has read the keys
-      fetch(Ks, KS, a.k_pool, c + WARPS);
+      if constexpr (SHARED) fetch(Vs, VS, a.v_pool, c);
+      else fetch(Ks, KS, a.k_pool, c + WARPS);
       bool whole = true;                                  // every row of this lane sees every key of the chunk
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -183,7 +194,8 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
           for (int e = 0; e < VW; ++e) acc[i][n][e] *= corr;
       }
       whole = __all_sync(0xffffffffu, whole);
-      af_wait<1>();                                       // this chunk's values (the next one's keys may be on their way)
+      if constexpr (SHARED) af_wait<0>();                 // this chunk's values
+      else af_wait<1>();                                  // (the next one's keys may be on their way)
       __syncwarp();
       const int seen = min(AF_CHUNK, last + 1 - c * AF_CHUNK);
       for (int j0 = 0; j0 < seen; j0 += 4) {
@@ -198,7 +210,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
           float v[NV][VW];
 #pragma unroll
           for (int n = 0; n < NV; ++n) {
-            const float* src = Vs + (j0 + j) * HD + n * KG * VW + kg * VW;
+            const float* src = Vs + (j0 + j) * VS + n * KG * VW + kg * VW;
             if constexpr (VW == 4) {
               const float4 x = *reinterpret_cast<const float4*>(src);
               v[n][0] = x.x; v[n][1] = x.y; v[n][2] = x.z; v[n][3] = x.w;
@@ -221,6 +233,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
         }
       }
       __syncwarp();                                       // values and probabilities have been read by all
+      if constexpr (SHARED) fetch(Ks, KS, a.k_pool, c + WARPS);
     }
     af_wait<0>();
     __syncwarp();
@@ -255,7 +268,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
     for (int w = 0; w < WARPS; ++w) {
       const float wgt = s_max[w][r] > -INFINITY ? expf(s_max[w][r] - M) : s_sum[w][r];       // no keys: 0 (scores that are no numbers stay so)
       L = fmaf(s_sum[w][r], wgt, L);
-      const float4 x = *reinterpret_cast<const float4*>(O0 + w * af_warp_floats<HD, ROWS>() + r * HD + d);
+      const float4 x = *reinterpret_cast<const float4*>(O0 + w * af_warp_floats<HD, ROWS, SHARED>() + r * HD + d);
       o[0] = fmaf(x.x, wgt, o[0]); o[1] = fmaf(x.y, wgt, o[1]); o[2] = fmaf(x.z, wgt, o[2]); o[3] = fmaf(x.w, wgt, o[3]);
     }
     const float inv = 1.0f / L;
@@ -269,12 +282,12 @@ __global__ void __launch_bounds__(WARPS * 32) attention_f32_kernel(const AfArgs 
   }
 }
 
-template <int HD, int ROWS, int WARPS>
+template <int HD, int ROWS, int WARPS, bool SHARED>
 int af_launch(const AfArgs& a, cudaStream_t stream) {
-  constexpr int smem = af_smem<HD, ROWS, WARPS>();
-  static const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<HD, ROWS, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr int smem = af_smem<HD, ROWS, WARPS, SHARED>();
+  static const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<HD, ROWS, WARPS, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   RL_REQUIRE(e == cudaSuccess, "rl_attention_f32: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-  attention_f32_kernel<HD, ROWS, WARPS><<<dim3((a.M + a.tokens - 1) / a.tokens, a.G), WARPS * 32, smem, stream>>>(a);
+  attention_f32_kernel<HD, ROWS, WARPS, SHARED><<<dim3((a.M + a.tokens - 1) / a.tokens, a.G), WARPS * 32, smem, stream>>>(a);
   RL_LAUNCH_CHECK("rl_attention_f32");
   return RL_OK;
 }
@@ -308,12 +321,20 @@ extern "C" int rl_attention_f32(const float* q, int ldq, const float* k_pool, co
   const int rows = tokens * hpg;
   AfArgs a = {q, k_pool, v_pool, page_table, slot_of_token, positions, gate, sinks, out,
               ldq, max_pages, ldo, num_tokens, num_heads, num_kv_heads, sink, ldg, gate_per_head, tokens, scale, softcap};
+  // More CTAs than SMs: a warp's keys and values share an area, two CTAs run on an SM, and a warp that waits for its loads leaves the SM to
+  // the other CTA's (128 registers a thread at width 64, a few of 16 rows' spilled).  One B200, areas of their own against one: 32
+  // heads over 8 of 64, 500 tokens 99 / 80 us, 2,000 978 / 755, 64 single tokens behind 700 59 / 43; of 128: 200 / 132, 2,333 / 1,396,
+  // 115 / 71.  Just beyond the SMs: 152 CTAs of 76 tokens 14.9 / 12.4, of 19 single tokens behind 700 29.3 / 21.7 (8 heads over 8,
+  // 290 tokens: 20.0 / 21.3, 310: 21.1 / 23.5 - the CTAs behind the first wave are the shortest there - 500: 38.9 / 31.8).  With an SM
+  // for every CTA the second one never comes and the areas of their own win: 8 tokens behind 2,000 67.8 / 74.5.  The order of every
+  // sum is the same either way.
+  const bool many = (size_t)((num_tokens + tokens - 1) / tokens) * num_kv_heads > (size_t)rl_num_sms();
   if (head_dim == 64) {
-    if (rows <= 4) return af_launch<64, 4, 8>(a, stream);
-    if (rows <= 8) return af_launch<64, 8, 8>(a, stream);
-    return af_launch<64, 16, 8>(a, stream);
+    if (rows <= 4) return many ? af_launch<64, 4, 8, true>(a, stream) : af_launch<64, 4, 8, false>(a, stream);
+    if (rows <= 8) return many ? af_launch<64, 8, 8, true>(a, stream) : af_launch<64, 8, 8, false>(a, stream);
+    return many ? af_launch<64, 16, 8, true>(a, stream) : af_launch<64, 16, 8, false>(a, stream);
   }
-  if (rows <= 4) return af_launch<128, 4, 4>(a, stream);
-  if (rows <= 8) return af_launch<128, 8, 4>(a, stream);
-  return af_launch<128, 16, 4>(a, stream);
+  if (rows <= 4) return many ? af_launch<128, 4, 4, true>(a, stream) : af_launch<128, 4, 4, false>(a, stream);
+  if (rows <= 8) return many ? af_launch<128, 8, 4, true>(a, stream) : af_launch<128, 8, 4, false>(a, stream);
+  return many ? af_launch<128, 16, 4, true>(a, stream) : af_launch<128, 16, 4, false>(a, stream);
 }

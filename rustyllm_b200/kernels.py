@@ -698,7 +698,7 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
     if (q.dtype == torch.float32 and vd == head_dim and not (window or chunk or values_in_keys)
             and library().rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, out.stride(0), q.data_ptr(), out.data_ptr())):
         # 32-bit heads of 64 or 128 that see every position: tiles of rows that share a key (csrc/attention_f32.cu; 500 tokens of
-        # 32 heads of 64: 101 us against 914 with the any-shape kernel; four single tokens behind 96 to 700: 15.6 against 151)
+        # 32 heads of 64: 80 us against 914 with the any-shape kernel; four single tokens behind 96 to 700: 15.6 against 151)
         _check(library().rl_attention_f32(
             q.data_ptr(), ldq, k_pool.data_ptr(), v_pool.data_ptr(), page_table.data_ptr(), page_table.shape[1],
             slot_of_token.data_ptr(), positions.data_ptr(), out.data_ptr(), out.stride(0), M, num_heads, num_kv_heads, head_dim,

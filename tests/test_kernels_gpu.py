@@ -1261,6 +1261,23 @@ def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
     assert torch.equal(again[:keep], out[:keep]) and not torch.isfinite(again[keep:]).any()
 
 
+@pytest.mark.parametrize("H,G,hd", [(8, 8, 64), (48, 8, 64), (72, 8, 64), (8, 8, 128), (48, 8, 128), (72, 8, 128)])
+def test_attention_f32_single_tokens_do_not_depend_on_how_many_there_are(H, G, hd):
+    """18 sequences of 8 KV heads are fewer CTAs than a B200 has SMs, 19 are more (values then take the place of the keys), three
+    times as many put two CTAs on an SM: the float64 result, and the same bits as alone."""
+    k = K()
+    lens = [1 + 37 * i % 610 for i in range(57)]
+    q, kp, vp, pt, sot, pos, ref = _attention_case(torch.float32, H, G, hd, [1] * len(lens), lens, seed=H + hd)
+    outs = {}
+    for n in (1, 18, 19, 57):
+        outs[n] = torch.full((n, H * hd), math.nan, device=DEV)
+        k.attention_simt(q[-n:].contiguous(), kp, vp, pt, sot[-n:].contiguous(), pos[-n:].contiguous(), outs[n], H, G, hd,
+                         1.0 / math.sqrt(hd), single_tokens=True)
+    torch.testing.assert_close(outs[57].double().cpu(), ref, rtol=2e-5, atol=2e-5)
+    for n in (1, 18, 19):
+        assert torch.equal(outs[n], outs[57][-n:])
+
+
 @pytest.mark.parametrize("H,G,hd", [(8, 2, 64), (6, 1, 128)])
 @pytest.mark.parametrize("options", ["sink", "sinks", "gate", "head gate", "softcap"])
 def test_attention_f32_options_follow_the_any_shape_kernel(H, G, hd, options):
