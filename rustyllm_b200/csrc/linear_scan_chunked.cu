@@ -13,6 +13,10 @@
 // behind the loads is 32-bit as there; sums of logarithms are 64-bit, so that exp(L_i - L_j) is as exact for late tokens of a chunk as for early
 // ones.  Outputs of a position depend on where chunks begin, that is on how a sequence was cut into steps, to rounding.  Error against 64 bits
 // relative to the outputs' rms: 0.8e-7 to 1.8e-7, the walk's 0.7e-7 to 6.7e-7 (tests/test_kernels_gpu.py).
+//
+// Logarithms are for decays that fade: a in [0, 1], as every trained model's (mode 1 gives no others).  A head of mode 0 whose decay
+// lies outside (below 0; beyond 1, where exp(L_i - L_j) would leave float's range before the recurrence does; no number) is walked
+// token by token in the second kernel, with the walk's bits, and left out of the other two.
 #include <math.h>
 
 #include "common.cuh"
@@ -77,6 +81,9 @@ __device__ __forceinline__ bool ch_find(const ChunkArgs& a, int index, int& t0, 
   return false;
 }
 
+// whether the head's decays are taken by their logarithms
+__device__ __forceinline__ bool ch_fades(const ChunkArgs& a, int h) { return a.mode || (a.rate[h] >= 0.f && a.rate[h] <= 1.f); }
+
 // The chunk's sums of log a (64-bit) and step sizes b, by the first warp: two tokens a lane
 template <typename T>
 __device__ __forceinline__ void ch_decays(const ChunkArgs& a, int h, int t0, int nt, double* L, float* bsize) {
@@ -124,7 +131,7 @@ __global__ void __launch_bounds__(CH_THREADS) chunk_add_kernel(const ChunkArgs a
   rl_pdl_wait();
   const int h = blockIdx.x, tid = threadIdx.x;
   int t0, nt;
-  if (!ch_find(a, blockIdx.y, t0, nt)) return;
+  if (!ch_fades(a, h) || !ch_find(a, blockIdx.y, t0, nt)) return;
   const T *k = (const T*)a.k + (size_t)(h / a.hpg) * DK, *v = (const T*)a.v + (size_t)h * DV;
   ChRows<T, DK> kr;
   ChRows<T, DV> vr;
@@ -183,12 +190,55 @@ __global__ void __launch_bounds__(CH_THREADS) chunk_add_kernel(const ChunkArgs a
             make_float4(acc[s][e][u][0], acc[s][e][u][1], acc[s][e][u][2], acc[s][e][u][3]);
 }
 
+// Four consecutive rows of a column of a head's state over a sequence's tokens, DK / 4 neighbouring lanes a column: the order of every
+// sum is the walk's (linear_scan.cu, its shape for many tokens), so are the bits.  Eight tokens' values are on their way at once.
+template <typename T, int DK, int DV>
+__device__ __noinline__ void ch_walk_tokens(const ChunkArgs& a, int b, int h, int at) {
+  constexpr int R = DK / 4, AHEAD = 8;
+  const int col = at / DK, row = at % DK;
+  const T *q = (const T*)a.q + (size_t)(h / a.hpg) * DK + row, *k = (const T*)a.k + (size_t)(h / a.hpg) * DK + row;
+  const T* v = (const T*)a.v + (size_t)h * DV + col;
+  float* st = a.state + (size_t)a.seq_slots[b] * a.state_stride + (size_t)h * DK * DV + at;
+  const float decay = a.rate[h], skip = a.skip ? a.skip[h] : 0.f;
+  float4 S = *reinterpret_cast<const float4*>(st);
+  const int hi = a.cu_seqlens[b + 1];
+  for (int t0 = a.cu_seqlens[b]; t0 < hi; t0 += AHEAD) {
+    float4 qq[AHEAD], kk[AHEAD];
+    float vv[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const size_t t = min(t0 + i, hi - 1);
+      qq[i] = ch_ld4(q + t * a.ldq);
+      kk[i] = ch_ld4(k + t * a.ldk);
+      vv[i] = rl_ld(v + t * a.ldv);
+    }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      if (t0 + i >= hi) break;
+      const float4 x = ch_value<T>(qq[i], a.act), y = ch_value<T>(kk[i], a.act);
+      const float z = a.act ? ch_silu(vv[i], T()) : vv[i];
+      S = make_float4(fmaf(decay, S.x, z * y.x), fmaf(decay, S.y, z * y.y), fmaf(decay, S.z, z * y.z), fmaf(decay, S.w, z * y.w));
+      float p = fmaf(S.w, x.w, fmaf(S.z, x.z, fmaf(S.y, x.y, fmaf(S.x, x.x, 0.f))));
+#pragma unroll
+      for (int o = 1; o < R; o <<= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+      if (row == 0) a.out[(size_t)(t0 + i) * a.ldo + (size_t)h * DV + col] = p + skip * z;
+    }
+  }
+  *reinterpret_cast<float4*>(st) = S;
+}
+
 // ---------------- the walk: the state in front of every chunk in place of what the chunk adds ----------------
-__global__ void __launch_bounds__(256) chunk_walk_kernel(const ChunkArgs a, int size) {
+template <typename T, int DK, int DV>
+__global__ void __launch_bounds__(256) chunk_walk_kernel(const __grid_constant__ ChunkArgs a) {
   rl_pdl_trigger();
   rl_pdl_wait();
+  constexpr int size = DK * DV;
+  static_assert(size % 1024 == 0, "a block's 256 threads hold four elements each");
   const int b = blockIdx.x, h = blockIdx.y, at = ((int)blockIdx.z * 256 + (int)threadIdx.x) * 4;
-  if (at >= size) return;
+  if (!ch_fades(a, h)) {
+    ch_walk_tokens<T, DK, DV>(a, b, h, at);
+    return;
+  }
   int first = 0;
   for (int i = 0; i < b; ++i) first += (a.cu_seqlens[i + 1] - a.cu_seqlens[i] + CH - 1) / CH;
   const int chunks = (a.cu_seqlens[b + 1] - a.cu_seqlens[b] + CH - 1) / CH;
@@ -273,7 +323,7 @@ __global__ void __launch_bounds__(CH_THREADS, 2) chunk_out_kernel(const ChunkArg
   rl_pdl_wait();
   const int h = blockIdx.x, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   int t0, nt;
-  if (!ch_find(a, blockIdx.y, t0, nt)) return;
+  if (!ch_fades(a, h) || !ch_find(a, blockIdx.y, t0, nt)) return;
   const T *q = (const T*)a.q + (size_t)(h / a.hpg) * DK, *k = (const T*)a.k + (size_t)(h / a.hpg) * DK, *v = (const T*)a.v + (size_t)h * DV;
   {
     ChRows<T, DK> qr, kr;
@@ -383,7 +433,7 @@ int ch_launch(const ChunkArgs& a, int chunks, cudaStream_t stream) {
   static const cudaError_t e1 = cudaFuncSetAttribute(chunk_out_kernel<T, DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, out_smem);
   RL_REQUIRE(e0 == cudaSuccess && e1 == cudaSuccess, "rl_linear_scan_chunked: cannot reserve %d and %d bytes of shared memory", add_smem, out_smem);
   rl_launch_pdl(chunk_add_kernel<T, DK, DV>, dim3(a.H, chunks), dim3(CH_THREADS), (size_t)add_smem, stream, a);
-  rl_launch_pdl(chunk_walk_kernel, dim3(a.num_seqs, a.H, (DK * DV + 1023) / 1024), dim3(256), 0, stream, a, DK * DV);
+  rl_launch_pdl(chunk_walk_kernel<T, DK, DV>, dim3(a.num_seqs, a.H, DK * DV / 1024), dim3(256), 0, stream, a);
   rl_launch_pdl(chunk_out_kernel<T, DK, DV>, dim3(a.H, chunks), dim3(CH_THREADS), (size_t)out_smem, stream, a);
   RL_LAUNCH_CHECK("rl_linear_scan_chunked");
   return RL_OK;

@@ -1397,7 +1397,7 @@ def test_gemm_f32_few_is_more_exact_than_the_ordered_sum_and_rows_do_not_depend_
 
 
 # ----------------------------------------------------------------------------- linear recurrences by chunks
-def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed):
+def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed, decays=(0.9, 0.5, 0.999, 1.0, 0.0)):
     """Inputs as views of one wide buffer, states that are not zero, and the recurrence in float64 on what the kernel reads."""
     M, G = sum(lens), H // hpg
     g = torch.Generator(device=DEV).manual_seed(seed)
@@ -1406,7 +1406,7 @@ def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed):
     k, q, v = buf[:, :G * dk], buf[:, G * dk:2 * G * dk], buf[:, 2 * G * dk:2 * G * dk + H * dv]
     dt = buf[:, 2 * G * dk + H * dv:2 * G * dk + H * dv + H]
     dt_bias, skip = rand(H), rand(H)
-    rate = torch.tensor([0.9, 0.5, 0.999, 1.0, 0.0][:H] * H, device=DEV)[:H].contiguous() if mode == 0 else rand(H) * 2.0
+    rate = torch.tensor(list(decays)[:H] * H, device=DEV)[:H].contiguous() if mode == 0 else rand(H) * 2.0
     slots = list(range(len(lens) - 1, -1, -1))
     state = torch.zeros(len(lens) + 1, 4 * H * dk * dv + 256, dtype=torch.uint8, device=DEV)
     state.view(torch.float32).copy_(rand(len(lens) + 1, H * dk * dv + 64))
@@ -1489,3 +1489,35 @@ def test_linear_scan_by_chunks_keeps_later_tokens_out_of_earlier_outputs_and_tak
     assert ask(ok) == 5
     for bad in (dict(ptr=ok + 4), dict(ld=126), dict(st=4), dict(M=255), dict(M=319, B=10), dict(a=96), dict(b=32), dict(M=100_000)):
         assert ask(**{"ptr": ok, **bad}) == 0, bad
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 128), (128, 64), (64, 64)])
+def test_linear_scan_decays_that_do_not_fade(dtype, dk, dv):
+    """Decays below zero and beyond one (and no number) in steps of many tokens, beside heads whose decays fade: the walk's bits, and
+    float64 where the recurrence stays small."""
+    k = K()
+    decays = (-0.5, 0.9, -1.0, 1.01, 40.0, -3.0, math.nan, math.inf)
+    H, lens = len(decays), [70, 5, 1, 64, 200, 33]
+    qkv, state, cu, slots, rate, kw, ref, last = _scan_case(dtype, 0, H, 1, dk, dv, lens, seed=dk + dv, decays=decays)
+    state[2] = 0                     # a fresh sequence: zeros stay zeros whatever the growth in front of its first token
+    walked_state, before = state.clone(), state.clone()
+    walk = _scan_walk(k, qkv, walked_state, cu, slots, rate, kw, H, 1, dk, dv)
+    out = torch.empty_like(walk)
+    launches = k.launch_count
+    k.linear_scan(*qkv, out, state, cu, slots, H, 1, dk, dv, rate, **kw)
+    assert k.launch_count - launches == 3, "the chunked form"
+    n = 4 * H * dk * dv
+    heads = lambda x: x.view(-1, H, dv)
+    states = lambda x: x[:, :n].contiguous().view(torch.float32).view(-1, H, dv, dk)
+    for h, a in enumerate(decays):
+        if a != 0.9:
+            for x, y in ((heads(out)[:, h], heads(walk)[:, h]), (states(state)[:, h], states(walked_state)[:, h])):
+                assert torch.equal(torch.nan_to_num(x, nan=7e33), torch.nan_to_num(y, nan=7e33)), a
+        if abs(a) <= 1.01:
+            rows = torch.ones(sum(lens), dtype=torch.bool, device=DEV)
+            rows[sum(lens[:3]):sum(lens[:4])] = False        # (the sequence whose state was set to zero: slot 2)
+            x, y = heads(out)[rows, h].double(), heads(ref)[rows, h]
+            assert ((x - y).square().mean().sqrt() / y.square().mean().sqrt()).item() < 1e-6, a
+    assert torch.isfinite(heads(out)[:, :4]).all()
+    assert torch.equal(state[:, n:], before[:, n:]) and torch.equal(state[len(lens)], before[len(lens)])
