@@ -294,11 +294,12 @@ int af_launch(const AfArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
-// Whether the kernel takes these: heads of 64 or 128 (keys and values alike), up to 16 query heads a KV head, rows of q and out
-// that 16-byte pieces can fetch.
-extern "C" int rl_attention_f32_supported(int num_heads, int num_kv_heads, int head_dim, int ldq, int ldo, const void* q, const void* out) {
+// Whether the kernel takes these: heads of 64 or 128 (keys and values alike), up to 16 query heads a KV head, rows of q and out and
+// pools that 16-byte pieces can fetch.
+extern "C" int rl_attention_f32_supported(int num_heads, int num_kv_heads, int head_dim, int ldq, int ldo, const void* q, const void* k_pool,
+                                          const void* v_pool, const void* out) {
   return num_kv_heads > 0 && num_heads % num_kv_heads == 0 && num_heads / num_kv_heads <= 16 && (head_dim == 64 || head_dim == 128) &&
-         num_kv_heads <= 65535 && ldq % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
+         num_kv_heads <= 65535 && ldq % 4 == 0 && ldo % 4 == 0 && (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15) == 0;
 }
 
 // q: float [M, ldq] with head h at columns [h * hd, (h + 1) * hd); out likewise, [M, ldo].  Pools: float [pages, G, RL_PAGE, hd].
@@ -309,8 +310,8 @@ extern "C" int rl_attention_f32(const float* q, int ldq, const float* k_pool, co
                                 int num_kv_heads, int head_dim, float scale, int sink, const float* gate, int ldg, float softcap,
                                 int gate_per_head, const float* sinks, int single_tokens, cudaStream_t stream) {
   RL_REQUIRE(num_tokens >= 0 && num_heads > 0 && num_kv_heads > 0 && max_pages > 0 && softcap >= 0.f, "rl_attention_f32: bad sizes");
-  RL_REQUIRE(rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, ldo, q, out),
-             "rl_attention_f32: %d heads over %d KV heads of %d, or rows 16-byte pieces cannot fetch", num_heads, num_kv_heads, head_dim);
+  RL_REQUIRE(rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, ldo, q, k_pool, v_pool, out),
+             "rl_attention_f32: %d heads over %d KV heads of %d, or rows or pools 16-byte pieces cannot fetch", num_heads, num_kv_heads, head_dim);
   RL_REQUIRE(ldq >= num_heads * head_dim && ldo >= num_heads * head_dim, "rl_attention_f32: row strides too small");
   RL_REQUIRE(gate == nullptr || ldg >= (gate_per_head ? num_heads : num_heads * head_dim), "rl_attention_f32: the gate's row stride is too small");
   if (num_tokens == 0) return RL_OK;

@@ -78,7 +78,7 @@ _SIGNATURES = {
                                _c_void_p, _c_void_p],
     "rl_rope_kv_write": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p,
                          _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
-    "rl_attention_f32_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "rl_attention_f32_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "rl_attention_f32": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                          _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_int, _c_float, _c_int, _c_void_p, _c_int, _c_void_p],
     "rl_attention_simt": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p,
@@ -696,7 +696,8 @@ def attention_simt(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, 
         assert gate.shape == (M, num_heads if gate_per_head else num_heads * vd) and gate.stride(1) == 1
         ldg = gate.stride(0) if M > 1 else gate.shape[1]
     if (q.dtype == torch.float32 and vd == head_dim and not (window or chunk or values_in_keys)
-            and library().rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, out.stride(0), q.data_ptr(), out.data_ptr())):
+            and library().rl_attention_f32_supported(num_heads, num_kv_heads, head_dim, ldq, out.stride(0), q.data_ptr(), k_pool.data_ptr(),
+                                                     v_pool.data_ptr(), out.data_ptr())):
         # 32-bit heads of 64 or 128 that see every position: tiles of rows that share a key (csrc/attention_f32.cu; 500 tokens of
         # 32 heads of 64: 80 us against 914 with the any-shape kernel; four single tokens behind 96 to 700: 15.6 against 151)
         _check(library().rl_attention_f32(

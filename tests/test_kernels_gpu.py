@@ -1295,6 +1295,24 @@ def test_attention_f32_options_follow_the_any_shape_kernel(H, G, hd, options):
     torch.testing.assert_close(out, plain, rtol=1e-5, atol=4e-6)
 
 
+@pytest.mark.parametrize("shifted", [(0, 1), (1, 0), (1, 1)])
+def test_attention_f32_pools_that_16_byte_pieces_cannot_fetch(shifted):
+    """Contiguous pools that begin 4 bytes behind a 16-byte boundary go to the any-shape kernel, whose loads are single elements."""
+    k = K()
+    H, G, hd, lens = 8, 2, 64, [40, 1, 130]
+    q, kp, vp, pt, sot, pos, ref = _attention_case(torch.float32, H, G, hd, lens, lens, seed=9)
+    pools = []
+    for x, s in zip((kp, vp), shifted):
+        room = torch.zeros(x.numel() + 4, device=DEV)
+        pools.append(room[s:s + x.numel()].view(x.shape).copy_(x))
+    args = (H, G, hd, q.stride(0), H * hd, q.data_ptr())
+    assert k.library().rl_attention_f32_supported(*args, kp.data_ptr(), vp.data_ptr(), q.data_ptr()) == 1
+    assert k.library().rl_attention_f32_supported(*args, pools[0].data_ptr(), pools[1].data_ptr(), q.data_ptr()) == 0
+    out = torch.empty_like(q)
+    k.attention_simt(q, *pools, pt, sot, pos, out, H, G, hd, 1.0 / math.sqrt(hd))
+    torch.testing.assert_close(out.double().cpu(), ref, rtol=2e-5, atol=2e-5)
+
+
 # ----------------------------------------------------------------------------- 32-bit products from bf16 cuts
 def _f32_split(k, a, w, bias=None, parts=0):
     out = torch.empty(a.shape[0], w.shape[0], device=DEV)
