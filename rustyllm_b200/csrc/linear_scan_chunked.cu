@@ -450,10 +450,9 @@ constexpr long long CH_WORK_LIMIT = 768LL << 20;       // bytes of work a call m
 }  // namespace
 
 // Chunks that the chunked form of a step of num_tokens tokens is launched for (its work: chunks * heads * (dk * dv + 1) floats), or 0 where the
-// walk of rl_linear_scan is the way: state widths other than 64 and 128, rows that pieces of four elements cannot fetch, fewer than
-// 256 tokens or 32 a sequence (three kernels take some 60 us however little there is: 16 heads of 128 x 128, 128 tokens of one sequence 59
-// us against 43, 256 tokens 56 against 83; 4 sequences of 32 tokens 53 against 45, 8 of 32 tokens 61 against 76, 4 of 64 tokens 65 against
-// 84), or more work than 768 MiB (some 24,000 tokens of 32 such heads).
+// form does not take the step: state widths other than 64 and 128, rows that pieces of four elements cannot fetch, fewer than 256 tokens or 32
+// a sequence (16 heads of 128 x 128, one sequence, walk / chunks: 128 tokens 43 / 59 us, 256 tokens 83 / 56), or more work than 768 MiB (some
+// 24,000 tokens of 32 such heads).  Whether a step that it takes is worth it is for the caller (scan_chunks_pay in kernels.py).
 extern "C" int rl_linear_scan_chunks(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, int dtype, const void* state,
                                      long long state_stride, int num_tokens, int num_seqs, int num_heads, int dk, int dv) {
   if ((dk != 64 && dk != 128) || (dv != 64 && dv != 128) || num_seqs <= 0 || num_tokens < 256 || num_tokens < 32LL * num_seqs) return 0;

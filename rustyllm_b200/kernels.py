@@ -1132,15 +1132,27 @@ def heads_linear(x: torch.Tensor, x_head: int, w: torch.Tensor, out: torch.Tenso
     _count()
 
 
+def scan_chunks_pay(num_tokens: int, longest: int, num_heads: int, dk: int, dv: int, dtype: torch.dtype) -> bool:
+    """Whether a recurrence over many tokens is worth its chunked form (csrc/linear_scan_chunked.cu): three kernels that take at
+    least 23 us for states of 64 x 64, 33 with one width of 128 and 48 with two, a quarter more in 32-bit (1 to 7 sequences, 2 to 8 heads).  The walk
+    takes a quarter of a microsecond a token of the longest sequence, or 1 us for 0.85 million multiply-adds of all.  One B200, bfloat16, walk / chunks:
+    4 heads of 128 x 128, 4 sequences of 64 tokens 22.8 / 56.1, 16 of 33 53.6 / 57.9, 2 of 200 64.0 / 59.0, 32 of 32 76.2 / 68.0; 8 heads of
+    64 x 64, 8 of 64 21.7 / 28.6, 3 of 100 30.5 / 24.9; 16 heads of 128 x 128, 8 of 32 76.0 / 62.8."""
+    walk = max(0.25 * longest, num_tokens * num_heads * dk * dv / 0.85e6)
+    least = 23.0 if dk == dv == 64 else 48.0 if dk == dv == 128 else 33.0
+    return walk >= (least if dtype == torch.bfloat16 else 1.25 * least)
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                 cu_seqlens: torch.Tensor, seq_slots: torch.Tensor, num_heads: int, heads_per_group: int, dk: int, dv: int,
                 rate: torch.Tensor, dt_raw: Optional[torch.Tensor] = None, dt_bias: Optional[torch.Tensor] = None,
-                skip: Optional[torch.Tensor] = None, silu: bool = False) -> None:
+                skip: Optional[torch.Tensor] = None, silu: bool = False, longest: int = 0) -> None:
     """S_t = a_t S_{t-1} + b_t k_t v_t^T, out_t = S_t^T q_t (+ skip[h] v_t) for every head of every sequence of the
     step, the state (float [H, dv, dk] a slot) read from and left in ``state``.  Without ``dt_raw``: a_t = rate[h],
     b_t = 1.  With it: dt = softplus(dt_raw[t, h] + dt_bias[h]), a_t = exp(-exp(rate[h]) * dt), b_t = dt.  q, k
     [M, (H / heads_per_group) * dk], v [M, H * dv] (views are fine), out float32 [M, H * dv].  ``silu``: q, k and v
-    pass through silu first."""
+    pass through silu first.  ``longest``: tokens of the longest sequence (0: not known, taken as twice the mean): the kernel is chosen
+    by the step's sizes, so a position's bits depend on the step that it came in; between any two choices they differ by rounding."""
     for t, name in ((q, "q"), (k, "k"), (v, "v")):
         _need(t, name, q.dtype, contiguous=False)
         assert t.stride(1) == 1
@@ -1159,8 +1171,10 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Te
         assert skip.numel() == num_heads
     sp, ss = _state_args(state)
     assert state.shape[1] >= 4 * num_heads * dk * dv
-    chunks = library().rl_linear_scan_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _dt(q), sp, ss,
-                                             M, seq_slots.numel(), num_heads, dk, dv)
+    chunks, num_seqs = 0, seq_slots.numel()
+    if M >= 32 * num_seqs and scan_chunks_pay(M, longest or min(M, -(-2 * M // max(num_seqs, 1))), num_heads, dk, dv, q.dtype):
+        chunks = library().rl_linear_scan_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _dt(q), sp, ss,
+                                                 M, num_seqs, num_heads, dk, dv)
     if chunks:      # many tokens: products a chunk of 64 instead of a walk (csrc/linear_scan_chunked.cu)
         work = torch.empty(chunks * num_heads * (dk * dv + 1), dtype=torch.float32, device=out.device)
         _check(library().rl_linear_scan_chunked(

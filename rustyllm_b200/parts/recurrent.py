@@ -94,7 +94,8 @@ class DecayLinearAttention(_StateMixer):
         q, k = proj[:, :H * dk], proj[:, H * dk:2 * H * dk]
         v, g = proj[:, 2 * H * dk:2 * H * dk + H * dv], proj[:, 2 * H * dk + H * dv:]
         o = torch.empty((M, H * dv), dtype=torch.float32, device=xn.device)
-        K.linear_scan(q, k, v, o, state, step.cu_seqlens, step.seq_slots, H, 1, dk, dv, self.decay, silu=True)
+        K.linear_scan(q, k, v, o, state, step.cu_seqlens, step.seq_slots, H, 1, dk, dv, self.decay, silu=True,
+                      longest=step.max_q_len)
         on = torch.empty((M, H * dv), dtype=xn.dtype, device=xn.device)
         K.gated_norm(o, g, self.norm_w, self.eps, on, groups=1, gate_act="sigmoid", gate_first=False)
         linear(on, self.wo, residual, _out_mode)
@@ -157,7 +158,7 @@ class SelectiveStateSpace(_StateMixer):
         x, b, c = xbc[:, :inner], xbc[:, inner:inner + G * N], xbc[:, inner + G * N:]
         y = torch.empty((M, inner), dtype=torch.float32, device=xn.device)
         K.linear_scan(c, b, x, y, scan_state, step.cu_seqlens, step.seq_slots, H, H // G, N, P, self.a_log,
-                      dt_raw=dt, dt_bias=self.dt_bias, skip=self.skip)
+                      dt_raw=dt, dt_bias=self.dt_bias, skip=self.skip, longest=step.max_q_len)
         yn = torch.empty((M, inner), dtype=xn.dtype, device=xn.device)
         K.gated_norm(y, z, self.norm_w, self.eps, yn, groups=self.norm_groups, gate_act="silu", gate_first=True)
         linear(yn, self.wo, residual, _out_mode)

@@ -1516,14 +1516,14 @@ def test_linear_scan_decays_that_do_not_fade(dtype, dk, dv):
     float64 where the recurrence stays small."""
     k = K()
     decays = (-0.5, 0.9, -1.0, 1.01, 40.0, -3.0, math.nan, math.inf)
-    H, lens = len(decays), [70, 5, 1, 64, 200, 33]
+    H, lens = len(decays), [70, 5, 1, 64, 260, 33]
     qkv, state, cu, slots, rate, kw, ref, last = _scan_case(dtype, 0, H, 1, dk, dv, lens, seed=dk + dv, decays=decays)
     state[2] = 0                     # a fresh sequence: zeros stay zeros whatever the growth in front of its first token
     walked_state, before = state.clone(), state.clone()
     walk = _scan_walk(k, qkv, walked_state, cu, slots, rate, kw, H, 1, dk, dv)
     out = torch.empty_like(walk)
     launches = k.launch_count
-    k.linear_scan(*qkv, out, state, cu, slots, H, 1, dk, dv, rate, **kw)
+    k.linear_scan(*qkv, out, state, cu, slots, H, 1, dk, dv, rate, longest=260, **kw)
     assert k.launch_count - launches == 3, "the chunked form"
     n = 4 * H * dk * dv
     heads = lambda x: x.view(-1, H, dv)
@@ -1539,3 +1539,24 @@ def test_linear_scan_decays_that_do_not_fade(dtype, dk, dv):
             assert ((x - y).square().mean().sqrt() / y.square().mean().sqrt()).item() < 1e-6, a
     assert torch.isfinite(heads(out)[:, :4]).all()
     assert torch.equal(state[:, n:], before[:, n:]) and torch.equal(state[len(lens)], before[len(lens)])
+
+
+@pytest.mark.parametrize("dtype,H,dk,dv,lens,longest,chunked", [
+    (torch.bfloat16, 4, 128, 128, [64] * 4, 64, False), (torch.bfloat16, 2, 128, 128, [100] * 3, 100, False),
+    (torch.bfloat16, 4, 128, 128, [33] * 16, 33, False), (torch.bfloat16, 4, 128, 128, [32] * 32, 32, True),
+    (torch.bfloat16, 2, 128, 128, [256], 256, True), (torch.bfloat16, 8, 64, 64, [64] * 8, 64, False),
+    (torch.bfloat16, 2, 64, 64, [100] * 3, 100, True), (torch.bfloat16, 4, 64, 128, [200, 33, 33, 33], 200, True),
+    (torch.bfloat16, 4, 64, 128, [75] * 4, 75, False), (torch.float32, 4, 128, 64, [40] * 8, 40, False),
+    (torch.bfloat16, 2, 64, 64, [200, 33, 33], 0, True), (torch.bfloat16, 2, 128, 128, [1] * 300, 1, False)])
+def test_linear_scan_takes_chunks_where_there_is_enough_to_do(dtype, H, dk, dv, lens, longest, chunked):
+    """Few heads and short sequences keep the walk, whose chain is shorter than three kernels; the result is the same to rounding."""
+    k = K()
+    qkv, state, cu, slots, rate, kw, ref, _ = _scan_case(dtype, 0, H, 1, dk, dv, lens, seed=11)
+    walk = _scan_walk(k, qkv, state.clone(), cu, slots, rate, kw, H, 1, dk, dv)
+    out, launches = torch.empty_like(walk), k.launch_count
+    k.linear_scan(*qkv, out, state, cu, slots, H, 1, dk, dv, rate, longest=longest, **kw)
+    assert k.launch_count - launches == (3 if chunked else 1)
+    rel = lambda x: ((x.double() - ref).square().mean().sqrt() / ref.square().mean().sqrt()).item()
+    assert rel(out) <= rel(walk) + 1e-7
+    if not chunked and len(lens) * 4 <= sum(lens):
+        assert torch.equal(out, walk)
