@@ -1143,6 +1143,14 @@ def scan_chunks_pay(num_tokens: int, longest: int, num_heads: int, dk: int, dv: 
     return walk >= (least if dtype == torch.bfloat16 else 1.25 * least)
 
 
+def _scan_work(floats: int, device: torch.device) -> Optional[torch.Tensor]:
+    """Room for a chunked recurrence's states (up to 768 MiB), or None where a cache has left too little: the walk needs none."""
+    try:
+        return torch.empty(floats, dtype=torch.float32, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor, state: torch.Tensor,
                 cu_seqlens: torch.Tensor, seq_slots: torch.Tensor, num_heads: int, heads_per_group: int, dk: int, dv: int,
                 rate: torch.Tensor, dt_raw: Optional[torch.Tensor] = None, dt_bias: Optional[torch.Tensor] = None,
@@ -1175,8 +1183,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Te
     if M >= 32 * num_seqs and scan_chunks_pay(M, longest or min(M, -(-2 * M // max(num_seqs, 1))), num_heads, dk, dv, q.dtype):
         chunks = library().rl_linear_scan_chunks(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _dt(q), sp, ss,
                                                  M, num_seqs, num_heads, dk, dv)
-    if chunks:      # many tokens: products a chunk of 64 instead of a walk (csrc/linear_scan_chunked.cu)
-        work = torch.empty(chunks * num_heads * (dk * dv + 1), dtype=torch.float32, device=out.device)
+    work = _scan_work(chunks * num_heads * (dk * dv + 1), out.device) if chunks else None
+    if work is not None:      # many tokens: products a chunk of 64 instead of a walk (csrc/linear_scan_chunked.cu)
         _check(library().rl_linear_scan_chunked(
             q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), _ptr(dt_raw), lddt, _dt(q), _ptr(dt_bias),
             rate.data_ptr(), _ptr(skip), mode, int(bool(silu)), cu_seqlens.data_ptr(), seq_slots.data_ptr(), seq_slots.numel(), sp, ss,

@@ -1560,3 +1560,21 @@ def test_linear_scan_takes_chunks_where_there_is_enough_to_do(dtype, H, dk, dv, 
     assert rel(out) <= rel(walk) + 1e-7
     if not chunked and len(lens) * 4 <= sum(lens):
         assert torch.equal(out, walk)
+
+
+def test_linear_scan_walks_where_memory_is_short(monkeypatch):
+    """A cache that has left no room for the chunked form's states: the step is walked, as it is below 256 tokens."""
+    k = K()
+    H, dk, dv = 2, 128, 128
+    qkv, state, cu, slots, rate, kw, _, _ = _scan_case(torch.bfloat16, 0, H, 1, dk, dv, [300], seed=12)
+    walk = _scan_walk(k, qkv, state.clone(), cu, slots, rate, kw, H, 1, dk, dv)
+    out, launches, plain = torch.empty_like(walk), k.launch_count, torch.empty
+
+    def no_room(*size, **options):
+        if size and isinstance(size[0], int) and size[0] >= 5 * H * dk * dv:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return plain(*size, **options)
+    monkeypatch.setattr(torch, "empty", no_room)
+    k.linear_scan(*qkv, out, state, cu, slots, H, 1, dk, dv, rate, longest=300, **kw)
+    monkeypatch.undo()
+    assert k.launch_count - launches == 1 and torch.equal(out, walk)
