@@ -53,7 +53,7 @@ gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, c
   for (int u = 0; u < U; ++u)
 #pragma unroll
     for (int r = 0; r < R; ++r) fetch(r, u, u);
-  rl_pdl_wait();                             // weights are written by no kernel of a step, the tokens' rows are
+  rl_pdl_wait();                             // a weight is written by no kernel of a step (where W is none, see few_launch), the tokens' rows are
   const float* A = rl_behind_wait(const_cast<float*>(A_));
   float* out = rl_behind_wait(out_);
   auto fill = [&](int i) {
@@ -137,10 +137,17 @@ gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, c
 }
 
 template <int R, int MT>
-int few_launch(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo, cudaStream_t stream) {
+int few_launch(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo, int early,
+               cudaStream_t stream) {
   const int rows = R * FEW_WARPS;
-  const cudaError_t e = rl_launch_pdl(gemm_f32_few_kernel<R, MT, 16 / R>, dim3((N + rows - 1) / rows), dim3(FEW_WARPS * 32), 0, stream, A, W, bias, out,
-                                      add, M, N, K, lda, ldo);
+  const dim3 grid((N + rows - 1) / rows), block(FEW_WARPS * 32);
+  cudaError_t e;
+  if (early) {
+    e = rl_launch_pdl(gemm_f32_few_kernel<R, MT, 16 / R>, grid, block, 0, stream, A, W, bias, out, add, M, N, K, lda, ldo);
+  } else {           // launched the ordinary way the kernel begins when all in front of it have ended
+    gemm_f32_few_kernel<R, MT, 16 / R><<<grid, block, 0, stream>>>(A, W, bias, out, add, M, N, K, lda, ldo);
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_f32_few: %s", cudaGetErrorString(e));
     return RL_ERR_CUDA;
@@ -158,14 +165,15 @@ extern "C" int rl_gemm_f32_few_supported(const void* A, const void* W, int M, in
 }
 
 // A: float [M, K], row stride lda; W: float [N, K] contiguous; out: float [M, N], row stride ldo; add != 0: added into out.
+// early != 0: W is a weight, which no kernel that may still run writes, so it may be read before the kernels in front have ended.
 extern "C" int rl_gemm_f32_few(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo,
-                               cudaStream_t stream) {
+                               int early, cudaStream_t stream) {
   RL_REQUIRE(rl_gemm_f32_few_supported(A, W, M, N, K, lda) && ldo >= N, "rl_gemm_f32_few: operands not supported (M=%d N=%d K=%d lda=%d ldo=%d)", M, N,
              K, lda, ldo);
   // Four rows a warp halve the tokens' loads a weight row; two leave more warps to stream where rows are few.  Four tokens, two / four rows:
   // 2,048 rows of 8,192 19.4 / 22.3 us, 3,072 of 2,048 7.2 / 8.3, 16,384 of 2,048 30.6 / 26.3, 128,256 of 2,048 189 / 162.
   const bool four = N >= 32 * rl_num_sms();
-#define FEW_GO(MT) (four ? few_launch<4, MT>(A, W, bias, out, add, M, N, K, lda, ldo, stream) : few_launch<2, MT>(A, W, bias, out, add, M, N, K, lda, ldo, stream))
+#define FEW_GO(MT) (four ? few_launch<4, MT>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream) : few_launch<2, MT>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream))
   if (M == 1) return FEW_GO(1);
   if (M == 2) return FEW_GO(2);
   if (M <= 4) return FEW_GO(4);

@@ -46,7 +46,7 @@ _SIGNATURES = {
     "rl_gemm_f32_split": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int,
                           _c_void_p],
     "rl_gemm_f32_few_supported": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int],
-    "rl_gemm_f32_few": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
+    "rl_gemm_f32_few": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "rl_linear_scan_chunks": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_int, _c_int, _c_int,
                               _c_int, _c_int],
     "rl_linear_scan_chunked": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p,
@@ -581,10 +581,11 @@ def random_fill(out: torch.Tensor, seed: int, mean: float, std: float) -> None:
 
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int,
-              bias: Optional[torch.Tensor] = None) -> None:
+              bias: Optional[torch.Tensor] = None, is_weight: bool = False) -> None:
     """out = a @ w.T (+ bias) of float or bf16 operands of any shape, float sums, on the CUDA cores; float operands of more
-    than 8 rows by ``gemm_f32_split`` and of up to 8 by csrc/gemm_f32_few.cu where they take them.  a: [M, K] (rows may be strided), w: [N, K] contiguous, same
-    dtype.  out_mode: OUT_SAME / OUT_F32 / OUT_ADD_F32."""
+    than 8 rows by ``gemm_f32_split`` and of up to 8 by csrc/gemm_f32_few.cu where they take them.  a: [M, K] (rows may be strided),
+    w: [N, K] contiguous, same dtype.  out_mode: OUT_SAME / OUT_F32 / OUT_ADD_F32.  ``is_weight``: ``w`` is a model's weight, which no
+    kernel of a step writes; it may then be read while the kernels in front still run."""
     _need(a, "a", contiguous=False); _need(w, "w", a.dtype); _need(out, "out", contiguous=False)
     M, K = a.shape
     N = w.shape[0]
@@ -604,7 +605,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int
         return
     if a.dtype == torch.float32 and library().rl_gemm_f32_few_supported(a.data_ptr(), w.data_ptr(), M, N, K, lda):
         _check(library().rl_gemm_f32_few(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), int(out_mode == OUT_ADD_F32), M, N, K, lda,
-                                         ldo, _stream()), "rl_gemm_f32_few")
+                                         ldo, int(bool(is_weight)), _stream()), "rl_gemm_f32_few")
         _count()
         return
     _check(library().rl_gemm_simt(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _dt(a), out_mode,

@@ -70,12 +70,12 @@ def linear(a: Union[torch.Tensor, NormedInput], weight: torch.Tensor, out: torch
         K.convert(a.contiguous(), a32)
         if out_mode == OUT_SAME:
             tmp = torch.empty(out.shape, dtype=torch.float32, device=a.device)
-            K.gemm_simt(a32, weight, tmp, OUT_F32, bias)
+            K.gemm_simt(a32, weight, tmp, OUT_F32, bias, is_weight=True)
             K.convert(tmp, out)
         else:
-            K.gemm_simt(a32, weight, out, out_mode, bias)
+            K.gemm_simt(a32, weight, out, out_mode, bias, is_weight=True)
         return
     if a.dtype == torch.bfloat16 and K.gemm_tc_supported(a, weight, out):
         K.gemm_tc(a, weight, out, out_mode, bias)
     else:
-        K.gemm_simt(a, weight, out, out_mode, bias)
+        K.gemm_simt(a, weight, out, out_mode, bias, is_weight=True)

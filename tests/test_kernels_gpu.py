@@ -1414,6 +1414,25 @@ def test_gemm_f32_few_is_more_exact_than_the_ordered_sum_and_rows_do_not_depend_
         assert not lib.rl_gemm_f32_few_supported(w.data_ptr(), w.data_ptr(), M, N, kk, lda)
 
 
+def test_gemm_f32_few_waits_for_a_second_operand_that_was_just_written():
+    """An operand that a kernel in front has only begun to write (it lets the next kernel start early) is no weight: the product by the
+    default call is the one of what was written.  Operands of 64 MB, so that the writing takes longer than the product's start."""
+    k = K()
+    N, K_ = 8192, 2048
+    a, x, ones = _rand(2, K_, seed=1), _rand(N, K_, seed=2), torch.ones(K_, device=DEV)
+    w, out = torch.zeros(N, K_, device=DEV), torch.empty(2, N, device=DEV)
+    for i in range(8):
+        x.add_(1.0)
+        k.rmsnorm(x, ones, w, 1e-5)
+        k.gemm_simt(a, w, out, k.OUT_F32)
+        torch.cuda.synchronize()
+        for is_weight in (False, True):
+            again = torch.empty_like(out)
+            k.gemm_simt(a, w, again, k.OUT_F32, is_weight=is_weight)
+            assert torch.equal(again, out)
+        w.zero_()
+
+
 # ----------------------------------------------------------------------------- linear recurrences by chunks
 def _scan_case(dtype, mode, H, hpg, dk, dv, lens, seed, decays=(0.9, 0.5, 0.999, 1.0, 0.0)):
     """Inputs as views of one wide buffer, states that are not zero, and the recurrence in float64 on what the kernel reads."""
