@@ -1,26 +1,29 @@
-// out[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) for float operands and more than 64 rows, on the tensor cores without
+// out[M, N] = A[M, K] * W[N, K]^T (+ bias[N]) for float operands and more than 8 rows, on the tensor cores without
 // giving up float's accuracy.
 //
-// A float is the exact sum of three bf16 numbers, its significand cut into runs of eight bits (x = h + m + l, by truncation,
-// so nothing overflows on the way).  The product of two floats is taken as h h' + (h m' + m h') + (h l' + m m' + l h'); what is
-// left out (m l', l m', l l') is below 2^-23 of the product.  bf16 products are exact in the tensor core's float accumulators;
-// those are only trusted with 64 values of k at a time - h h' in one accumulator, the small terms in another, so that they
-// are not rounded against the large ones - and are then added to sums in registers, rounded to nearest.  The error against 64 bits
+// A float is the exact sum of three bf16 numbers: x = h + m + l, h the bf16 nearest to x, m the one nearest to what is left (below
+// 2^-8 of x's power of two), l the rest (below 2^-17).  The product of two floats is taken as h h' + (h m' + m h') + (h l' + m m' + l h');
+// what is left out (m l', l m', l l'; with tiles of up to 64 tokens m l' is in) is below 2^-24 of the product, of either sign: half a unit
+// in the last place, a float rounding.  (Cut by truncation the residuals are twice as large and have the operand's sign: up to
+// 2^-21 is left out, always towards zero.)  bf16 products are exact in the tensor core's float accumulators;
+// those are only trusted with 64 values of k at a time, in every block of columns the smaller terms first, and are then added to
+// sums in registers, rounded to nearest.  The error against 64 bits
 // is smaller than that of the k-ordered sum it replaces (rms over the rms of the result, K = 2,048 / 8,192: 1.6e-7 / 2.0e-7
-// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that).
+// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-22).
 //
 // What bounds it: shared memory.  Per 64 values of k a tile of 128 x 128 takes 24 products of 128 x 128 x 16 (1,536 clocks of the
 // tensor pipe), which read 192 KB of operands, and the cutting warps write 96 KB.  The register tile on the CUDA cores
-// that this replaces (gemm_simt_big_kernel) reached 14 to 47 TFLOP/s.  500 tokens, 2,048 -> 16,384: 237 us (142 TFLOP/s)
-// against 828; 8,192 -> 2,048: 116 against 1,232.
+// that this replaces (gemm_simt_big_kernel) reached 14 to 47 TFLOP/s.  500 tokens, 2,048 -> 16,384: 235 us (143 TFLOP/s)
+// against 828; 8,192 -> 2,048: 122 against 1,232.
 //
-// Roles in a CTA of 16 warps: fifteen fetch floats from global memory (the next block's loads are in flight while this block is
-// cut) and write the three bf16 tiles of both operands in the tensor core's swizzled layout; one thread issues the products;
-// eight of the fifteen also add the accumulators to their registers and store.  Few tiles: the K range of a tile is cut over a cluster of
-// 2, 4 or 8 CTAs, added in order through distributed shared memory.
+// Roles in a CTA: eight warps fetch floats from global memory (the next block's loads are in flight while this block is
+// cut) and write the three bf16 tiles of both operands in the tensor core's swizzled layout; eight warps (four for tiles of up to 64
+// tokens) add the accumulators to their registers and store; one thread issues the products: of the first summing warp, or of a warp of
+// its own for tiles of up to 64 tokens.  Few tiles: the K range of a tile is cut over a cluster of
+// 2 or 4 CTAs, added in order through distributed shared memory.
 //
-// Infinities and NaNs do not survive the cutting (inf - inf), so an output that is no finite number is computed again, alone
-// and in the order of k, by the plain sum.
+// Infinities and NaNs do not survive the cutting (inf - inf), and floats above the largest bf16 (3.39e38) are rounded to infinity, so an
+// output that is no finite number is computed again, alone and in the order of k, by the plain sum.
 #include "tc_device.cuh"
 
 namespace {
@@ -28,7 +31,7 @@ namespace {
 constexpr int SP_BK = 64;                                               // floats of K a stage
 constexpr int SP_TILE_W = 128 * SP_BK * 2;                              // one bf16 tile of W: 128 rows of 128 bytes
 // Warps: eight cut; with 128 tokens a tile eight add, the first of which also issues the products (sixteen warps, so that a
-// thread may have 128 registers); with fewer four add and one issues.
+// thread may have 128 registers); with fewer four add and one more issues.
 constexpr int SP_CONVERT = 8;
 template <int BT> constexpr int sp_sum() { return BT > 64 ? 8 : 4; }
 template <int BT> constexpr int sp_issuer() { return BT > 64 ? SP_CONVERT : SP_CONVERT + sp_sum<BT>(); }
@@ -42,20 +45,30 @@ template <int BT> constexpr int sp_stage() { return 3 * (SP_TILE_W + BT * SP_BK 
 template <int BT> constexpr int sp_stages() { return BT > 64 ? 2 : 3; }
 template <int BT> constexpr int sp_smem() { return sp_stages<BT>() * sp_stage<BT>() + 1024 + 256; }
 
+// two floats -> their nearest bf16 numbers, the first in the low half
+__device__ __forceinline__ uint32_t sp_round2(float x0, float x1) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(x1), "f"(x0));
+  return d;
+}
+
 // four floats -> four bf16 of each cut
 __device__ __forceinline__ void sp_cut(const float4& a, uint2& h, uint2& m, uint2& l) {
   const float x[4] = {a.x, a.y, a.z, a.w};
-  uint32_t u[4], v[4], w[4];
+  uint32_t c[3][2];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    u[e] = __float_as_uint(x[e]);
-    const float r = x[e] - __uint_as_float(u[e] & 0xffff0000u);       // exact
-    v[e] = __float_as_uint(r);
-    w[e] = __float_as_uint(r - __uint_as_float(v[e] & 0xffff0000u));  // exact, eight bits at most
+  for (int p = 0; p < 2; ++p) {
+    float r0 = x[2 * p], r1 = x[2 * p + 1];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      c[i][p] = sp_round2(r0, r1);
+      r0 -= __uint_as_float(c[i][p] << 16);              // exact: 16 bits are left, then 8
+      r1 -= __uint_as_float(c[i][p] & 0xffff0000u);
+    }
   }
-  h = make_uint2(__byte_perm(u[0], u[1], 0x7632), __byte_perm(u[2], u[3], 0x7632));
-  m = make_uint2(__byte_perm(v[0], v[1], 0x7632), __byte_perm(v[2], v[3], 0x7632));
-  l = make_uint2(__byte_perm(w[0], w[1], 0x7632), __byte_perm(w[2], w[3], 0x7632));
+  h = make_uint2(c[0][0], c[0][1]);
+  m = make_uint2(c[1][0], c[1][1]);
+  l = make_uint2(c[2][0], c[2][1]);
 }
 
 // A load that stays where it is written (a plain one is moved down to its use, behind the wait it was to be hidden under).

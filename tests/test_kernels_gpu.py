@@ -1357,6 +1357,30 @@ def test_gemm_f32_split_is_as_exact_as_the_ordered_sum(M, N, K_, parts):
     assert torch.equal(again, out)
 
 
+@pytest.mark.parametrize("M", [20, 40, 64, 65, 200])
+def test_gemm_f32_split_of_single_products_and_of_one_sign(M):
+    """Sums of one product (a row's only value meets a row's only value), significands of every kind beside those whose cuts are worst, M in
+    every token tile.  Bound: 2^-24 left out, one unit (2^-23) that the tensor core may cut off where the small terms join h h', two float
+    roundings of 2^-24 each; half a percent for the terms' own sizes.  And sums of values of one sign, where errors cannot average out."""
+    k = K()
+    N, K_ = 300, 256
+    hard = torch.tensor([1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -8 - 2.0 ** -23, 1 + 2.0 ** -8, 2 - 2.0 ** -23, 1 + 2.0 ** -16 - 2.0 ** -23,
+                         1 + 2.0 ** -8 - 2.0 ** -16 - 2.0 ** -23, 1 + 2.0 ** -9 + 2.0 ** -17 + 2.0 ** -23, -(1 + 2.0 ** -7 - 2.0 ** -23)], device=DEV)
+    a, w = torch.zeros(M, K_, device=DEV), torch.zeros(N, K_, device=DEV)
+    a[:, 77], w[:, 77] = 1.0 + torch.rand(M, device=DEV, generator=torch.Generator(DEV).manual_seed(1)), _rand(N, seed=2)
+    a[:8, 77], w[:8, 77] = hard, hard
+    got, ref = _f32_split(k, a, w).double(), torch.outer(a[:, 77].double(), w[:, 77].double())
+    worst = ((got - ref) / ref).abs().max().item() * 2.0 ** 23
+    print(f"worst {worst:.2f} units of 2^-23, mean {((got - ref) / ref).mean().item() * 2.0 ** 23:.3f}")
+    assert worst <= 2.0 * 1.005
+    a, w = _rand(M, 2048, seed=3).abs(), _rand(N, 2048, seed=4).abs()
+    ref = a.double() @ w.double().T
+    err = lambda x: ((x.double() - ref) / ref).square().mean().sqrt().item()
+    out, plain = _f32_split(k, a, w), _f32_ordered(k, a, w)
+    print(f"one sign: split {err(out):.3g}, ordered {err(plain):.3g}")
+    assert err(out) <= err(plain)
+
+
 def test_gemm_f32_split_keeps_what_is_no_finite_number_and_the_largest_floats():
     k = K()
     M, N, K_ = 70, 256, 256
