@@ -3,18 +3,18 @@
 //
 // A float is the exact sum of three bf16 numbers: x = h + m + l, h the bf16 nearest to x, m the one nearest to what is left (below
 // 2^-8 of x's power of two), l the rest (below 2^-17).  The product of two floats is taken as h h' + (h m' + m h') + (h l' + m m' + l h');
-// what is left out (m l', l m', l l'; with tiles of up to 64 tokens m l' is in) is below 2^-24 of the product, of either sign: half a unit
+// what is left out (m l', l m', l l'; with tiles of up to 64 tokens l m' is in) is below 2^-24 of the product, of either sign: half a unit
 // in the last place, a float rounding.  (Cut by truncation the residuals are twice as large and have the operand's sign: up to
 // 2^-21 is left out, always towards zero.)  bf16 products are exact in the tensor core's float accumulators;
-// those are only trusted with 64 values of k at a time, in every block of columns the smaller terms first, and are then added to
+// those are only trusted with 64 values of k at a time (they cut off what does not fit) and are then added to
 // sums in registers, rounded to nearest.  The error against 64 bits
 // is smaller than that of the k-ordered sum it replaces (rms over the rms of the result, K = 2,048 / 8,192: 1.6e-7 / 2.0e-7
-// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-22).
+// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-23, with up to 64 tokens to 2^-22).
 //
 // What bounds it: shared memory.  Per 64 values of k a tile of 128 x 128 takes 24 products of 128 x 128 x 16 (1,536 clocks of the
 // tensor pipe), which read 192 KB of operands, and the cutting warps write 96 KB.  The register tile on the CUDA cores
-// that this replaces (gemm_simt_big_kernel) reached 14 to 47 TFLOP/s.  500 tokens, 2,048 -> 16,384: 235 us (143 TFLOP/s)
-// against 828; 8,192 -> 2,048: 122 against 1,232.
+// that this replaces (gemm_simt_big_kernel) reached 14 to 47 TFLOP/s.  500 tokens, 2,048 -> 16,384: 249 us (135 TFLOP/s)
+// against 828; 8,192 -> 2,048: 121 against 1,232.
 //
 // Roles in a CTA: eight warps fetch floats from global memory (the next block's loads are in flight while this block is
 // cut) and write the three bf16 tiles of both operands in the tensor core's swizzled layout; eight warps (four for tiles of up to 64
@@ -36,7 +36,7 @@ constexpr int SP_CONVERT = 8;
 template <int BT> constexpr int sp_sum() { return BT > 64 ? 8 : 4; }
 template <int BT> constexpr int sp_issuer() { return BT > 64 ? SP_CONVERT : SP_CONVERT + sp_sum<BT>(); }
 template <int BT> constexpr int sp_threads() { return BT > 64 ? 512 : 32 * (SP_CONVERT + sp_sum<BT>() + 1); }
-// Tensor memory: an accumulator is two blocks of BT columns (of A's h and of its m and l) or, with fewer tokens, three (h, m, l); as many
+// Tensor memory: an accumulator is two blocks of BT columns (the large terms, small ones) or, with fewer tokens, three; as many
 // as 512 columns hold
 template <int BT> constexpr int sp_acc_cols() { return BT > 32 ? 256 : 128; }
 template <int BT> constexpr int sp_accs() { return 512 / sp_acc_cols<BT>(); }
@@ -134,8 +134,11 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   };
 
   // ---------------- the products of block kb (one thread) ----------------
-  // A's tiles of h, m and l lie one behind the other, so one instruction multiplies a cut of W with two or three of them: an instruction
-  // takes some 100 clocks however few its columns (500 tokens, 2,048 -> 16,384: 252 us with one for every two cuts, 237 so)
+  // Instructions that add to one accumulator run in the order they were issued in only if they have one shape.  With 128 tokens two accumulators
+  // of 128 columns are all there is room for (twice): h h', and the small terms, which are then not cut off against it (five instructions
+  // for every 16 values of k and one more: 249 us where four wider ones of mixed shapes took 235).  With fewer tokens an instruction
+  // takes some 100 clocks however few its columns, so a cut of W meets A's h and m, whose tiles lie one behind the other, in one of them: columns
+  // of h h' + m h' + l h' and of h m' + m m' + l m', the small terms first; h l' apart.
   auto issue = [&](int kb, int s, int phase) {
     const int b = kb % ACCS;
     if (kb >= ACCS && !mbar_wait(smem_u32(&acc_empty[b]), ((kb / ACCS) & 1) ^ 1, abort_flag)) { give_up(23); return false; }
@@ -147,19 +150,26 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     for (int i = 0; i < 3; ++i) w[i] = make_smem_desc(smem_u32(st + i * SP_TILE_W));
     const uint64_t a = make_smem_desc(smem_u32(st + 3 * SP_TILE_W));
     const uint32_t d = tmem_base + (uint32_t)(b * sp_acc_cols<BT>());
-    // in every block of columns the small terms first, so that they are rounded against one another and not against h h'
-    constexpr int BLOCKS = BT > 64 ? 2 : 3;
+    constexpr int TILE = BT * SP_BK * 2;
+    const uint64_t al = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + 2 * TILE));
+    auto product = [&](uint32_t cols, uint64_t cut_w, uint64_t cut_a, int n, bool anew) {
 #pragma unroll
-    for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(d, w[1] + 2 * k, a + 2 * k, make_idesc(128, BLOCKS * BT), k > 0 ? 1u : 0u);
-#pragma unroll
-    for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(d, w[2] + 2 * k, a + 2 * k, make_idesc(128, BT), 1u);
-    if constexpr (BLOCKS == 2) {
-      const uint64_t al = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + 2 * BT * SP_BK * 2));
-#pragma unroll
-      for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(d + BT, w[0] + 2 * k, al + 2 * k, make_idesc(128, BT), 1u);
+      for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(cols, cut_w + 2 * k, cut_a + 2 * k, make_idesc(128, n), anew && k == 0 ? 0u : 1u);
+    };
+    if constexpr (BT > 64) {
+      const uint64_t am = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + TILE));
+      product(d + BT, w[2], a, BT, true);
+      product(d + BT, w[1], am, BT, false);
+      product(d + BT, w[0], al, BT, false);
+      product(d + BT, w[1], a, BT, false);
+      product(d + BT, w[0], am, BT, false);
+      product(d, w[0], a, BT, true);
+    } else {
+      product(d + 2 * BT, w[0], al, BT, true);
+      product(d, w[2], a, 2 * BT, true);
+      product(d, w[1], a, 2 * BT, false);
+      product(d, w[0], a, 2 * BT, false);
     }
-#pragma unroll
-    for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(d, w[0] + 2 * k, a + 2 * k, make_idesc(128, BLOCKS * BT), 1u);
     umma_commit(smem_u32(&empty_bar[s]));
     umma_commit(smem_u32(&acc_full[b]));
     return true;
