@@ -1202,8 +1202,9 @@ def test_rope_of_many_tokens_gives_the_bits_of_few(H, G, hd):
 @pytest.mark.parametrize("M", [65, 79, 81, 129, 143, 145, 256, 257, 271, 289, 293, 513, 530, 769])
 @pytest.mark.parametrize("splits", [1, 2, 4])
 def test_gemm_tc_token_tiles_of_every_height(M, splits):
-    """Numbers of tokens whose equal tiles are and are not multiples of 16 and of 32 (the epilogue's halves), in one part (the persistent
-    kernel) and as clusters, in every form of output; rows behind the last stay as they are.  Tolerances as above: K = 520 float sums,
+    """Numbers of tokens whose equal tiles are and are not multiples of 16 and of 32 (the epilogue's halves), as clusters, and in one part
+    (the persistent kernel, which cuts fewer tiles than SMs into narrow ones of 64 tokens; its tiles of full height: the next test), in
+    every form of output; rows behind the last stay as they are.  Tolerances as above: K = 520 float sums,
     one rounding to bf16."""
     k = K()
     N, K_ = 390, 520
@@ -1226,6 +1227,37 @@ def test_gemm_tc_token_tiles_of_every_height(M, splits):
     act = res[:, :N // 2].to(torch.bfloat16).contiguous()
     k.gemm_tc(a, w * 0.05, act[:M], k.OUT_SWIGLU, force_splits=splits)
     small = a.double() @ (w * 0.05).double().T
+    torch.testing.assert_close(act[:M].double(), torch.nn.functional.silu(small[:, 0::2]) * small[:, 1::2], rtol=2e-2, atol=2e-2)
+    assert torch.equal(act[M:], res[M:, :N // 2].to(torch.bfloat16))
+    k.check_device_errors()
+
+
+@pytest.mark.parametrize("M", [65, 79, 100, 128, 129, 145, 257, 271, 293, 320, 530, 769, 1000])
+def test_gemm_tc_persistent_tiles_of_full_height(M):
+    """149 weight tiles, so that on 148 SMs every token tile has a wave of its full height (80 to 256 tokens: the epilogue's halves are 64 + 16,
+    96 + 48, 96 + 64, 96 + 96, 128 + 80, 128 + 128; the last token tile and the last weight tile are ragged) and narrow tiles follow it: every form
+    of output; rows behind the last stay as they are.  K = 72 float sums, one rounding to bf16."""
+    k = K()
+    N, K_ = 148 * 128 + 66, 72
+    a, w, bias = _rand(M, K_, dtype=torch.bfloat16, seed=1), _rand(N, K_, dtype=torch.bfloat16, seed=2), _rand(N, seed=3)
+    ref = a.double() @ w.double().T
+    f32 = dict(rtol=1e-4, atol=8e-5 * math.sqrt(K_))
+    res = _rand(M + 5, N, seed=4)
+    out = res.clone()
+    k.gemm_tc(a, w, out[:M], k.OUT_ADD_F32, bias)
+    torch.testing.assert_close(out[:M].double(), ref + bias.double() + res[:M].double(), **f32)
+    assert torch.equal(out[M:], res[M:])
+    out = res.clone()
+    k.gemm_tc(a, w, out[:M], k.OUT_F32)
+    torch.testing.assert_close(out[:M].double(), ref, **f32)
+    assert torch.equal(out[M:], res[M:])
+    same = res.to(torch.bfloat16)
+    k.gemm_tc(a, w, same[:M], k.OUT_SAME, bias)
+    torch.testing.assert_close(same[:M].double(), ref + bias.double(), rtol=1e-2, atol=1e-2 * math.sqrt(K_))
+    assert torch.equal(same[M:], res[M:].to(torch.bfloat16))
+    act = res[:, :N // 2].to(torch.bfloat16).contiguous()
+    k.gemm_tc(a, w * 0.15, act[:M], k.OUT_SWIGLU)
+    small = a.double() @ (w * 0.15).double().T
     torch.testing.assert_close(act[:M].double(), torch.nn.functional.silu(small[:, 0::2]) * small[:, 1::2], rtol=2e-2, atol=2e-2)
     assert torch.equal(act[M:], res[M:, :N // 2].to(torch.bfloat16))
     k.check_device_errors()
