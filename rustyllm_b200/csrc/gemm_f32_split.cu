@@ -6,10 +6,10 @@
 // what is left out (m l', l m', l l'; with tiles of up to 64 tokens l m' is in) is below 2^-24 of the product, of either sign: half a unit
 // in the last place, a float rounding.  (Cut by truncation the residuals are twice as large and have the operand's sign: up to
 // 2^-21 is left out, always towards zero.)  bf16 products are exact in the tensor core's float accumulators;
-// those are only trusted with 64 values of k at a time (they cut off what does not fit) and are then added to
-// sums in registers, rounded to nearest.  The error against 64 bits
+// those are only trusted with 64 values of k at a time - h h' in one, the small terms in another, so that they are not cut off against the
+// large ones - and are then added to sums in registers, rounded to nearest.  The error against 64 bits
 // is smaller than that of the k-ordered sum it replaces (rms over the rms of the result, K = 2,048 / 8,192: 1.6e-7 / 2.0e-7
-// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-23, with up to 64 tokens to 2^-22).
+// against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-23).
 //
 // What bounds it: shared memory.  Per 64 values of k a tile of 128 x 128 takes 24 products of 128 x 128 x 16 (1,536 clocks of the
 // tensor pipe), which read 192 KB of operands, and the cutting warps write 96 KB.  The register tile on the CUDA cores
@@ -24,6 +24,8 @@
 //
 // Infinities and NaNs do not survive the cutting (inf - inf), and floats above the largest bf16 (3.39e38) are rounded to infinity, so an
 // output that is no finite number is computed again, alone and in the order of k, by the plain sum.
+#include <type_traits>
+
 #include "tc_device.cuh"
 
 namespace {
@@ -36,7 +38,7 @@ constexpr int SP_CONVERT = 8;
 template <int BT> constexpr int sp_sum() { return BT > 64 ? 8 : 4; }
 template <int BT> constexpr int sp_issuer() { return BT > 64 ? SP_CONVERT : SP_CONVERT + sp_sum<BT>(); }
 template <int BT> constexpr int sp_threads() { return BT > 64 ? 512 : 32 * (SP_CONVERT + sp_sum<BT>() + 1); }
-// Tensor memory: an accumulator is two blocks of BT columns (the large terms, small ones) or, with fewer tokens, three; as many
+// Tensor memory: an accumulator is two blocks of BT columns (h h', the small terms) or, with fewer tokens, three; as many
 // as 512 columns hold
 template <int BT> constexpr int sp_acc_cols() { return BT > 32 ? 256 : 128; }
 template <int BT> constexpr int sp_accs() { return 512 / sp_acc_cols<BT>(); }
@@ -134,11 +136,11 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   };
 
   // ---------------- the products of block kb (one thread) ----------------
-  // Instructions that add to one accumulator run in the order they were issued in only if they have one shape.  With 128 tokens two accumulators
-  // of 128 columns are all there is room for (twice): h h', and the small terms, which are then not cut off against it (five instructions
-  // for every 16 values of k and one more: 249 us where four wider ones of mixed shapes took 235).  With fewer tokens an instruction
-  // takes some 100 clocks however few its columns, so a cut of W meets A's h and m, whose tiles lie one behind the other, in one of them: columns
-  // of h h' + m h' + l h' and of h m' + m m' + l m', the small terms first; h l' apart.
+  // Instructions that add to one accumulator run in the order they were issued in only if they have one shape, and what does not fit a
+  // float is cut off: h h' has an accumulator of its own, the small terms another.  With 128 tokens two of 128 columns are all there is room for
+  // (twice): six instructions for every 16 values of k (249 us where four wider ones of mixed shapes took 235).  With fewer tokens an instruction
+  // takes some 100 clocks however few its columns, so the small terms' instructions multiply a cut of W with two of A's, whose tiles lie one
+  // behind the other (w[2] with m as well, which costs nothing).
   auto issue = [&](int kb, int s, int phase) {
     const int b = kb % ACCS;
     if (kb >= ACCS && !mbar_wait(smem_u32(&acc_empty[b]), ((kb / ACCS) & 1) ^ 1, abort_flag)) { give_up(23); return false; }
@@ -150,26 +152,20 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     for (int i = 0; i < 3; ++i) w[i] = make_smem_desc(smem_u32(st + i * SP_TILE_W));
     const uint64_t a = make_smem_desc(smem_u32(st + 3 * SP_TILE_W));
     const uint32_t d = tmem_base + (uint32_t)(b * sp_acc_cols<BT>());
-    constexpr int TILE = BT * SP_BK * 2;
-    const uint64_t al = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + 2 * TILE));
+    constexpr int TILE = BT * SP_BK * 2, SMALL = BT > 64 ? BT : 2 * BT;          // columns of the small terms
+    const uint64_t am = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + TILE));
     auto product = [&](uint32_t cols, uint64_t cut_w, uint64_t cut_a, int n, bool anew) {
 #pragma unroll
       for (int k = 0; k < SP_BK / UMMA_K; ++k) umma_bf16(cols, cut_w + 2 * k, cut_a + 2 * k, make_idesc(128, n), anew && k == 0 ? 0u : 1u);
     };
-    if constexpr (BT > 64) {
-      const uint64_t am = make_smem_desc(smem_u32(st + 3 * SP_TILE_W + TILE));
-      product(d + BT, w[2], a, BT, true);
-      product(d + BT, w[1], am, BT, false);
-      product(d + BT, w[0], al, BT, false);
-      product(d + BT, w[1], a, BT, false);
-      product(d + BT, w[0], am, BT, false);
-      product(d, w[0], a, BT, true);
-    } else {
-      product(d + 2 * BT, w[0], al, BT, true);
-      product(d, w[2], a, 2 * BT, true);
-      product(d, w[1], a, 2 * BT, false);
-      product(d, w[0], a, 2 * BT, false);
+    product(d + BT, w[2], a, SMALL, true);
+    if constexpr (SMALL == BT) {
+      product(d + BT, w[1], am, SMALL, false);
+      product(d + BT, w[0], make_smem_desc(smem_u32(st + 3 * SP_TILE_W + 2 * TILE)), SMALL, false);
     }
+    product(d + BT, w[1], a, SMALL, false);
+    product(d + BT, w[0], am, SMALL, false);
+    product(d, w[0], a, BT, true);
     umma_commit(smem_u32(&empty_bar[s]));
     umma_commit(smem_u32(&acc_full[b]));
     return true;
@@ -240,21 +236,15 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     // ---------------- sums: a warp's quarter of the rows (lanes), its share of the token columns ----------------
     constexpr int NC = BT / (SUM / 4), BLOCKS = BT > 64 ? 2 : 3;
     const int quarter = warp & 3, share = (warp - SP_CONVERT) >> 2;
+    const int n = n0 + quarter * 32 + lane;
+    // With up to 64 tokens a tile the bias goes in front of the last block's terms, the small ones first: it is then not one more rounding of a
+    // finished sum.  (With 128 a second form of the loop below takes registers that are not there: 249 -> 282 us.)
+    constexpr bool BIAS_INSIDE = BT <= 64;
+    const float b = BIAS_INSIDE && bias && split == 0 && n < N ? bias[n] : 0.f;
     float acc[NC];
 #pragma unroll
     for (int j = 0; j < NC; ++j) acc[j] = 0.f;
-    int s = 0, phase = 0;
-    for (int kb = 0; kb <= num_kb; ++kb) {
-      if (warp == ISSUER && kb < num_kb) {       // they run while the sums of the block in front are added
-        if (lane == 0 && !*abort_flag) issue(kb, s, phase);
-        __syncwarp();
-        if (++s == STAGES) { s = 0; phase ^= 1; }
-      }
-      if (kb == 0) continue;
-      const int b = (kb - 1) % ACCS;
-      if (!mbar_wait(smem_u32(&acc_full[b]), ((kb - 1) / ACCS) & 1, abort_flag)) { give_up(22); break; }
-      tc_fence_after();
-      const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * sp_acc_cols<BT>() + share * NC);
+    auto add_block = [&](uint32_t t, auto last) {
 #pragma unroll
       for (int q = 0; q < NC / 16; ++q) {
         uint32_t r[16], v[16];
@@ -268,11 +258,30 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
         tmem_ld16(t + q * 16, r);
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[q * 16 + j] += __uint_as_float(v[j]) + __uint_as_float(r[j]);
+        for (int j = 0; j < 16; ++j) {
+          float& sum = acc[q * 16 + j];
+          if constexpr (decltype(last)::value) sum = ((sum + b) + __uint_as_float(v[j])) + __uint_as_float(r[j]);
+          else sum += __uint_as_float(v[j]) + __uint_as_float(r[j]);
+        }
       }
+    };
+    int s = 0, phase = 0;
+    for (int kb = 0; kb <= num_kb; ++kb) {
+      if (warp == ISSUER && kb < num_kb) {       // they run while the sums of the block in front are added
+        if (lane == 0 && !*abort_flag) issue(kb, s, phase);
+        __syncwarp();
+        if (++s == STAGES) { s = 0; phase ^= 1; }
+      }
+      if (kb == 0) continue;
+      const int buf = (kb - 1) % ACCS;
+      if (!mbar_wait(smem_u32(&acc_full[buf]), ((kb - 1) / ACCS) & 1, abort_flag)) { give_up(22); break; }
+      tc_fence_after();
+      const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * sp_acc_cols<BT>() + share * NC);
+      if (BIAS_INSIDE && kb == num_kb) add_block(t, std::bool_constant<BIAS_INSIDE>());
+      else add_block(t, std::false_type());
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+      if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));
     }
     if (splits > 1) {
       // the other parts' sums come through their shared memory (every product has read it: this thread has seen its part's
@@ -296,9 +305,8 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
       __syncwarp();
       cluster_sync_all();                        // nobody leaves while another part still reads its shared memory
     }
-    const int n = n0 + quarter * 32 + lane;
     if (split == 0 && n < N && !*abort_flag) {
-      const float b = bias ? bias[n] : 0.f;
+      const float at_end = !BIAS_INSIDE && bias ? bias[n] : 0.f;
       const int j0 = m0 + share * NC;
 #pragma unroll
       for (int c = 0; c < NC; c += 16) {
@@ -310,8 +318,8 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
           const int m = j0 + c + j;
           if (m >= M) continue;
           float v = acc[c + j];
-          if (!(fabsf(v) <= 3.402823466e38f)) v = sp_plain_dot(A + (size_t)m * lda, W + (size_t)n * K, K);
-          v += b;
+          if (!(fabsf(v) <= 3.402823466e38f)) v = sp_plain_dot(A + (size_t)m * lda, W + (size_t)n * K, K) + b;
+          if constexpr (!BIAS_INSIDE) v += at_end;
           out[(size_t)m * ldo + n] = add ? old[j] + v : v;
         }
       }
