@@ -181,7 +181,8 @@ __device__ __forceinline__ void tile_epilogue(uint32_t tmem_acc, int quarter, in
 }
 
 // BT: tokens per CTA (MMA N).  Grid: (parts * ceil(N_out / 128), ceil(M_tokens / BT)) in
-// clusters of `parts` CTAs along x; the CTA's rank in its cluster is its part of K.
+// clusters of `parts` CTAs along x; the CTA's rank in its cluster is its part of K.  More than 64 tokens a tile come here in two parts or
+// more, without a norm, a rotation or groups (unsplit and grouped ones go to the persistent kernel below).
 template <int BT, bool DEEP>
 __global__ void __launch_bounds__(tc_threads<BT>(), TcConfig<BT, DEEP>::MIN_CTAS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
@@ -204,7 +205,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int num_splits = (int)cluster_size(), split = (int)cluster_rank();
   const int n0 = (blockIdx.x / num_splits) * BLOCK_N_OUT;   // first weight row (output feature) of this CTA
-  const int tile_m = BT > 64 && fuse.tile_m > 0 ? fuse.tile_m : BT;      // tokens of a tile
+  const int tile_m = BT > 64 ? fuse.tile_m : BT;            // tokens of a tile
   const int m0 = blockIdx.y * tile_m;                       // first token of this CTA
   int w_row0 = n0;                                          // first row of the weight tile in the weight's tensor map
   if (fuse.tile_group != nullptr) {
@@ -298,24 +299,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if constexpr (BT <= 64) {
       if (fuse.scale_partials != nullptr)    // while the products still run
         epilogue_row_scales<BT>(fuse, m0, M, K, warp & 3, lane, fuse_smem);
-    }
-    if (out_mode == TC_OUT_ROPE_KV) {
-      // position of every token of the tile and the row of the cache pools it is stored in
-      int* tok_pos = (int*)(fuse_smem + BT);
-      int* tok_row = tok_pos + BT;
-      for (int t = threadIdx.x - 64; t < BT; t += 128) {
-        const int m = m0 + t;
-        int pos = 0, row = 0;
-        if (m < M) {
-          pos = fuse.positions[m];
-          if (fuse.k_pool != nullptr) {
-            const int page = fuse.page_table[(size_t)fuse.slot_of_token[m] * fuse.max_pages + pos / RL_PAGE];
-            row = page * fuse.num_kv_heads * RL_PAGE + pos % RL_PAGE;        // + kv head * RL_PAGE
+      if (out_mode == TC_OUT_ROPE_KV) {
+        // position of every token of the tile and the row of the cache pools it is stored in
+        int* tok_pos = (int*)(fuse_smem + BT);
+        int* tok_row = tok_pos + BT;
+        for (int t = threadIdx.x - 64; t < BT; t += 128) {
+          const int m = m0 + t;
+          int pos = 0, row = 0;
+          if (m < M) {
+            pos = fuse.positions[m];
+            if (fuse.k_pool != nullptr) {
+              const int page = fuse.page_table[(size_t)fuse.slot_of_token[m] * fuse.max_pages + pos / RL_PAGE];
+              row = page * fuse.num_kv_heads * RL_PAGE + pos % RL_PAGE;        // + kv head * RL_PAGE
+            }
           }
+          tok_pos[t] = pos; tok_row[t] = row;
         }
-        tok_pos[t] = pos; tok_row[t] = row;
+        epilogue_sync();
       }
-      epilogue_sync();
     }
     const bool ok = mbar_wait(smem_u32(accum_bar), 0, abort_flag);
     if (!ok && !*abort_flag) { *abort_flag = 1; atomicExch(err, 3); }
@@ -323,10 +324,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int quarter = warp & 3;                    // lanes this warp may read
     const int second = BT > 64 ? (warp - 2) >> 2 : 0;        // 1: the second warp of a quarter
     const int row = quarter * 32 + lane;             // accumulator row = weight row of the tile
-    if (ok && num_splits == 1) {
-      // (with eight epilogue warps the tokens in two halves, as in the persistent kernel)
-      const int cols = min(tile_m, M - m0), half = BT > 64 ? min(cols, (tile_m / 2 + 31) & ~31) : cols, c0 = second ? half : 0;
-      tile_epilogue<BT>(tmem_base + (uint32_t)c0, quarter, lane, n0, m0 + c0, second ? cols - half : half, M, N, ldo, bias, out, out_mode, fuse, fuse_smem);
+    if (BT <= 64 && ok && num_splits == 1) {
+      tile_epilogue<BT>(tmem_base, quarter, lane, n0, m0, min(BT, M - m0), M, N, ldo, bias, out, out_mode, fuse, fuse_smem);
     } else if (num_splits > 1 && ok) {
       // this part's partial tile -> own shared memory (the ring is free: every MMA has
       // completed), as [token column][weight row] floats
