@@ -603,6 +603,7 @@ static int balanced_tile(int M, int BT) {
   return (each + 15) / 16 * 16;
 }
 
+// ma: the activations in boxes of fuse.tile_m rows, the height of a tile (grouped: BT)
 template <int BT>
 static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, const void* A, int lda, const float* bias,
                                 void* out, int out_mode, int M, int N, int K, int ldo, int* err, cudaStream_t stream,
@@ -617,7 +618,7 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
     configured = true;
   }
   const int num_sms = rl_num_sms();
-  const int tile_m = tile_group != nullptr ? BT : balanced_tile(M, BT);
+  const int tile_m = fuse.tile_m;
   const int tiles_m = (M + tile_m - 1) / tile_m, tiles_n = (N + BLOCK_N_OUT - 1) / BLOCK_N_OUT;
   const int total = tiles_m * tiles_n;
   // the tiles behind the last full wave: the narrowest token tile (from 64 tokens: below, the
@@ -638,18 +639,14 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
       }
     }
   }
-  CUtensorMap ma_tile = ma, ma_tail = ma;      // the same activations in boxes as tall as a tile, and as a narrow tile
-  if (tile_m != BT) {
-    const int rc = tc_make_map(&ma_tile, A, M, K, lda, tile_m);
-    if (rc != RL_OK) return rc;
-  }
-  if (tail.bt != BT) {
+  CUtensorMap ma_tail = ma;      // the same activations in boxes as tall as a narrow tile
+  if (tail.bt != tile_m) {
     const int rc = tc_make_map(&ma_tail, A, M, K, lda, tail.bt);
     if (rc != RL_OK) return rc;
   }
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
   cudaError_t e = rl_launch_pdl(gemm_tc_persistent_kernel<BT>, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)Cfg::SMEM_BYTES, stream,
-                                mw, ma_tile, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, tail, tile_group, group_rows,
+                                mw, ma, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, tail, tile_group, group_rows,
                                 fuse.act_limit, fuse.act_alpha);
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_tc: launch of the persistent kernel failed: %s", cudaGetErrorString(e));
@@ -843,7 +840,8 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   CUtensorMap mw, ma;
   int rc = tc_make_map(&mw, W, N, K, K, BLOCK_N_OUT);
   if (rc != RL_OK) return rc;
-  rc = tc_make_map(&ma, A, M, K, lda, bt);
+  fuse.tile_m = bt > 64 ? balanced_tile(M, bt) : bt;
+  rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
   if (rc != RL_OK) return rc;
   switch (bt) {
     case 16: return launch_tc<16>(mw, ma, bias, out, out_mode, M, N, K, ldo, err, splits, kb_per, fuse, stream);
@@ -852,11 +850,6 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
     default: break;
   }
   if (splits > 1) {       // few tiles of many tokens: the parts of a tile as a cluster, as for few tokens
-    fuse.tile_m = balanced_tile(M, bt);
-    if (fuse.tile_m != bt) {
-      rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
-      if (rc != RL_OK) return rc;
-    }
     if (bt == 128) return launch_tc<128>(mw, ma, bias, out, out_mode, M, N, K, ldo, err, splits, kb_per, fuse, stream);
     return launch_tc<256>(mw, ma, bias, out, out_mode, M, N, K, ldo, err, splits, kb_per, fuse, stream);
   }
@@ -905,7 +898,7 @@ extern "C" int rl_gemm_tc_grouped(const void* A, const void* W, void* out, int o
              "rl_gemm_tc_grouped: the token tile must be 16, 32, 64, 128 or 256 and divide M (%d, %d)", bt, M);
   RL_REQUIRE((long long)groups * N <= 2147483647LL && M / bt <= 65535, "rl_gemm_tc_grouped: too many weight rows or token tiles");
   TcFuse fuse = {};
-  fuse.tile_group = tile_group; fuse.group_rows = N;
+  fuse.tile_group = tile_group; fuse.group_rows = N; fuse.tile_m = bt;
   fuse.act_limit = act_limit; fuse.act_alpha = act_alpha;
   fuse.norm_count = 4 * ((N + BLOCK_N_OUT - 1) / BLOCK_N_OUT);
   const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;

@@ -65,7 +65,7 @@ struct TcFuse {
   int group_rows;
   // constants of the clamped gate (out_mode TC_OUT_CLAMPED only)
   float act_limit, act_alpha;
-  // tokens of a tile of the cluster kernel for more than 64 tokens (0: all that the kernel's form holds)
+  // tokens of a tile
   int tile_m;
 };
 
