@@ -19,8 +19,9 @@
 // one dependent multiply-add a state element and token; everything else (the loads of q and k from shared
 // memory, the dot product, the shuffles) is latency to hide, so R grows with dk (8, 16, 32: a block of 128,
 // 256 or 512 threads, at most 8 state elements a thread): more warps an SM, fewer instructions a thread.
-// The order of every sum is fixed by the sizes alone, so a position's output does not depend on how the
-// sequence was cut into steps or on the batch.  State layout per slot: [H, dv, dk].
+// The order of every sum is fixed by the sizes and `wide` alone, so within one shape of this kernel a position's output does not depend
+// on how the sequence was cut into steps or on the batch (modes 0 and 1 over many tokens run by chunks instead, linear_scan_chunked.cu, whose
+// borders follow the cut: to rounding).  State layout per slot: [H, dv, dk].
 #include <math.h>
 
 #include "common.cuh"
