@@ -8,7 +8,7 @@
 // 2^-21 is left out, always towards zero.)  bf16 products are exact in the tensor core's float accumulators;
 // those are only trusted with 64 values of k at a time - h h' in one, the small terms in another, so that they are not cut off against the
 // large ones - and are then added to sums in registers, rounded to nearest.  The error against 64 bits
-// is smaller than that of the k-ordered sum it replaces (rms over the rms of the result, K = 2,048 / 8,192: 1.6e-7 / 2.0e-7
+// is smaller than that of the k-ordered sum it replaces (rms over the rms of the result, K = 2,048 / 8,192: 1.3e-7 / 1.6e-7
 // against 8.1e-7 / 1.6e-6; tests/test_kernels_gpu.py holds it to that, and single products to 2^-23).
 //
 // What bounds it: shared memory.  Per 64 values of k a tile of 128 x 128 takes 24 products of 128 x 128 x 16 (1,536 clocks of the
@@ -345,8 +345,8 @@ gemm_f32_split_kernel(const float* __restrict__ A, const float* __restrict__ W, 
 int sp_token_tile(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 // The K range of a tile in as many parts (1, 2 or 4: the cluster's size) as still fit one CTA an SM, at least four blocks of 64 a
-// part: 64 tiles (500 tokens, 2,048 output columns) leave more than half of the SMs idle otherwise (K = 8,192: 215 us whole,
-// 116 us in two parts).  Eight parts lose: one CTA adds seven others' sums (16 tiles, K = 8,192: 84 us against 65 in four).
+// part: 64 tiles (500 tokens, 2,048 output columns) leave more than half of the SMs idle otherwise (K = 8,192: 224 us whole,
+// 122 us in two parts).  Eight parts lose: one CTA adds seven others' sums (16 tiles, K = 8,192: 90 us against 70 in four).
 int sp_parts(int M, int N, int K) {
   const int bt = sp_token_tile(M), tiles = ((N + 127) / 128) * ((M + bt - 1) / bt), total_kb = (K + SP_BK - 1) / SP_BK;
   int parts = 1;
@@ -382,8 +382,7 @@ int sp_launch(const float* A, const float* W, const float* bias, float* out, int
 }  // namespace
 
 // 1 where the split product is taken instead of the CUDA cores: rows that 16-byte pieces can fetch, a tile's width of outputs, sums from
-// K = 256 on (shorter ones it does not make more exactly than the ordered sum: K = 64 1.7e-7 against 1.4e-7 of the result's rms, K = 256
-// 2.1e-7 against 2.3e-7), and more than 8 tokens (up to there gemm_f32_few.cu: see there).
+// K = 256 on, where it is twice as exact as the ordered sum (1.1e-7 against 2.2e-7 of the result's rms; K = 64: 1.1e-7 against 1.4e-7), and more than 8 tokens (up to there gemm_f32_few.cu: see there).
 extern "C" int rl_gemm_f32_split_supported(const void* A, const void* W, int M, int N, int K, int lda) {
   return M > 8 && N >= 128 && K >= 256 && K % 4 == 0 && lda % 4 == 0 && lda >= K && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 &&
          (N + 127) / 128 <= 65535;

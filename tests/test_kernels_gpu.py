@@ -138,6 +138,8 @@ def test_gemm_simt_all_modes(dtype, M, N, K_):
 
 
 def test_gemm_simt_rows_do_not_depend_on_the_batch():
+    """The sum in the order of k (here for float sums shorter than 256; longer ones with more than 8 rows go by tiles of tokens and differ by
+    rounding)."""
     k = K()
     a = _rand(130, 172, seed=8)
     w = _rand(96, 172, seed=9)
