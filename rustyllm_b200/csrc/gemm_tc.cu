@@ -655,6 +655,253 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
   return RL_OK;
 }
 
+// ------------------------------------------------------------------ persistent variant by pairs of CTAs
+// Two CTAs on neighbouring SMs (a cluster of two) hold one tile of 256 weight rows: tcgen05.mma with cta_group::2, M = 256,
+// each CTA staging its own 128 weight rows and half of the tile's tokens, each with its 128 rows of the accumulator in its own
+// tensor memory.  What bounds the kernel above is what its SMs pull out of L2 and what the tensor cores read out of shared memory: a CTA
+// alone fetches 48 KB for a block of K of 128 x 256 outputs, a CTA of a pair 32 KB.  One B200, us, CTAs alone / pairs: 2,048 tokens,
+// 4,096 -> 28,672 with SwiGLU 358 / 346 (1.39 PFLOP/s, the power cap), 4,096 -> 6,144 82 / 76, 4,096 -> 4,096 added into the residual
+// 67.7 / 57.0, 14,336 -> 4,096 204 / 190; 5,514 tokens, 2,048 -> 16,384 285 / 276, 8,192 -> 2,048 179 / 167; 293 tokens, 4,096 -> 28,672
+// 90.9 / 86.2.  Roles, the two accumulators and the narrow tiles of the last wave are as above; the leader's (rank 0)
+// issuing thread works for both CTAs, both producers' loads arrive at the leader's barriers, and a commit arrives in both CTAs.
+static constexpr int PAIR_ROWS = 2 * BLOCK_N_OUT;
+static constexpr int PAIR_MAX_STAGES = 10;
+static constexpr int PAIR_RING_BYTES = 6 * (BLOCK_N_OUT + 128) * BLOCK_K * 2;      // six stages of tiles of 256 tokens
+static constexpr int PAIR_SMEM_BYTES = PAIR_RING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+static constexpr int PAIR_ACC_COLS = 256;
+
+__device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(leader_bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void pair_umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Arrives on the barrier at this place in both CTAs once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void pair_umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_PERSISTENT_THREADS, 1)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                    const __grid_constant__ CUtensorMap map_a_tail, const float* __restrict__ bias,
+                    void* __restrict__ out, int out_mode, int M, int N, int K, int ldo, int* __restrict__ err,
+                    int tile_m, int tiles_m, int num_tiles, int stages, const TcTail tail, float act_limit, float act_alpha) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t* tiles = smem;
+  uint64_t* bars = (uint64_t*)(smem + PAIR_RING_BYTES);
+  uint64_t* full_bar = bars;                                 // [stages]  the leader's are used: both CTAs' loads arrive there
+  uint64_t* empty_bar = bars + PAIR_MAX_STAGES;              // [stages]
+  uint64_t* acc_full = bars + 2 * PAIR_MAX_STAGES;           // [2]
+  uint64_t* acc_empty = bars + 2 * PAIR_MAX_STAGES + 2;      // [2]       the leader's are used
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * PAIR_MAX_STAGES + 4);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
+  const int stage_bytes = (BLOCK_N_OUT + tile_m / 2) * BLOCK_K * 2;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&acc_full[i]), 1);
+      mbar_init(smem_u32(&acc_empty[i]), 16);      // one arrival per epilogue warp of both CTAs
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a_tail) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * PAIR_ACC_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();        // both CTAs' barriers are ready, both have their tensor memory
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  rl_pdl_trigger();
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---------------- producer of this CTA's half: its 128 weight rows, its half of the tokens ----------------
+      int s = 0, laps = 0;                          // place in the ring
+      bool waited = false, ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
+        const int n0 = at.n0 * 2 + rank * BLOCK_N_OUT;
+        const int m0 = at.m0 + rank * (at.bt / 2);
+        const CUtensorMap* ma = at.bt == tile_m ? &map_a : &map_a_tail;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (laps > 0 && !mbar_wait(smem_u32(&empty_bar[s]), (laps & 1) ^ 1, abort_flag)) {
+            if (!*abort_flag) { *abort_flag = 1; atomicExch(err, 1); }
+            ok = false;
+            break;
+          }
+          const uint32_t fb = dsmem_addr(smem_u32(&full_bar[s]), 0);
+          if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), (PAIR_ROWS + at.bt) * BLOCK_K * 2);
+          uint8_t* st = tiles + (size_t)s * stage_bytes;
+          pair_load_2d(smem_u32(st), &map_w, fb, kb * BLOCK_K, n0);
+          // weights may be requested before the preceding kernels have finished, activations not
+          if (!waited) { rl_pdl_wait(); waited = true; }
+          pair_load_2d(smem_u32(st + BLOCK_N_OUT * BLOCK_K * 2), ma, fb, kb * BLOCK_K, m0);
+          if (++s == stages) { s = 0; ++laps; }
+        }
+      }
+      // every stage filled has been read (the arrivals come from the leader): nothing of this CTA is in flight when it ends
+      for (int i = 0; i < stages && ok; ++i) {
+        if (laps > 0) ok = mbar_wait(smem_u32(&empty_bar[s]), (laps & 1) ^ 1, abort_flag);
+        if (++s == stages) { s = 0; ++laps; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      // ---------------- MMA issuer, for both CTAs ----------------
+      int s = 0, laps = 0, t = 0;
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        const TcTileAt mat = tc_tile_at(tile, tiles_m, tile_m, tail);
+        const uint32_t idesc = make_idesc(PAIR_ROWS, mat.bt);
+        const int buf = t & 1;
+        const uint32_t acc_phase = (t >> 1) & 1;
+        if (t >= 2 && !mbar_wait(smem_u32(&acc_empty[buf]), acc_phase ^ 1, abort_flag)) {   // both epilogues done with this accumulator
+          if (!*abort_flag) { *abort_flag = 1; atomicExch(err, 4); }
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PAIR_ACC_COLS);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!mbar_wait(smem_u32(&full_bar[s]), laps & 1, abort_flag)) {
+            if (!*abort_flag) { *abort_flag = 1; atomicExch(err, 2); }
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          uint8_t* st = tiles + (size_t)s * stage_bytes;
+          const uint64_t da = make_smem_desc(smem_u32(st));
+          const uint64_t db = make_smem_desc(smem_u32(st + BLOCK_N_OUT * BLOCK_K * 2));
+#pragma unroll
+          for (int k = 0; k < BLOCK_K / UMMA_K; ++k)
+            pair_umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          pair_umma_commit(smem_u32(&empty_bar[s]));
+          if (++s == stages) { s = 0; ++laps; }
+        }
+        if (ok) pair_umma_commit(smem_u32(&acc_full[buf]));
+        ++t;
+      }
+    }
+  } else {
+    // ---------------- epilogue warps: this CTA's 128 weight rows ----------------
+    rl_pdl_wait();
+    const int quarter = warp & 3, second = (warp - 2) >> 2;      // as in the kernel above
+    int t = 0;
+    for (int tile = pair; tile < num_tiles; tile += pairs) {
+      const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
+      const int buf = t & 1;
+      const uint32_t acc_phase = (t >> 1) & 1;
+      if (!mbar_wait(smem_u32(&acc_full[buf]), acc_phase, abort_flag)) {
+        if (!*abort_flag) { *abort_flag = 1; atomicExch(err, 3); }
+        break;
+      }
+      tc_fence_after();
+      TcFuse fuse = {};
+      fuse.act_limit = act_limit;
+      fuse.act_alpha = act_alpha;
+      const int cols = min(at.bt, M - at.m0), half = min(cols, (at.bt / 2 + 31) & ~31), c0 = second ? half : 0;
+      tile_epilogue<256>(tmem_base + (uint32_t)(buf * PAIR_ACC_COLS + c0), quarter, lane, at.n0 * 2 + rank * BLOCK_N_OUT, at.m0 + c0,
+                         second ? cols - half : half, M, N, ldo, bias, out, out_mode, fuse, nullptr);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) pair_arrive(dsmem_addr(smem_u32(&acc_empty[buf]), 0));    // this warp has read the accumulator
+      ++t;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();        // nobody leaves while the other still signals it or reads its operands
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_ACC_COLS) : "memory");
+}
+
+// The height of equal tiles that cover M tokens with as few of them as tiles of 256 do, in steps of 32 (the instruction's two halves
+// in steps of 16).
+static int pair_tile(int M) {
+  const int tiles = (M + 255) / 256, each = (M + tiles - 1) / tiles;
+  return (each + 31) / 32 * 32;
+}
+
+// Whether the pairs take a product of more than 128 tokens that is not split over K: where its tiles are more than one wave of them.
+// In one wave nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster barriers): us, CTAs
+// alone / pairs, 2,048 tokens 2,048 -> 3,072 34.2 / 36.2, 2,048 -> 2,048 26.9 / 29.5; 1,500 tokens 18.1 / 18.7, 18.5 / 19.5.
+static bool pairs_pay(int M, int N) {
+  return (M + 255) / 256 * ((N + PAIR_ROWS - 1) / PAIR_ROWS) > rl_num_sms() / 2;
+}
+
+static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const float* bias, void* out, int out_mode, int M, int N, int K,
+                          int ldo, int* err, cudaStream_t stream, const TcFuse& fuse) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
+    RL_REQUIRE(e == cudaSuccess, "rl_gemm_tc: cannot reserve %d bytes of shared memory: %s", PAIR_SMEM_BYTES, cudaGetErrorString(e));
+    configured = true;
+  }
+  const int pairs = rl_num_sms() / 2, tile_m = pair_tile(M);
+  const int tiles_m = (M + tile_m - 1) / tile_m, tiles_n = (N + PAIR_ROWS - 1) / PAIR_ROWS;
+  const int total = tiles_m * tiles_n;
+  TcTail tail = {total, tile_m, 0, 0, 0, 1, 0};
+  int num_tiles = total;
+  const int full = (total / pairs) * pairs;
+  if (full < total) {       // the tiles behind the last full wave are cut narrower along the tokens, as above
+    const int n_first = full / tiles_m, t0_first = (full % tiles_m) * tile_m;
+    for (int bt = 64; bt < tile_m; bt += 32) {
+      const int count_first = (M - t0_first + bt - 1) / bt, per_n = (M + bt - 1) / bt;
+      const int cnt = count_first + (tiles_n - n_first - 1) * per_n;
+      if (cnt <= pairs) {
+        tail = {full, bt, n_first, t0_first, count_first, per_n};
+        num_tiles = full + cnt;
+        break;
+      }
+    }
+  }
+  CUtensorMap ma, ma_tail;
+  int rc = tc_make_map(&ma, A, M, K, lda, tile_m / 2);
+  if (rc != RL_OK) return rc;
+  ma_tail = ma;
+  if (tail.bt != tile_m) {
+    rc = tc_make_map(&ma_tail, A, M, K, lda, tail.bt / 2);
+    if (rc != RL_OK) return rc;
+  }
+  const int stage_bytes = (BLOCK_N_OUT + tile_m / 2) * BLOCK_K * 2;
+  const int stages = PAIR_RING_BYTES / stage_bytes < PAIR_MAX_STAGES ? PAIR_RING_BYTES / stage_bytes : PAIR_MAX_STAGES;
+  const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
+  cudaError_t e = rl_launch_pdl(gemm_tc_pair_kernel, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)PAIR_SMEM_BYTES, stream, mw, ma, ma_tail,
+                                bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, stages, tail,
+                                fuse.act_limit, fuse.act_alpha);
+  if (e != cudaSuccess) {
+    rl_set_error("rl_gemm_tc: launch of the kernel by pairs failed: %s", cudaGetErrorString(e));
+    return RL_ERR_CUDA;
+  }
+  return RL_OK;
+}
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
@@ -840,6 +1087,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   CUtensorMap mw, ma;
   int rc = tc_make_map(&mw, W, N, K, K, BLOCK_N_OUT);
   if (rc != RL_OK) return rc;
+  if (bt > 128 && splits == 1 && pairs_pay(M, N)) return launch_tc_pair(mw, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
   fuse.tile_m = bt > 64 ? balanced_tile(M, bt) : bt;
   rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
   if (rc != RL_OK) return rc;

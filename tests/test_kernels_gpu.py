@@ -1265,6 +1265,25 @@ def test_gemm_tc_persistent_tiles_of_full_height(M):
     k.check_device_errors()
 
 
+@pytest.mark.parametrize("M,N,K_", [(129, 150 * 128 + 2, 8), (300, 75 * 256 - 130, 1032), (256, 75 * 256, 640), (777, 26 * 256 + 2, 2056)])
+def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
+    """More tiles of 256 x 256 than pairs of SMs, so pairs of CTAs take them: a K shorter than a block, rings that go round several times
+    with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave.  Float sums of K products."""
+    k = K()
+    assert k.gemm_tc_splits(M, N, K_) == 1
+    a, w = _rand(M, K_, dtype=torch.bfloat16, seed=1), _rand(N, K_, dtype=torch.bfloat16, seed=2)
+    ref = a.double() @ w.double().T
+    res = _rand(M + 3, N, seed=4)
+    out = res.clone()
+    k.gemm_tc(a, w, out[:M], k.OUT_ADD_F32)
+    torch.testing.assert_close(out[:M].double(), ref + res[:M].double(), rtol=1e-4, atol=8e-5 * math.sqrt(K_))
+    assert torch.equal(out[M:], res[M:])
+    again = res.clone()
+    k.gemm_tc(a, w, again[:M], k.OUT_ADD_F32)
+    assert torch.equal(out, again)
+    k.check_device_errors()
+
+
 # ----------------------------------------------------------------------------- 32-bit attention by tiles of rows
 @pytest.mark.parametrize("H,G,hd", [(4, 4, 64), (8, 2, 64), (15, 3, 64), (16, 1, 64), (3, 3, 128), (6, 1, 128), (28, 2, 128)])
 def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
