@@ -27,7 +27,12 @@
 //   O += P V    tcgen05.mma with P in tensor memory as A and the value tile as an
 //               MN-major B operand (values are stored [position][head_dim]); O stays in
 //               tensor memory over all key tiles
-// Tensor memory: S 0-255, O 256-.., P behind O (512 columns at head size 128).
+// Heads of 64 (keys and values): one buffer of S and of P, 256 columns of tensor memory, 96 KB of shared memory and 80 registers a
+// thread, so that two CTAs share an SM, and two threads a row, one for each half of a tile's keys, who exchange the halves'
+// maxima through shared memory; the running maximum stays in their registers.  With one CTA an SM its eight warps issued in 35 % of the
+// slots and the special-function unit ran 45 % of the time: two warps a scheduler do not cover one another's waits, and nothing
+// ran under a CTA's start and end.  Sixteen warps do better: 32 heads over 8, 8,192 tokens 504 -> 442 us, 4,096 141 -> 130.
+// Tensor memory: the S buffers, O behind them, P behind O (512 columns at head size 128).
 // A key tile is two cache pages (128 positions).  Warp 0 feeds TMA, warps 1 and 2 issue the two
 // products (a thread each: issuing blocks while the tensor pipe is full, and one thread's waits
 // and commits for one product would stand in the way of the other), warps 4-11 do the softmax and the final normalisation (with the registers that the
@@ -50,8 +55,6 @@ constexpr int TQ = 128;          // query rows per CTA
 constexpr int TK = 128;          // keys per tile = two pages
 constexpr int FA_THREADS = 384;       // warp 0: TMA, warp 1: S = Q K^T, warp 2: O += P V, warp 3: idle, warps 4-11: softmax
 constexpr int FA_PV_WARP = 2;
-// registers a thread: the first warpgroup hands most of its share to the two softmax warpgroups
-constexpr int FA_REGS_FEED = 56, FA_REGS_SOFTMAX = 224;
 constexpr uint32_t FA_WAIT_LIMIT = 1u << 22;
 constexpr int HALF_BYTES = 128 * 64 * 2;               // [128 rows x 64 bf16], 16 KB
 // sizes that depend on the widths of a key head HD and of a value head VD (64 or 128 each): halves of 64 dimensions
@@ -62,11 +65,20 @@ template <int HD, int VD> struct FaSizes {
   static constexpr int V_TILE_BYTES = V_HALVES * HALF_BYTES;   // a value tile
   // keys are asked for a tile further ahead than values: the scores of a tile are computed as soon as the
   // buffer is free, a whole tile before its P V
-  static constexpr int K_STAGES = HD == 64 ? 4 : 3;
-  static constexpr int V_STAGES = VD == 64 ? 3 : 2;
+  static constexpr bool TWO = HD == 64 && VD == 64;            // two CTAs an SM: what they hold fits twice (see above)
+  static constexpr int K_STAGES = TWO ? 3 : HD == 64 ? 4 : 3;
+  static constexpr int V_STAGES = TWO ? 2 : VD == 64 ? 3 : 2;
+  static constexpr int CTAS = TWO ? 2 : 1;
+  static constexpr int BUFS = TWO ? 1 : 2;                     // buffers of S and of P: tiles that are in the softmax at a time
+  static constexpr int SPLIT = TWO ? 2 : 1;                    // threads that share a row of a tile
+  static constexpr int GROUPS = 2;                             // groups of four softmax warps = BUFS * SPLIT
+  // registers a thread: the first warpgroup hands most of its share to the two softmax warpgroups (two CTAs an SM: 80 a
+  // thread at launch, 4 * 32 * 32 + 8 * 32 * 104 = 384 * 80)
+  static constexpr int REGS_FEED = TWO ? 32 : 56, REGS_SOFTMAX = TWO ? 104 : 224;
+  static constexpr int TMEM_COLS = TWO ? 256 : 512;
   // + alignment slack, barriers, and the softmax threads' exchange: running maxima (two tiles in turn), and the
   // groups' last maxima and sums
-  static constexpr int SMEM = Q_BYTES + K_STAGES * TILE_BYTES + V_STAGES * V_TILE_BYTES + 1024 + 512 + 3 * 2 * TQ * 4;
+  static constexpr int SMEM = Q_BYTES + K_STAGES * TILE_BYTES + V_STAGES * V_TILE_BYTES + 1024 + 512 + (2 + 2 * GROUPS + (SPLIT > 1 ? 2 * GROUPS : 0)) * TQ * 4;
 };
 constexpr float LAZY_LOG2 = 8.0f;                      // rescale O only when the maximum grew by more than 2^8
 
@@ -190,7 +202,7 @@ __host__ __device__ constexpr uint32_t fa_idesc(int m, int n, int b_mn) {
 }
 
 template <int HD, int VD>
-__global__ void __launch_bounds__(FA_THREADS, 1)
+__global__ void __launch_bounds__(FA_THREADS, FaSizes<HD, VD>::CTAS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ page_table, int max_pages,
                             const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slots,
@@ -203,7 +215,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   uint8_t* q_tile = smem;                                   // [2 halves][128 x 64]
   using SZ = FaSizes<HD, VD>;
   constexpr int HALVES = SZ::HALVES, V_HALVES = SZ::V_HALVES, Q_BYTES = SZ::Q_BYTES, TILE_BYTES = SZ::TILE_BYTES, V_TILE_BYTES = SZ::V_TILE_BYTES;
-  constexpr int K_STAGES = SZ::K_STAGES, V_STAGES = SZ::V_STAGES;
+  constexpr int K_STAGES = SZ::K_STAGES, V_STAGES = SZ::V_STAGES, BUFS = SZ::BUFS, SPLIT = SZ::SPLIT, GROUPS = SZ::GROUPS;
   uint8_t* k_ring = smem + Q_BYTES;                         // [stage][halves]
   uint8_t* v_ring = k_ring + K_STAGES * TILE_BYTES;         // [stage][halves]
   uint64_t* bars = (uint64_t*)(v_ring + V_STAGES * V_TILE_BYTES);
@@ -218,13 +230,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   uint64_t* pv_done = p_full + 2;          // [2]: the P V of a tile (by parity) has completed
   uint64_t* o_full = pv_done + 2;          // 1
   uint64_t* m_ready = o_full + 1;          // [tile parity][quarter]: the running maximum after a tile
-  uint32_t* tmem_slot = (uint32_t*)(m_ready + 8);
+  uint64_t* x_ready = m_ready + 8;         // [quarter]: both halves' maxima of a tile
+  uint32_t* tmem_slot = (uint32_t*)(x_ready + 4);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   int* s_seq = (int*)(tmem_slot + 2);
   int* s_tile = (int*)(tmem_slot + 3);
   float* m_shared = (float*)((uint8_t*)bars + 512);         // [tile parity][row]: running maximum after that tile
   float* x_m = m_shared + 2 * TQ;                            // [group][row]: the maximum the group's sum is scaled by
-  float* x_sum = x_m + 2 * TQ;                               // [group][row]
+  float* x_sum = x_m + GROUPS * TQ;                          // [group][row]
+  float* x_half = x_sum + GROUPS * TQ;                       // [tile parity][half][row] (two threads a row): the half's maximum
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -235,10 +249,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     for (int i = 0; i < V_STAGES; ++i) { fa_mbar_init(fa_smem_u32(&v_full[i]), 1); fa_mbar_init(fa_smem_u32(&v_empty[i]), 1); }
     for (int i = 0; i < 2; ++i) fa_mbar_init(fa_smem_u32(&s_full[i]), 1);
     for (int i = 0; i < 2; ++i) {
-      fa_mbar_init(fa_smem_u32(&s_free[i]), 4); fa_mbar_init(fa_smem_u32(&p_full[i]), 4);
+      fa_mbar_init(fa_smem_u32(&s_free[i]), 4 * SPLIT); fa_mbar_init(fa_smem_u32(&p_full[i]), 4 * SPLIT);
       fa_mbar_init(fa_smem_u32(&pv_done[i]), 1);
     }
     for (int i = 0; i < 8; ++i) fa_mbar_init(fa_smem_u32(&m_ready[i]), 1);
+    for (int i = 0; i < 4; ++i) fa_mbar_init(fa_smem_u32(&x_ready[i]), 2);
     fa_mbar_init(fa_smem_u32(o_full), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -247,7 +262,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_smem_u32(tmem_slot)), "r"((uint32_t)SZ::TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   rl_pdl_wait();       // everything below reads what earlier kernels of the step wrote
@@ -272,8 +287,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   __syncthreads();
   fa_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // S buffers at columns 0 and 128, O at 256, the two P buffers (64 columns each) behind O
-  const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + 256, tmem_p = tmem_base + 256 + VD;
+  // the S buffers (128 columns each), O behind them, the P buffers (64 columns each) behind O
+  const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + BUFS * TK, tmem_p = tmem_base + BUFS * TK + VD;
   const int b = *s_seq;
   const bool have_work = b < num_seqs;      // the grid is sized exactly; defensive
   const int h = blockIdx.x, gkv = h / (H / G);
@@ -298,7 +313,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   if (warp < 4) {
     // ---- the feeding warps: a few registers are enough; the rest goes to the softmax warps ----
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA_REGS_FEED));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SZ::REGS_FEED));
     if (warp == 0) {
       if (lane == 0 && have_work) {
         // ---------------- TMA producer ----------------
@@ -345,8 +360,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // way of the other.  They need no order between them: every dependency is an mbarrier.
         constexpr uint32_t idesc_s = fa_idesc(TQ, TK, 0);     // both K-major
         bool ok = fa_wait(fa_smem_u32(q_full), 0, abort_flag);
-        auto issue_s = [&](int i) -> bool {                   // scores of tile i into S buffer i % 2
-          const int st = i % K_STAGES, sb = i & 1;
+        auto issue_s = [&](int i) -> bool {                   // scores of tile i into S buffer i % BUFS
+          const int st = i % K_STAGES, sb = i % BUFS;
           if (!fa_wait(fa_smem_u32(&k_full[st]), (i / K_STAGES) & 1, abort_flag)) return false;
           fa_fence_after();
           uint8_t* base = k_ring + (size_t)st * TILE_BYTES;
@@ -361,12 +376,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           return true;
         };
         if (ok && num_kt > 0) ok = issue_s(0);
-        if (ok && num_kt > 1) ok = issue_s(1);
-        for (int i = 0; i + 2 < num_kt && ok; ++i) {
-          // the scores of the tile after next, as soon as this tile's are in its threads' registers:
-          // they are computed while this tile and the next are being exponentiated
-          ok = fa_wait(fa_smem_u32(&s_free[i & 1]), (i >> 1) & 1, abort_flag);
-          if (ok) ok = issue_s(i + 2);
+        if (BUFS > 1 && ok && num_kt > 1) ok = issue_s(1);
+        for (int i = 0; i + BUFS < num_kt && ok; ++i) {
+          // the scores of the buffer's next tile, as soon as this tile's are in its threads' registers:
+          // they are computed while this tile (with two buffers: and the next) is being exponentiated
+          ok = fa_wait(fa_smem_u32(&s_free[i % BUFS]), (i / BUFS) & 1, abort_flag);
+          if (ok) ok = issue_s(i + BUFS);
         }
         if (!ok && !*abort_flag) { *abort_flag = 1; atomicExch(err, 12); }
       }
@@ -377,16 +392,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         bool ok = true;
         for (int i = 0; i < num_kt && ok; ++i) {
           if (!fa_wait(fa_smem_u32(&v_full[i % V_STAGES]), (i / V_STAGES) & 1, abort_flag)) { ok = false; break; }
-          if (!fa_wait(fa_smem_u32(&p_full[i & 1]), (i >> 1) & 1, abort_flag)) { ok = false; break; }
+          if (!fa_wait(fa_smem_u32(&p_full[i % BUFS]), (i / BUFS) & 1, abort_flag)) { ok = false; break; }
           fa_fence_after();
           uint8_t* vbase = v_ring + (size_t)(i % V_STAGES) * V_TILE_BYTES;
 #pragma unroll
           for (int k = 0; k < TK / 16; ++k) {                 // 16 positions a step
             // P of this tile: 16 keys = 8 columns of packed bf16 pairs a step, in the P buffer of its parity
             const uint64_t db = fa_desc_mnmajor(fa_smem_u32(vbase + k * 16 * 128), HALF_BYTES);
-            fa_mma_a_tmem(tmem_o, tmem_p + (uint32_t)((i & 1) * (TK / 2) + 8 * k), db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+            fa_mma_a_tmem(tmem_o, tmem_p + (uint32_t)((i % BUFS) * (TK / 2) + 8 * k), db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
           }
-          fa_commit(fa_smem_u32(&pv_done[i & 1]));            // O, and this parity's P buffer, are free again once these have completed
+          fa_commit(fa_smem_u32(&pv_done[i % BUFS]));         // O, and this P buffer, are free again once these have completed
           fa_commit(fa_smem_u32(&v_empty[i % V_STAGES]));
         }
         if (ok) fa_commit(fa_smem_u32(o_full));
@@ -394,11 +409,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FA_REGS_SOFTMAX));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SZ::REGS_SOFTMAX));
     if (have_work) {
-      // ---------------- softmax warps: group 0 takes the even key tiles, group 1 the odd ones ----------------
-      constexpr int OC = VD / 2;                              // output columns a thread writes at the end
+      // ---------------- softmax warps.  Two buffers: group 0 takes the even key tiles, group 1 the odd ones.  One buffer:
+      // group 0 takes the first half of every tile's keys, group 1 the second ----------------
+      constexpr int OC = VD / GROUPS;                         // output columns a thread writes at the end
+      constexpr int CW = TK / SPLIT;                          // keys of a tile that a thread takes
       const int quarter = warp & 3, grp = (warp - 4) >> 2;
+      const int sb = grp / SPLIT, half = grp % SPLIT;         // its buffer; its part of the keys
       const int r = quarter * 32 + lane;                      // row of the tile = lane of tensor memory
       const int pos = start_pos + qt0 + r;                    // position of this row's query
       const int lo = chunk > 0 ? pos - pos % chunk : pos + 1 - window;   // the first position it sees (kept first tokens aside)
@@ -406,17 +424,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       float m_mine = -INFINITY, l_run = 0.f;                  // maximum this group's sum is scaled by; the sum
       bool ok = true;                                         // warp-uniform
       const float2 sc2 = make_float2(scale_log2e, scale_log2e);
-      for (int i = grp; i < num_kt && ok; i += 2) {
-        const int sb = grp, key0 = tile_of(i) * TK;           // S buffer = tile parity = group
-        ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&s_full[sb]), (i >> 1) & 1, abort_flag));
+      for (int i = sb; i < num_kt && ok; i += BUFS) {
+        const int key0 = tile_of(i) * TK + half * CW;         // the thread's first key
+        ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&s_full[sb]), (i / BUFS) & 1, abort_flag));
         if (!ok) break;
         fa_fence_after();
-        const uint32_t s_addr = tmem_s0 + lane_addr + (uint32_t)(sb * TK);
-        // the row's 128 scores into registers with one wait; the S buffer is then free for the tile
+        const uint32_t s_addr = tmem_s0 + lane_addr + (uint32_t)(sb * TK + half * CW);
+        // the row's 128 (or 64) scores into registers with one wait; the S buffer is then free for the tile
         // after next.  Everything below is straight-line code over the registers
-        uint32_t sa[TK];
+        uint32_t sa[CW];
 #pragma unroll
-        for (int c = 0; c < TK / 32; ++c) fa_ld32(s_addr + 32 * c, sa + 32 * c);
+        for (int c = 0; c < CW / 32; ++c) fa_ld32(s_addr + 32 * c, sa + 32 * c);
         fa_wait_ld();
         fa_fence_before();
         __syncwarp();
@@ -426,35 +444,35 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           // (cap_in = scale / cap, cap_out = cap / scale) so that what follows stays as it is.
           // tanh(x) = 1 - 2 / (e^{2x} + 1): two fast special-function operations, absolute error about 1e-7
 #pragma unroll
-          for (int j = 0; j < TK; ++j) {
+          for (int j = 0; j < CW; ++j) {
             const float e2x = fa_exp2(__uint_as_float(sa[j]) * cap_in * 2.8853900817779268f);
             sa[j] = __float_as_uint(cap_out * (1.0f - __fdividef(2.0f, e2x + 1.0f)));
           }
         }
         // The tile on the diagonal (no window) has code of its own, by 32-key chunks; every other tile
         // runs straight-line code over all 128 scores, which the scheduler can reorder freely.
-        const bool diag = window <= 0 && chunk <= 0 && key0 + TK - 1 > start_pos + qt0;     // warp-uniform
-        int live = TK / 32;                     // diagonal tile: chunks that some row of this warp sees
+        const bool diag = window <= 0 && chunk <= 0 && key0 + CW - 1 > start_pos + qt0;     // warp-uniform
+        int live = CW / 32;                     // diagonal tile: chunks that some row of this warp sees
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
         if (!diag) {
           if (window > 0 || chunk > 0) {
 #pragma unroll
-            for (int j = 0; j < TK; ++j) {
+            for (int j = 0; j < CW; ++j) {
               const int key = key0 + j;
               if (!(key <= pos && (key >= lo || key < keep_first))) sa[j] = 0xff800000u;          // -inf
             }
           }
 #pragma unroll
-          for (int j = 0; j < TK; j += 2) mx4[(j >> 1) & 3] = fa_max3(mx4[(j >> 1) & 3], __uint_as_float(sa[j]), __uint_as_float(sa[j + 1]));
+          for (int j = 0; j < CW; j += 2) mx4[(j >> 1) & 3] = fa_max3(mx4[(j >> 1) & 3], __uint_as_float(sa[j]), __uint_as_float(sa[j + 1]));
         } else {
           // key j of the tile is visible to this row if j <= lim.  Rows grow with the lane, so the chunks
           // left of the warp's first row's limit need no mask, and those right of its last row's limit
           // are dropped whole: no maxima, no exponentials, P = 0
           const int lim = pos - key0;
           const int lim0 = __shfl_sync(0xffffffffu, lim, 0), lim31 = __shfl_sync(0xffffffffu, lim, 31);
-          live = lim31 < 0 ? 0 : min(TK / 32, (lim31 >> 5) + 1);
+          live = lim31 < 0 ? 0 : min(CW / 32, (lim31 >> 5) + 1);
 #pragma unroll
-          for (int c = 0; c < TK / 32; ++c) {
+          for (int c = 0; c < CW / 32; ++c) {
             if (c < live) {
               if (32 * c + 31 > lim0) {
 #pragma unroll
@@ -466,20 +484,33 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
           }
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2e;
-        // the running maximum after the tile before (the other group's), and after this one: lazy, moved
+        float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2e;
+        if constexpr (SPLIT > 1) {
+          // the row's other half, through shared memory.  Places take turns by tile parity: a warp writes the place of the
+          // tile after next behind the next tile's barrier, where the other warp arrives when it has read this tile's
+          float* xh = x_half + (i & 1) * SPLIT * TQ;
+          xh[half * TQ + r] = mx;
+          __syncwarp();
+          if (lane == 0) fa_arrive(fa_smem_u32(&x_ready[quarter]));
+          ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&x_ready[quarter]), i & 1, abort_flag));
+          if (!ok) break;
+          mx = fmaxf(mx, xh[(half ^ 1) * TQ + r]);
+        }
+        // the running maximum after the tile before (two buffers: the other group's), and after this one: lazy, moved
         // (with O and the sums rescaled) only when it grew by more than 2^8
-        float m_prev = -INFINITY;
-        if (i > 0) {
+        float m_prev = BUFS > 1 ? -INFINITY : m_mine;
+        if (BUFS > 1 && i > 0) {
           ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&m_ready[((i - 1) & 1) * 4 + quarter]), ((i - 1) >> 1) & 1, abort_flag));
           if (!ok) break;
           m_prev = m_shared[((i - 1) & 1) * TQ + r];
         }
         float m_now = m_prev;
         if (mx > m_prev + LAZY_LOG2 || (m_prev == -INFINITY && mx > -INFINITY)) m_now = mx;
-        m_shared[(i & 1) * TQ + r] = m_now;
-        __syncwarp();
-        if (lane == 0) fa_arrive(fa_smem_u32(&m_ready[(i & 1) * 4 + quarter]));   // the next tile's threads may go on
+        if (BUFS > 1) {
+          m_shared[(i & 1) * TQ + r] = m_now;
+          __syncwarp();
+          if (lane == 0) fa_arrive(fa_smem_u32(&m_ready[(i & 1) * 4 + quarter]));   // the next tile's threads may go on
+        }
         const float corr = m_now != m_prev ? fa_exp2(m_prev - m_now) : 1.0f;       // 0 on the first visible tile
         const bool any_rescale = __any_sync(0xffffffffu, corr != 1.0f);
         if (m_mine != m_now) { l_run *= fa_exp2(m_mine - m_now); m_mine = m_now; }
@@ -497,7 +528,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         };
         if (!diag) {
 #pragma unroll
-          for (int j = 0; j < TK; j += 2) {
+          for (int j = 0; j < CW; j += 2) {
             const float2 t = fa_ffma2(make_float2(__uint_as_float(sa[j]), __uint_as_float(sa[j + 1])), sc2, nm2);
             const float2 p2 = make_float2(fa_exp2(t.x), fa_exp2(t.y));
             sum2[(j >> 1) & 3] = fa_fadd2(sum2[(j >> 1) & 3], p2);
@@ -506,7 +537,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           }
         } else {
 #pragma unroll
-          for (int c = 0; c < TK / 32; ++c) {
+          for (int c = 0; c < CW / 32; ++c) {
             if (c < live) {
 #pragma unroll
               for (int j = 32 * c; j < 32 * c + 32; j += 2) soft2(j);
@@ -516,23 +547,25 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
           }
         }
-        // the P buffer of this parity is free once the P V of the tile two back has completed; the barriers
+        // the P buffer is free once the P V of its last tile has completed; with two buffers the barriers
         // take turns by tile parity, and this thread waited for the tile four back on the same one
-        if (i >= 2) {
-          ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&pv_done[i & 1]), ((i - 2) >> 1) & 1, abort_flag));
+        if (i >= BUFS) {
+          ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&pv_done[sb]), ((i - BUFS) / BUFS) & 1, abort_flag));
           if (!ok) break;
         }
-        // O is only touched once the previous tile's P V has completed: waited for only if this warp has a
-        // row to rescale (the tile three back is done, as the one two back is; the barrier cannot have run
-        // ahead: the next P V needs our arrival)
+        // O is only touched once the previous tile's P V has completed (two buffers: waited for only if this warp has a
+        // row to rescale; the tile three back is done, as the one two back is; the barrier cannot have run
+        // ahead: the next P V needs our arrival).  Threads that share a row rescale a part of it each
         if (any_rescale && i > 0) {
-          ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&pv_done[(i - 1) & 1]), ((i - 1) >> 1) & 1, abort_flag));
-          if (!ok) break;
+          if (BUFS > 1) {
+            ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(&pv_done[(i - 1) & 1]), ((i - 1) >> 1) & 1, abort_flag));
+            if (!ok) break;
+          }
           fa_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < VD / 32; ++c) {               // the whole row of O
+          for (int c = 0; c < VD / 32 / SPLIT; ++c) {
             uint32_t v[32];
-            const uint32_t o_addr = tmem_o + lane_addr + (uint32_t)(c * 32);
+            const uint32_t o_addr = tmem_o + lane_addr + (uint32_t)(half * (VD / SPLIT) + c * 32);
             fa_ld32(o_addr, v);
             fa_wait_ld();
 #pragma unroll
@@ -543,16 +576,16 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         }
         fa_fence_after();
         // 16 keys are 8 columns of packed pairs
-        const uint32_t p_addr = tmem_p + lane_addr + (uint32_t)(sb * (TK / 2));
+        const uint32_t p_addr = tmem_p + lane_addr + (uint32_t)(sb * (TK / 2) + half * (CW / 2));
 #pragma unroll
-        for (int c = 0; c < TK / 32; ++c) fa_st16(p_addr + 16 * c, *reinterpret_cast<uint32_t(*)[16]>(sa + 16 * c));
+        for (int c = 0; c < CW / 32; ++c) fa_st16(p_addr + 16 * c, *reinterpret_cast<uint32_t(*)[16]>(sa + 16 * c));
         fa_wait_st();
         const float2 s01 = fa_fadd2(sum2[0], sum2[1]), s23 = fa_fadd2(sum2[2], sum2[3]);
         l_run += (s01.x + s01.y) + (s23.x + s23.y);
         // P is ready for the tensor cores
         fa_fence_before();
         __syncwarp();
-        if (lane == 0) fa_arrive(fa_smem_u32(&p_full[grp]));
+        if (lane == 0) fa_arrive(fa_smem_u32(&p_full[sb]));
       }
       // ---- O / l -> out ----
       if (ok) ok = __all_sync(0xffffffffu, fa_wait(fa_smem_u32(o_full), 0, abort_flag));
@@ -608,7 +641,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
   fa_fence_before();
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FaSizes<HD, VD>::TMEM_COLS) : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
