@@ -429,6 +429,9 @@ struct TcTail {
                      // grouped products: the CTAs that run together then share few groups' weights and token tiles
 };
 struct TcTileAt { int n0, m0, bt; };
+// A product a head in one launch (tiles 0: one product): heads lie one after another in the weight (N rows each), a_step columns
+// apart in the activations and out_step apart in the output; the walk goes head by head.
+struct TcHeads { int tiles, a_step, out_step; };
 __device__ __forceinline__ TcTileAt tc_tile_at(int tile, int tiles_m, int BT, const TcTail& t) {
   if (t.tiles_n > 0) return {(tile % t.tiles_n) * BLOCK_N_OUT, (tile / t.tiles_n) * BT, BT};
   if (tile < t.first) return {(tile / tiles_m) * BLOCK_N_OUT, (tile % tiles_m) * BT, BT};
@@ -445,7 +448,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                           const __grid_constant__ CUtensorMap map_a_tail, const float* __restrict__ bias,
                           void* __restrict__ out, int out_mode, int M, int N, int K,
                           int ldo, int* __restrict__ err, int tile_m, int tiles_m, int num_tiles, const TcTail tail,
-                          const int* __restrict__ tile_group, int group_rows, float act_limit, float act_alpha) {
+                          const int* __restrict__ tile_group, int group_rows, float act_limit, float act_alpha, const TcHeads heads) {
   // tile_group (null: none): the weight is stacked matrices of group_rows rows, and the token tile of BT rows at
   // m0 multiplies with matrix tile_group[m0 / BT]; negative: the tile is skipped by every role alike.  The table
   // is written by a kernel in front, so each role reads it behind its wait.
@@ -493,8 +496,9 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       bool waited = false, ok = true;
       if (tile_group != nullptr) { rl_pdl_wait(); waited = true; }
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
-        int n0 = at.n0;
+        const int head = heads.tiles > 0 ? tile / heads.tiles : 0, x0 = head * heads.a_step;
+        const TcTileAt at = tc_tile_at(tile - head * heads.tiles, tiles_m, tile_m, tail);
+        int n0 = at.n0 + head * N;
         const int m0 = at.m0;
         if (tile_group != nullptr) {
           const int group = tile_group[m0 / BT];
@@ -516,7 +520,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
           // weights may be requested before the preceding kernels have finished, activations not
           if (!waited) { rl_pdl_wait(); waited = true; }
           uint8_t* sa = st + BLOCK_N_OUT * BLOCK_K * 2;
-          tma_load_2d(smem_u32(sa), at.bt == tile_m ? &map_a : &map_a_tail, fb, kb * BLOCK_K, m0);
+          tma_load_2d(smem_u32(sa), at.bt == tile_m ? &map_a : &map_a_tail, fb, x0 + kb * BLOCK_K, m0);
         }
       }
     }
@@ -527,7 +531,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       bool ok = true;
       if (tile_group != nullptr) rl_pdl_wait();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const TcTileAt mat = tc_tile_at(tile, tiles_m, tile_m, tail);
+        const TcTileAt mat = tc_tile_at(heads.tiles > 0 ? tile % heads.tiles : tile, tiles_m, tile_m, tail);
         if (tile_group != nullptr && tile_group[mat.m0 / BT] < 0) continue;
         const uint32_t idesc = make_idesc(BLOCK_N_OUT, mat.bt);
         const int buf = t & 1;
@@ -568,7 +572,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     const int quarter = warp & 3, second = (warp - 2) >> 2;
     int t = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
+      const int head = heads.tiles > 0 ? tile / heads.tiles : 0;
+      const TcTileAt at = tc_tile_at(tile - head * heads.tiles, tiles_m, tile_m, tail);
       if (tile_group != nullptr && tile_group[at.m0 / BT] < 0) continue;
       const int buf = t & 1;
       const uint32_t acc_phase = (t >> 1) & 1;
@@ -581,8 +586,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
       fuse.act_limit = act_limit;
       fuse.act_alpha = act_alpha;
       const int cols = min(at.bt, M - at.m0), half = min(cols, (at.bt / 2 + 31) & ~31), c0 = second ? half : 0;
-      tile_epilogue<BT>(tmem_base + (uint32_t)(buf * BT + c0), quarter, lane, at.n0, at.m0 + c0, second ? cols - half : half, M, N, ldo, bias, out,
-                        out_mode, fuse, nullptr);
+      tile_epilogue<BT>(tmem_base + (uint32_t)(buf * BT + c0), quarter, lane, at.n0, at.m0 + c0, second ? cols - half : half, M, N, ldo, bias,
+                        (__nv_bfloat16*)out + (size_t)head * heads.out_step, out_mode, fuse, nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buf]));    // this warp has read the accumulator
@@ -607,7 +612,7 @@ static int balanced_tile(int M, int BT) {
 template <int BT>
 static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, const void* A, int lda, const float* bias,
                                 void* out, int out_mode, int M, int N, int K, int ldo, int* err, cudaStream_t stream,
-                                const TcFuse& fuse) {
+                                const TcFuse& fuse, int num_heads = 0, int a_step = 0, int out_step = 0) {
   const int* tile_group = fuse.tile_group;
   const int group_rows = fuse.group_rows;
   using Cfg = TcConfig<BT>;
@@ -621,13 +626,14 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
   const int tile_m = fuse.tile_m;
   const int tiles_m = (M + tile_m - 1) / tile_m, tiles_n = (N + BLOCK_N_OUT - 1) / BLOCK_N_OUT;
   const int total = tiles_m * tiles_n;
+  const TcHeads heads = {num_heads > 0 ? total : 0, a_step, out_step};
   // the tiles behind the last full wave: the narrowest token tile (from 64 tokens: below, the
   // weight tile's trip through shared memory takes longer than the products) that leaves no
   // more of them than there are CTAs
   TcTail tail = {total, tile_m, 0, 0, 0, 1, tile_group != nullptr ? tiles_n : 0};
-  int num_tiles = total;
+  int num_tiles = num_heads > 0 ? num_heads * total : total;
   const int full = (total / num_sms) * num_sms;
-  if (full < total && tile_group == nullptr) {      // grouped: a narrow tile could lie across two groups' rows
+  if (full < total && tile_group == nullptr && num_heads == 0) {      // grouped: a narrow tile could lie across two groups' rows
     const int n_first = full / tiles_m, t0_first = (full % tiles_m) * tile_m;
     for (int bt = 64; bt < tile_m; bt += 16) {
       const int count_first = (M - t0_first + bt - 1) / bt, per_n = (M + bt - 1) / bt;
@@ -647,7 +653,7 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
   cudaError_t e = rl_launch_pdl(gemm_tc_persistent_kernel<BT>, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)Cfg::SMEM_BYTES, stream,
                                 mw, ma, ma_tail, bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, tail, tile_group, group_rows,
-                                fuse.act_limit, fuse.act_alpha);
+                                fuse.act_limit, fuse.act_alpha, heads);
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_tc: launch of the persistent kernel failed: %s", cudaGetErrorString(e));
     return RL_ERR_CUDA;
@@ -1163,6 +1169,33 @@ extern "C" int rl_gemm_tc_grouped(const void* A, const void* W, void* out, int o
     case 128: return launch_tc_persistent<128>(mw, ma, A, lda, nullptr, out, out_mode, M, N, K, ldo, err, stream, fuse);
     default: return launch_tc_persistent<256>(mw, ma, A, lda, nullptr, out, out_mode, M, N, K, ldo, err, stream, fuse);
   }
+}
+
+// A product a head in one launch: out[m, h * out_step + n] = sum_k A[m, h * a_step + k] W[h, n, k] in bf16, W: [heads, N, K] contiguous.
+// K a multiple of 64 (a block of K must not reach into the next head's columns), a_step and lda multiples of 8.  For many
+// tokens: 16 heads, 2,000 tokens, 128 -> 512 and 512 -> 128 as a launch a head were bound by their launches.
+extern "C" int rl_gemm_tc_heads(const void* A, const void* W, void* out, int M, int N, int K, int lda, int ldo, int a_step, int out_step,
+                                int heads, int* err, cudaStream_t stream) {
+  RL_REQUIRE(heads > 0 && K % BLOCK_K == 0 && a_step >= K && a_step % 8 == 0 && out_step >= N && err != nullptr,
+             "rl_gemm_tc_heads: heads of %d (step %d) -> %d (step %d) are not supported: K must be a multiple of %d, the step in A of 8", K, a_step, N,
+             out_step, BLOCK_K);
+  const int width = (heads - 1) * a_step + K;
+  RL_REQUIRE(M > 0 && N > 0 && lda >= width && lda % 8 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0,
+             "rl_gemm_tc_heads: bad sizes, or bases that are not 16-byte aligned (M=%d N=%d lda=%d)", M, N, lda);
+  RL_REQUIRE(ldo >= (heads - 1) * out_step + N, "rl_gemm_tc_heads: output rows of %d do not hold %d heads", ldo, heads);
+  const long long rows = (long long)heads * N, most = (long long)heads * ((M + 63) / 64) * ((N + 127) / 128);
+  RL_REQUIRE(rows <= 2147483647LL && most <= 2147483647LL, "rl_gemm_tc_heads: too many weight rows or tiles");
+  TcFuse fuse = {};
+  CUtensorMap mw, ma;
+  int rc = tc_make_map(&mw, W, (int)rows, K, K, BLOCK_N_OUT);
+  if (rc != RL_OK) return rc;
+  const int bt = M <= 128 ? 128 : 256;
+  fuse.tile_m = balanced_tile(M, bt);
+  rc = tc_make_map(&ma, A, M, width, lda, fuse.tile_m);
+  if (rc != RL_OK) return rc;
+  if (bt == 128)
+    return launch_tc_persistent<128>(mw, ma, A, lda, nullptr, out, TC_OUT_BF16, M, N, K, ldo, err, stream, fuse, heads, a_step, out_step);
+  return launch_tc_persistent<256>(mw, ma, A, lda, nullptr, out, TC_OUT_BF16, M, N, K, ldo, err, stream, fuse, heads, a_step, out_step);
 }
 
 // 1 if rl_gemm_tc_qkv_rope takes the shape: head size 128 or 64, the whole head rotated, a step

@@ -153,6 +153,7 @@ _SIGNATURES = {
     "rl_moe_combine": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_gemm_tc_grouped": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                            _c_void_p, _c_int, _c_int, _c_float, _c_float, _c_void_p],
+    "rl_gemm_tc_heads": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_repeat_penalty": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p],
     "rl_argmax": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_sample_temperature": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -1130,6 +1131,26 @@ def heads_linear(x: torch.Tensor, x_head: int, w: torch.Tensor, out: torch.Tenso
         ldg = gate.stride(0) if M > 1 else H * N
     _check(library().rl_heads_linear(x.data_ptr(), ldx, int(x_head), w.data_ptr(), out.data_ptr(), ldo, int(out_head), _dt(x),
                                      M, H, N, Kd, _ptr(gate), ldg, _stream()), "rl_heads_linear")
+    _count()
+
+
+def gemm_tc_heads_supported(x: torch.Tensor, w: torch.Tensor, x_head: int) -> bool:
+    """Whether ``gemm_tc_heads`` takes these operands: bf16, more than 64 tokens, K a multiple of 64 (a block of K must not reach
+    into the next head's columns), rows and heads of ``x`` multiples of 8 elements apart, bases 16-byte aligned."""
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or not w.is_contiguous() or x.stride(1) != 1 or x.shape[0] <= 64:
+        return False
+    return (w.shape[2] % 64 == 0 and x_head % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_tc_heads(x: torch.Tensor, x_head: int, w: torch.Tensor, out: torch.Tensor, out_head: int) -> None:
+    """A product a head in one launch on the tensor cores, for many tokens: out[m, a * out_head + n] =
+    sum_k w[a, n, k] x[m, a * x_head + k].  x: [M, >= (H - 1) * x_head + K]; w: [H, N, K]; out: [M, >= (H - 1) * out_head + N]; all bf16."""
+    _need(x, "x", torch.bfloat16, contiguous=False); _need(w, "w", torch.bfloat16); _need(out, "out", torch.bfloat16, contiguous=False)
+    H, N, Kd = w.shape
+    M = x.shape[0]
+    assert out.stride(1) == 1 and out.shape[0] == M and x.shape[1] >= (H - 1) * x_head + Kd and out.shape[1] >= (H - 1) * out_head + N
+    _check(library().rl_gemm_tc_heads(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, Kd, x.stride(0), out.stride(0), int(x_head), int(out_head),
+                                      H, _tc_error_word(x.device).data_ptr(), _stream()), "rl_gemm_tc_heads")
     _count()
 
 

@@ -128,11 +128,13 @@ class LatentAttention(Mixer):
             linear(cq, self.wuq, q, OUT_SAME)
         ql = torch.empty((M, H * (r + rd)), dtype=dt, device=dev)       # a head: [Wuk^T q_plain | rot(q_rot)]
         K.latent_query(q, ql, H, hd, rd, r, step.positions, pos.inv_freq, pos.rotary_dim, pos.interleaved, magnitude=magnitude)
-        # a product a head: with few tokens they only stream weights and run as one launch; with many, one tensor-core
-        # product a head
+        # a product a head: with few tokens they only stream weights and run as one launch on the CUDA cores; with many, one
+        # launch on the tensor cores where no block of K reaches into the next head, else a launch a head
         few = M <= self.FEW_TOKENS and self.wuk.dtype == dt and self.wuv.dtype == dt
         if few and hd <= K.HEADS_LINEAR_MAX_K:
             K.heads_linear(q, hd + rd, self.wuk, ql, r + rd)
+        elif K.gemm_tc_heads_supported(q, self.wuk, hd + rd):
+            K.gemm_tc_heads(q, hd + rd, self.wuk, ql, r + rd)
         else:
             for a in range(H):
                 linear(q[:, a * (hd + rd):a * (hd + rd) + hd], self.wuk[a], ql[:, a * (r + rd):a * (r + rd) + r], OUT_SAME)
@@ -140,11 +142,15 @@ class LatentAttention(Mixer):
         K.attention(ql, k_pool, k_pool, group.page_table, step, ol, H, 1, r + rd, self.scale, self.window or 0, value_dim=r,
                     gate=gates if self.head_gate else None, gate_per_head=self.head_gate, values_in_keys=True)
         o = torch.empty((M, H * vd), dtype=dt, device=dev)
+        wuv = self.wuv.view(H, vd, r)
         if few and r <= K.HEADS_LINEAR_MAX_K:
-            K.heads_linear(ol, r, self.wuv.view(H, vd, r), o, vd, gate=gates if self.element_gate else None)
+            K.heads_linear(ol, r, wuv, o, vd, gate=gates if self.element_gate else None)
         else:
-            for a in range(H):
-                linear(ol[:, a * r:(a + 1) * r], self.wuv[a * vd:(a + 1) * vd], o[:, a * vd:(a + 1) * vd], OUT_SAME)
+            if K.gemm_tc_heads_supported(ol, wuv, r):
+                K.gemm_tc_heads(ol, r, wuv, o, vd)
+            else:
+                for a in range(H):
+                    linear(ol[:, a * r:(a + 1) * r], self.wuv[a * vd:(a + 1) * vd], o[:, a * vd:(a + 1) * vd], OUT_SAME)
             if self.element_gate:
                 K.sigmoid_gate(o, gates)
         return linear(o, self.wo, residual, _out_mode)

@@ -1284,6 +1284,24 @@ def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
     k.check_device_errors()
 
 
+@pytest.mark.parametrize("M,H,N,K_,gap", [(65, 3, 40, 64, 8), (129, 16, 512, 128, 64), (300, 5, 130, 192, 0), (1000, 2, 128, 512, 24)])
+def test_gemm_tc_heads_is_a_product_a_head(M, H, N, K_, gap):
+    """Heads that lie apart in wider rows on both sides; what lies between them stays as it is.  Float sums, one rounding to bf16."""
+    k = K()
+    x = _rand(M, H * (K_ + gap), dtype=torch.bfloat16, seed=1)
+    w = _rand(H, N, K_, dtype=torch.bfloat16, seed=2)
+    old = _rand(M, H * (N + 6), dtype=torch.bfloat16, seed=3)
+    out = old.clone()
+    assert k.gemm_tc_heads_supported(x, w, K_ + gap)
+    k.gemm_tc_heads(x, K_ + gap, w, out, N + 6)
+    got, was = out.view(M, H, N + 6), old.view(M, H, N + 6)
+    ref = torch.einsum("mhk,hnk->mhn", x.view(M, H, K_ + gap)[:, :, :K_].double(), w.double())
+    torch.testing.assert_close(got[:, :, :N].double(), ref, rtol=1e-2, atol=1e-3 * math.sqrt(K_))
+    assert torch.equal(got[:, :, N:], was[:, :, N:])
+    assert not k.gemm_tc_heads_supported(x, w[:, :, :K_ - 8].contiguous(), K_ + gap)      # a block of K would reach into the next head
+    k.check_device_errors()
+
+
 # ----------------------------------------------------------------------------- 32-bit attention by tiles of rows
 @pytest.mark.parametrize("H,G,hd", [(4, 4, 64), (8, 2, 64), (15, 3, 64), (16, 1, 64), (3, 3, 128), (6, 1, 128), (28, 2, 128)])
 def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
