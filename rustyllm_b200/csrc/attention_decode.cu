@@ -59,6 +59,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 #define DEC_STAGES 3
+#define DEC_MAX_CLUSTER 8   // chunks of a sequence that are one cluster
 __device__ __forceinline__ void dec_cp_async16(uint32_t dst, const void* src, int src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -469,14 +470,27 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv
     const int lo = split * per, hi = min(lo + per, m * VD);
     for (int idx = lo + threadIdx.x; idx < hi; idx += DEC_WARPS * 32) {
       const int r = idx / VD, d = idx % VD;
+      // all chunks' numbers requested before the first is used: one trip through the cluster's shared memory instead of
+      // one a chunk and loop
+      float mc[DEC_MAX_CLUSTER], lc[DEC_MAX_CLUSTER], oc[DEC_MAX_CLUSTER];
+#pragma unroll
+      for (int c = 0; c < DEC_MAX_CLUSTER; ++c) {
+        mc[c] = -INFINITY; lc[c] = oc[c] = 0.f;
+        if (c < num_splits) {
+          mc[c] = dec_peer_f32(c_o + 16 * VD + r, c);
+          lc[c] = dec_peer_f32(c_o + 16 * VD + 16 + r, c);
+          oc[c] = dec_peer_f32(c_o + r * VD + d, c);
+        }
+      }
       float M = -INFINITY;
-      for (int c = 0; c < num_splits; ++c) M = fmaxf(M, dec_peer_f32(c_o + 16 * VD + r, c));
+#pragma unroll
+      for (int c = 0; c < DEC_MAX_CLUSTER; ++c) M = fmaxf(M, mc[c]);
       float L = 0.f, O = 0.f;
-      for (int c = 0; c < num_splits; ++c) {
-        const float mc = dec_peer_f32(c_o + 16 * VD + r, c);
-        const float wgt = (mc > -INFINITY) ? exp2f(mc - M) : 0.f;
-        L += dec_peer_f32(c_o + 16 * VD + 16 + r, c) * wgt;
-        O += dec_peer_f32(c_o + r * VD + d, c) * wgt;
+#pragma unroll
+      for (int c = 0; c < DEC_MAX_CLUSTER; ++c) {
+        const float wgt = (mc[c] > -INFINITY) ? exp2f(mc[c] - M) : 0.f;
+        L += lc[c] * wgt;
+        O += oc[c] * wgt;
       }
       out[(size_t)b * ldo + (size_t)(gkv * m + r) * VD + d] = __float2bfloat16_rn(dec_finish(O, L, M, fin, b, (gkv * m + r) * VD + d));
     }
