@@ -347,6 +347,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---- all parts of the tile have their partial in shared memory ----
     __syncwarp();
     cluster_sync_all();
+    bool arrived = false;
     if (warp >= 2 && !*abort_flag) {
       // 32 lanes x 4 consecutive weight rows cover the 128 rows with 16-byte loads.  This CTA
       // owns the token columns j with j % parts == its rank; its epilogue warps take
@@ -388,6 +389,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
           for (int u = 0; u < U; ++u) { v[u].x += t[u].x; v[u].y += t[u].y; v[u].z += t[u].z; v[u].w += t[u].w; }
         }
+        if (j0 + step * U >= cols) {      // (warp-uniform) the last of this warp's reads: the other parts need not wait for its stores
+          __syncwarp();
+          cluster_arrive();
+          arrived = true;
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           const int j = j0 + u * step;
@@ -398,7 +404,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
     }
     __syncwarp();
-    cluster_sync_all();      // nobody leaves while another part still reads its shared memory
+    if (!arrived) cluster_arrive();
+    cluster_wait();          // nobody leaves while another part still reads its shared memory
   }
   tc_fence_before();
   __syncthreads();

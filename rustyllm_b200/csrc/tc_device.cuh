@@ -154,6 +154,9 @@ __device__ __forceinline__ uint32_t cluster_size() { uint32_t r; asm volatile("m
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the two halves of the above
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // address of the same shared-memory location in the cluster's CTA `rank`
 __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local_addr, uint32_t rank) {
   uint32_t r;
