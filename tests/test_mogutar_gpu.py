@@ -253,6 +253,38 @@ def test_norms_on_a_sublayers_output(dtype):
     torch.testing.assert_close(g.double().cpu(), P.gelu_tanh(t) * table[tokens][:, col0:col0 + width], **tol(dtype))
 
 
+@pytest.mark.parametrize("d", [3, 1024, 1025, 2048, 2050, 4096, 4097])
+def test_norm_and_add_at_the_edges_of_its_register_forms(d):
+    """Rows a thread holds 4, 8 or 16 values of, whole and with an end, and rows that are too long."""
+    from rustyllm_b200 import kernels as K
+    torch.manual_seed(d)
+    x, y0, y1 = (torch.randn(3, d, dtype=F64).float() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(d, dtype=F64)).float()
+    for terms in (1, 2):
+        xd, xb = x.clone().to(DEV), torch.empty((3, d), dtype=torch.bfloat16, device=DEV)
+        K.norm_add(xd, y0.to(DEV), 1.2, y1.to(DEV) if terms == 2 else None, 0.9, w.to(DEV), 1e-5, xb)
+        v = 1.2 * y0.double() + (0.9 * y1.double() if terms == 2 else 0.0)
+        torch.testing.assert_close(xd.double().cpu(), x.double() + P.rms_norm(v, w.double(), 1e-5), rtol=1e-5, atol=1e-5)
+        assert torch.equal(xb, xd.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,n,groups", [(600, 30, 7), (600, 128, 7), (600, 129, 7), (600, 512, 7), (600, 513, 7), (5, 1024, 1), (5, 1025, 2), (5, 2049, 1), (5, 4096, 1), (5, 4097, 1)])
+def test_gated_norm_at_the_edges_of_its_register_forms(dtype, M, n, groups):
+    """A warp or a block a group, 4, 8 or 16 values a thread, and groups that are too long."""
+    from rustyllm_b200 import kernels as K
+    torch.manual_seed(n)
+    y, gate = torch.randn(M, n * groups, dtype=F64).float(), rounded(torch.randn(M, n * groups, dtype=F64), dtype)
+    w = (1 + 0.1 * torch.randn(n * groups, dtype=F64)).float()
+    out = torch.empty((M, n * groups), dtype=tdt(dtype), device=DEV)
+    K.gated_norm(y.to(DEV), gate.to(tdt(dtype)).to(DEV), w.to(DEV), 1e-5, out, groups=groups, gate_act="silu", gate_first=True)
+    ref = P.rms_norm((y.double() * P.silu(gate)).view(M, groups, n), None, 1e-5).reshape(M, n * groups) * w.double()
+    torch.testing.assert_close(out.double().cpu(), ref, **tol(dtype))
+    if groups == 1:
+        K.gated_norm(y.to(DEV), gate.to(tdt(dtype)).to(DEV), w.to(DEV), 1e-5, out, groups=1, gate_act="sigmoid", gate_first=False)
+        torch.testing.assert_close(out.double().cpu(), P.rms_norm(y.double(), w.double(), 1e-5) * P.sigmoid(gate), **tol(dtype))
+
+
 @pytest.mark.parametrize("E,top,groups", [(12, 2, (3, 2)), (12, 3, (4, 1)), (6, 6, None), (9, 1, (9, 3)), (40, 3, (5, 2)), (7, 2, (1, 1))])
 @pytest.mark.parametrize("M", [5, 200])
 def test_router_with_sigmoid_scores_and_groups(E, top, groups, M):
