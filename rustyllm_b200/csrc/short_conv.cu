@@ -251,6 +251,123 @@ qkv_prepare_kernel(const T* __restrict__ u, int ldu, T* __restrict__ q_out, int 
   }
 }
 
+// The same for many tokens where all heads are 32 V wide and rotated whole or not at all: a warp takes one head of PREP_RUN
+// consecutive rows, a lane V neighbouring channels, so an input is loaded once a run instead of once a tap, in pieces of V, and the
+// filters, norm weights and frequencies once a run.  The pair (i, i + half) lies 16 lanes apart; each of the two lanes computes the
+// angles of half of its frequencies and they exchange them.  The kernel above waits for a load a channel and tap: 1,500 tokens of 24
+// heads with four taps, norms and rotation 36 -> 21 us.
+#define PREP_RUN 4
+template <typename T, int V, int TAPS>
+__global__ void __launch_bounds__(PREP_WARPS * 32)
+qkv_prepare_run_kernel(const T* __restrict__ u, int ldu, T* __restrict__ q_out, int ldq, const float* __restrict__ conv_w,
+                       const float* __restrict__ state, long long state_stride, const float* __restrict__ q_norm,
+                       const float* __restrict__ k_norm, float eps, const int* __restrict__ positions,
+                       const int* __restrict__ slot_of_token, const int* __restrict__ page_table, int max_pages,
+                       const float* __restrict__ inv_freq, int rot, float magnitude, int H, int G, T* __restrict__ k_pool,
+                       T* __restrict__ v_pool, int M) {
+  constexpr int HD = 32 * V;
+  rl_pdl_trigger();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hs = blockIdx.y * PREP_WARPS + warp;          // head slot: [0, H) queries, [H, H + G) keys, then G values
+  if (hs >= H + 2 * G) return;
+  const bool is_q = hs < H, is_v = hs >= H + G, rotate = !is_v && rot > 0;
+  const int C = (H + 2 * G) * HD, c = hs * HD + V * lane;
+  float f[V][TAPS], nw[V], freq[V / 2];
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) f[k][j] = TAPS > 1 ? conv_w[(size_t)(c + k) * TAPS + j] : 1.f;        // (one tap: no filter)
+  const float* norm = is_v ? nullptr : is_q ? q_norm : k_norm;
+#pragma unroll
+  for (int k = 0; k < V; ++k) nw[k] = norm ? norm[V * lane + k] : 1.f;
+  // frequencies V * (lane & 15) + k of the pair's first element: the lower lane takes the first V / 2 of them, the upper the rest
+  const bool low = lane < 16;
+#pragma unroll
+  for (int k = 0; k < V / 2; ++k) freq[k] = rotate ? inv_freq[V * (lane & 15) + (low ? 0 : V / 2) + k] : 0.f;
+  rl_pdl_wait();
+  u = rl_behind_wait(u);
+  const int m0 = blockIdx.x * PREP_RUN, rows = min(PREP_RUN, M - m0);
+  ConvVec<T, V> in[PREP_RUN];
+  int slots[PREP_RUN], pos[PREP_RUN];
+#pragma unroll
+  for (int r = 0; r < PREP_RUN; ++r)
+    if (r < rows) {
+      in[r] = *reinterpret_cast<const ConvVec<T, V>*>(u + (size_t)(m0 + r) * ldu + c);
+      slots[r] = slot_of_token[m0 + r];
+      pos[r] = positions[m0 + r];
+    }
+  float hist[V][TAPS];                   // hist[k][j]: the input TAPS - 1 - j positions back; [TAPS - 1] is the row's own
+#pragma unroll
+  for (int r = 0; r < PREP_RUN; ++r) {
+    if (r >= rows) break;
+    const int m = m0 + r;
+    if constexpr (TAPS > 1) {
+      if (r == 0 || slots[r] != slots[r > 0 ? r - 1 : 0]) {
+        const int n = r == 0 ? conv_rows_back(slot_of_token, m, TAPS) : 0;
+        const float* st = state + (size_t)slots[r] * state_stride;
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+#pragma unroll
+          for (int j = 0; j < TAPS - 1; ++j) hist[k][j] = conv_input(u, ldu, st, C, TAPS, m, n, TAPS - 1 - j, c + k);
+      } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+#pragma unroll
+          for (int j = 0; j < TAPS - 1; ++j) hist[k][j] = hist[k][j + 1];
+      }
+    }
+    float val[V], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      hist[k][TAPS - 1] = rl_ld(&in[r].v[k]);
+      if constexpr (TAPS > 1) {
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) acc = fmaf(f[k][j], hist[k][j], acc);
+        val[k] = acc;
+      } else {
+        val[k] = hist[k][0];
+      }
+      ss = fmaf(val[k], val[k], ss);
+    }
+    if (norm) {
+      const float q = 1.0f / sqrtf(rl_warp_sum(ss) / (float)HD + eps);
+#pragma unroll
+      for (int k = 0; k < V; ++k) val[k] = val[k] * q * nw[k];
+    }
+    if (rotate) {
+      float sn[V], cs[V];
+#pragma unroll
+      for (int k = 0; k < V / 2; ++k) {
+        float a, b;
+        sincosf((float)pos[r] * freq[k], &a, &b);
+        a *= magnitude;
+        b *= magnitude;
+        const float oa = __shfl_xor_sync(0xffffffffu, a, 16), ob = __shfl_xor_sync(0xffffffffu, b, 16);
+        sn[k] = low ? a : oa; sn[k + V / 2] = low ? oa : a;
+        cs[k] = low ? b : ob; cs[k + V / 2] = low ? ob : b;
+      }
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const float other = __shfl_xor_sync(0xffffffffu, val[k], 16);
+        val[k] = low ? val[k] * cs[k] - other * sn[k] : val[k] * cs[k] + other * sn[k];
+      }
+    }
+    T* dst;
+    if (is_q) {
+      dst = q_out + (size_t)m * ldq + (size_t)hs * HD;
+    } else {
+      if (k_pool == nullptr) continue;
+      const int page = page_table[(size_t)slots[r] * max_pages + pos[r] / RL_PAGE];
+      dst = (is_v ? v_pool : k_pool) + (((size_t)page * G + (hs - H - (is_v ? G : 0))) * RL_PAGE + pos[r] % RL_PAGE) * HD;
+    }
+    ConvVec<T, V> res;
+#pragma unroll
+    for (int k = 0; k < V; ++k) rl_st(&res.v[k], val[k]);
+    *reinterpret_cast<ConvVec<T, V>*>(dst + V * lane) = res;
+  }
+}
+
 // u [M, ldu] (channels [0, C)), w float [C, taps], bias float [C] or null, act 0 none / 1 silu,
 // state float [slots, state_stride] (this convolution's [taps - 1, C] at the given pointer), out [M, ldo].
 // rl_short_conv_parts: the output as equal parts of `part` channels, each a matrix [M, ldo] of its own, out_part
@@ -345,6 +462,22 @@ extern "C" int rl_qkv_prepare(const void* u, int ldu, void* q_out, int ldq, int 
              "rl_qkv_prepare: row strides too small");
   RL_REQUIRE((k_pool == nullptr) == (v_pool == nullptr), "rl_qkv_prepare: give both cache pools or none");
   if (num_tokens == 0) return RL_OK;
+  // many bf16 tokens, heads of 128 (four channels a lane, 8 bytes) all alike, rotated whole or not at all: by runs of rows
+  if (dtype == RL_BF16 && num_tokens >= 128 && head_dim == 128 && value_dim == 128 && (rotary_dim == 0 || rotary_dim == head_dim) &&
+      (conv_w == nullptr || taps == 4) && ldu % 4 == 0 && ldq % 4 == 0 &&
+      (((uintptr_t)u | (uintptr_t)q_out | (uintptr_t)k_pool | (uintptr_t)v_pool) & 7) == 0) {
+    const dim3 runs((num_tokens + PREP_RUN - 1) / PREP_RUN, (num_heads + 2 * num_kv_heads + PREP_WARPS - 1) / PREP_WARPS);
+#define RL_PREP_RUN(TAPS)                                                                                                            \
+  rl_launch_pdl(qkv_prepare_run_kernel<__nv_bfloat16, 4, TAPS>, runs, PREP_WARPS * 32, 0, stream, (const __nv_bfloat16*)u, ldu,     \
+                (__nv_bfloat16*)q_out, ldq, conv_w, state, state_stride, q_norm, k_norm, eps, positions, slot_of_token, page_table, \
+                max_pages, inv_freq, rotary_dim, magnitude, num_heads, num_kv_heads, (__nv_bfloat16*)k_pool, (__nv_bfloat16*)v_pool, \
+                num_tokens)
+    if (conv_w) RL_PREP_RUN(4);
+    else RL_PREP_RUN(1);      // no filter
+#undef RL_PREP_RUN
+    RL_LAUNCH_CHECK("rl_qkv_prepare");
+    return RL_OK;
+  }
   const dim3 grid(num_tokens, (num_heads + 2 * num_kv_heads + PREP_WARPS - 1) / PREP_WARPS);
   if (dtype == RL_F32)
     rl_launch_pdl(qkv_prepare_kernel<float>, grid, PREP_WARPS * 32, 0, stream, (const float*)u, ldu, (float*)q_out, ldq, conv_w, taps,

@@ -285,6 +285,43 @@ def test_gated_norm_at_the_edges_of_its_register_forms(dtype, M, n, groups):
         torch.testing.assert_close(out.double().cpu(), P.rms_norm(y.double(), w.double(), 1e-5) * P.sigmoid(gate), **tol(dtype))
 
 
+@pytest.mark.parametrize("taps,norm,rot", [(4, True, 128), (4, False, 128), (None, True, 0), (4, False, 0), (None, False, 128)])
+def test_prepared_heads_of_many_tokens_as_by_the_general_kernel(taps, norm, rot):
+    """Runs of rows that begin inside, at and behind a sequence's start, sequences shorter than the filter and than a run, a last run that is
+    not whole; against the kernel that takes a token and head at a time (an output that begins between two 8-byte pieces sends the
+    call there).  Without norms and rotation the same bits; with them float sums and products are rounded in another order: one bf16
+    rounding may flip."""
+    from rustyllm_b200 import kernels as K
+    torch.manual_seed(7)
+    H, G, hd, bf = 5, 2, 128, torch.bfloat16
+    lens, before = [1, 2, 3, 150, 6, 9], [0, 70, 1, 3, 0, 200]
+    M, C = sum(lens), (H + 2 * G) * hd
+    slots = [4, 0, 2, 5, 1, 3]
+    slot_of = i32([s for s, n in zip(slots, lens) for _ in range(n)])
+    pos = i32([b + i for b, n in zip(before, lens) for i in range(n)])
+    pages = torch.randperm(6 * 4).to(torch.int32).view(6, 4).to(DEV)
+    u = torch.randn(M, C, device=DEV).to(bf)
+    w = torch.randn(C, taps, device=DEV) if taps else None
+    state = None
+    if taps:
+        area, state = state_area(6, 4 * 3 * C)
+        state.view(torch.float32).copy_(torch.randn(6, 3 * C))
+    qn, kn = (1 + 0.1 * torch.randn(hd, device=DEV) for _ in range(2))
+    freq = torch.rand(64, device=DEV)
+    got = []
+    for pad in (0, 1):
+        q = torch.zeros(M * H * hd + pad, dtype=bf, device=DEV)[pad:].view(M, H * hd)
+        kp, vp = (torch.zeros(24, G, 64, hd, dtype=bf, device=DEV) for _ in range(2))
+        K.qkv_prepare(u, q, w, state, qn if norm else None, kn if norm else None, 1e-5, pos, slot_of, pages, freq, rot, 1.1, H, G, hd, hd, kp, vp)
+        got.append((q, kp, vp))
+    for a, b in zip(*got):
+        if norm or rot:
+            torch.testing.assert_close(a.float(), b.float(), rtol=2.0 ** -7, atol=2.0 ** -12)
+        else:
+            assert torch.equal(a, b)
+    assert torch.equal(got[0][2], got[1][2])
+
+
 @pytest.mark.parametrize("E,top,groups", [(12, 2, (3, 2)), (12, 3, (4, 1)), (6, 6, None), (9, 1, (9, 3)), (40, 3, (5, 2)), (7, 2, (1, 1))])
 @pytest.mark.parametrize("M", [5, 200])
 def test_router_with_sigmoid_scores_and_groups(E, top, groups, M):
