@@ -57,7 +57,7 @@ constexpr int FA_THREADS = 384;       // warp 0: TMA, warp 1: S = Q K^T, warp 2:
 constexpr int FA_PV_WARP = 2;
 constexpr uint32_t FA_WAIT_LIMIT = 1u << 22;
 constexpr int HALF_BYTES = 128 * 64 * 2;               // [128 rows x 64 bf16], 16 KB
-// sizes that depend on the widths of a key head HD and of a value head VD (64 or 128 each): halves of 64 dimensions
+// sizes that depend on the widths of a key head HD (64, 128 or 192) and of a value head VD (64 or 128): halves of 64 dimensions
 template <int HD, int VD> struct FaSizes {
   static constexpr int HALVES = HD / 64, V_HALVES = VD / 64;
   static constexpr int Q_BYTES = HALVES * HALF_BYTES;          // 16 or 32 KB
@@ -66,7 +66,9 @@ template <int HD, int VD> struct FaSizes {
   // keys are asked for a tile further ahead than values: the scores of a tile are computed as soon as the
   // buffer is free, a whole tile before its P V
   static constexpr bool TWO = HD == 64 && VD == 64;            // two CTAs an SM: what they hold fits twice (see above)
-  static constexpr int K_STAGES = TWO ? 3 : HD == 64 ? 4 : 3;
+  // heads of 192: 128 key dimensions of their own and 64 that all heads share (see rl_attention_prefill_tc_shared_part)
+  static constexpr bool SHARED_PART = HD == 192;
+  static constexpr int K_STAGES = SHARED_PART ? 2 : TWO ? 3 : HD == 64 ? 4 : 3;
   static constexpr int V_STAGES = TWO ? 2 : VD == 64 ? 3 : 2;
   static constexpr int CTAS = TWO ? 2 : 1;
   static constexpr int BUFS = TWO ? 1 : 2;                     // buffers of S and of P: tiles that are in the softmax at a time
@@ -209,7 +211,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int* __restrict__ kv_lens, int num_seqs, __nv_bfloat16* __restrict__ out, int ldo,
                             int H, int G, float scale_log2e, int window, int* __restrict__ err,
                             const int* __restrict__ tile_order, int sink, const __nv_bfloat16* __restrict__ gate, int ldg,
-                            float cap_in, float cap_out, int keep_first, int chunk, int gate_per_head, const float* __restrict__ sinks) {
+                            float cap_in, float cap_out, int keep_first, int chunk, int gate_per_head, const float* __restrict__ sinks,
+                            const __grid_constant__ CUtensorMap map_shared, int shared_col) {
   extern __shared__ uint8_t fa_smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)fa_smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* q_tile = smem;                                   // [2 halves][128 x 64]
@@ -327,14 +330,21 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
           const int kt = tile_of(i), st = i % (values ? V_STAGES : K_STAGES);
           const int p0 = pages[2 * kt];
           const int p1 = (2 * kt + 1) * RL_PAGE < kv_len ? pages[2 * kt + 1] : p0;   // beyond the sequence: any valid page (all masked)
-          const int r0 = (p0 * G + gkv) * RL_PAGE, r1 = (p1 * G + gkv) * RL_PAGE;
+          // pages of a head's rows; with a shared part: rows of all heads side by side
+          const int r0 = (SZ::SHARED_PART ? p0 : p0 * G + gkv) * RL_PAGE, r1 = (SZ::SHARED_PART ? p1 : p1 * G + gkv) * RL_PAGE;
           const uint32_t fb = fa_smem_u32(values ? &v_full[st] : &k_full[st]);
           uint8_t* base = values ? v_ring + (size_t)st * V_TILE_BYTES : k_ring + (size_t)st * TILE_BYTES;
           const CUtensorMap* map = values ? &map_v : &map_k;
           fa_expect_tx(fb, values ? V_TILE_BYTES : TILE_BYTES);
           for (int half = 0; half < (values ? V_HALVES : HALVES); ++half) {     // 64 head dimensions a half; 64 positions a page
-            fa_tma_2d(fa_smem_u32(base + half * HALF_BYTES), map, fb, 64 * half, r0);
-            fa_tma_2d(fa_smem_u32(base + half * HALF_BYTES + 64 * 128), map, fb, 64 * half, r1);
+            int x = 64 * half;
+            const CUtensorMap* from = map;
+            if constexpr (SZ::SHARED_PART) {
+              if (!values && half == HALVES - 1) { from = &map_shared; x = shared_col; }
+              else x += h * (values ? VD : HD - 64);
+            }
+            fa_tma_2d(fa_smem_u32(base + half * HALF_BYTES), from, fb, x, r0);
+            fa_tma_2d(fa_smem_u32(base + half * HALF_BYTES + 64 * 128), from, fb, x, r1);
           }
         };
         auto stage_free = [&](uint64_t* empty, int stages, int i) -> bool {      // without waiting
@@ -753,10 +763,47 @@ extern "C" int rl_attention_prefill_tc_wide(const void* q, int ldq, const void* 
 #define FA_GO(HD, VD)                                                                                                          \
   fa_launch<HD, VD>(dim3(num_heads, num_tiles), stream, mq, mk, mv, page_table, max_pages, cu_seqlens, seq_slots, kv_lens,     \
                     num_seqs, (__nv_bfloat16*)out, ldo, num_heads, num_kv_heads, scale * 1.4426950408889634f, window, err,      \
-                    tile_order, sink, (const __nv_bfloat16*)gate, ldg, cap_in, cap_out, keep_first, chunk, gate_per_head, sinks)
+                    tile_order, sink, (const __nv_bfloat16*)gate, ldg, cap_in, cap_out, keep_first, chunk, gate_per_head, sinks, mk, 0)
   if (head_dim == 64) return value_dim == 64 ? FA_GO(64, 64) : FA_GO(64, 128);
   return value_dim == 64 ? FA_GO(128, 64) : FA_GO(128, 128);
 #undef FA_GO
+}
+
+// For attention through a latent whose keys and values were made (parts/latent.py): a pair of positions takes 2 x (192 + 128) operations a head
+// on tcgen05 where the heads over one cached row (attention_shared_key.cu, mma.sync) take 2 x (576 + 512).
+// Key heads of 192, of which the last 64 dimensions are the same row for all heads, value heads of 128, neither in a paged pool: keys
+// [rows, num_heads * 128] and values [rows, num_heads * 128] hold a position's heads side by side, the shared part lies in columns
+// shared_col .. + 64 of shared [rows, ld_shared]; positions lie in runs of RL_PAGE rows, entry p of a sequence's table being the run
+// of positions p * RL_PAGE on (rows behind the sequence's end hold finite values).  q [M, num_heads * 192].  The rest as above.
+extern "C" int rl_attention_prefill_tc_shared_part(const void* q, int ldq, const void* keys, const void* values, const void* shared,
+                                                   int ld_shared, int shared_col, int num_runs, const int* run_table, int max_runs,
+                                                   const int* cu_seqlens, const int* table_rows, const int* kv_lens, int num_seqs,
+                                                   int num_tiles, int num_tokens, void* out, int ldo, int num_heads, float scale, int window,
+                                                   int* err, const int* tile_order, const void* gate, int ldg, int gate_per_head,
+                                                   cudaStream_t stream) {
+  RL_REQUIRE(gate == nullptr || (gate_per_head && ldg >= num_heads) || (!gate_per_head && ldg >= num_heads * 128 && ldg % 8 == 0 && ((uintptr_t)gate & 15) == 0),
+             "rl_attention_prefill_tc_shared_part: the gate must be 16-byte aligned with a row stride that is a multiple of 8 and holds all heads");
+  RL_REQUIRE(num_heads > 0 && num_seqs >= 0 && num_tiles >= 0 && num_tiles <= 65535 && num_tokens >= 0 && num_runs > 0 && scale > 0.f && window >= 0 && err != nullptr,
+             "rl_attention_prefill_tc_shared_part: bad sizes");
+  RL_REQUIRE(ldq >= num_heads * 192 && ldq % 8 == 0 && ldo >= num_heads * 128 && ldo % 8 == 0 && ld_shared % 8 == 0 && shared_col % 8 == 0 &&
+             shared_col >= 0 && ld_shared >= shared_col + 64,
+             "rl_attention_prefill_tc_shared_part: row strides and columns must be multiples of 8 elements and hold all heads");
+  RL_REQUIRE((((uintptr_t)q | (uintptr_t)out | (uintptr_t)keys | (uintptr_t)values | (uintptr_t)shared) & 15) == 0,
+             "rl_attention_prefill_tc_shared_part: pointers must be 16-byte aligned");
+  if (num_seqs == 0 || num_tiles == 0) return RL_OK;
+  const long long rows = (long long)num_runs * RL_PAGE;
+  CUtensorMap mq, mk, mv, ms;
+  int rc = fa_make_map(&mq, q, num_tokens, num_heads * 192, ldq, TQ);
+  if (rc != RL_OK) return rc;
+  rc = fa_make_map(&mk, keys, rows, num_heads * 128, num_heads * 128, RL_PAGE);
+  if (rc != RL_OK) return rc;
+  rc = fa_make_map(&mv, values, rows, num_heads * 128, num_heads * 128, RL_PAGE);
+  if (rc != RL_OK) return rc;
+  rc = fa_make_map(&ms, shared, rows, ld_shared, ld_shared, RL_PAGE);
+  if (rc != RL_OK) return rc;
+  return fa_launch<192, 128>(dim3(num_heads, num_tiles), stream, mq, mk, mv, run_table, max_runs, cu_seqlens, table_rows, kv_lens, num_seqs,
+                             (__nv_bfloat16*)out, ldo, num_heads, num_heads, scale * 1.4426950408889634f, window, err, tile_order, 0,
+                             (const __nv_bfloat16*)gate, ldg, 0.f, 0.f, 0, 0, gate_per_head, (const float*)nullptr, ms, shared_col);
 }
 
 extern "C" int rl_attention_prefill_tc_headgate(const void* q, int ldq, const void* k_pool, const void* v_pool, int num_pages,

@@ -448,6 +448,48 @@ extern "C" int rl_latent_query(const void* q, int ldq, int dtype, int num_heads,
   return RL_OK;
 }
 
+// ------------------------------------------------------------------ the cached rows that a step sees, out of their pages
+// A block a page: out [runs * RL_PAGE, width] takes the pages of sequence after sequence, from the pair of pages (the attention's tile)
+// that holds the first position any of the step's rows sees; table [num_seqs, max_pages] says which run of RL_PAGE rows a page became,
+// and table_rows = 0, 1, ...  Rows behind a sequence's end come as they are in its last page.  Bound by one read and one write of
+// the rows.
+__global__ void __launch_bounds__(HP_THREADS)
+latent_gather_kernel(const uint4* __restrict__ pool, int pieces, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slots,
+                     const int* __restrict__ kv_lens, int num_seqs, const int* __restrict__ page_table, int max_pages, int window,
+                     uint4* __restrict__ out, int* __restrict__ table, int* __restrict__ table_rows) {
+  rl_pdl_trigger();
+  rl_pdl_wait();
+  int run = blockIdx.x;
+  for (int b = 0; b < num_seqs; ++b) {
+    const int kv = kv_lens[b], start = kv - (cu_seqlens[b + 1] - cu_seqlens[b]);
+    const int first = window > 0 ? max(0, start + 1 - window) : 0;
+    const int p0 = first / (2 * RL_PAGE) * 2, n = (kv - 1) / RL_PAGE + 1 - p0;
+    if (run >= n) { run -= n; continue; }
+    const int page = page_table[(size_t)seq_slots[b] * max_pages + p0 + run];
+    if (threadIdx.x == 0) {
+      table[(size_t)b * max_pages + p0 + run] = blockIdx.x;
+      if (run == 0) table_rows[b] = b;
+    }
+    const uint4* src = rl_behind_wait(pool) + (size_t)page * RL_PAGE * pieces;
+    uint4* dst = out + (size_t)blockIdx.x * RL_PAGE * pieces;
+    for (int i = threadIdx.x; i < RL_PAGE * pieces; i += HP_THREADS) dst[i] = src[i];
+    return;
+  }
+}
+
+// pool [pages, 1, RL_PAGE, width] bf16, width a multiple of 8; num_runs: the pages of all sequences as said above (the caller counts them).
+extern "C" int rl_latent_gather(const void* pool, int width, const int* cu_seqlens, const int* seq_slots, const int* kv_lens, int num_seqs,
+                                const int* page_table, int max_pages, int window, int num_runs, void* out, int* table, int* table_rows,
+                                cudaStream_t stream) {
+  RL_REQUIRE(width > 0 && width % 8 == 0 && (((uintptr_t)pool | (uintptr_t)out) & 15) == 0 && num_seqs > 0 && num_runs >= 0 && window >= 0,
+             "rl_latent_gather: rows of %d are not whole 16-byte pieces, or bad sizes", width);
+  if (num_runs == 0) return RL_OK;
+  rl_launch_pdl(latent_gather_kernel, num_runs, HP_THREADS, 0, stream, (const uint4*)pool, width / 8, cu_seqlens, seq_slots, kv_lens, num_seqs,
+                page_table, max_pages, window, (uint4*)out, table, table_rows);
+  RL_LAUNCH_CHECK("rl_latent_gather");
+  return RL_OK;
+}
+
 // ------------------------------------------------------------------ a product a head, few tokens
 // out[m, a * out_head + n] = sum_k W[a][n][k] * x[m, a * x_head + k]: every head a has a matrix [N, K] of its own
 // and its own K columns of x (H small products as one launch; with few tokens they only stream the weights).

@@ -154,6 +154,11 @@ _SIGNATURES = {
     "rl_gemm_tc_grouped": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                            _c_void_p, _c_int, _c_int, _c_float, _c_float, _c_void_p],
     "rl_gemm_tc_heads": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "rl_latent_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p,
+                         _c_void_p, _c_void_p],
+    "rl_attention_prefill_tc_shared_part": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int,
+                                            _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
+                                            _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p],
     "rl_repeat_penalty": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p],
     "rl_argmax": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_sample_temperature": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -1943,6 +1948,58 @@ def attention_prefill_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Te
         _tc_error_word(q.device).data_ptr(), _ptr(tile_order), int(bool(sink)), gptr, ldg, float(softcap or 0.0),
         int(keep_first or 0), int(chunk or 0), int(bool(gate_per_head and gate is not None)), vd, _sinks(sinks, num_heads),
         _stream()), "rl_attention_prefill_tc")
+    _count()
+
+
+def latent_runs(q_lens, kv_lens, window: int) -> int:
+    """How many runs of PAGE_SIZE rows ``latent_gather`` fills for sequences of these lengths."""
+    runs = 0
+    for n, kv in zip(q_lens, kv_lens):
+        first = max(0, kv - n + 1 - window) if window else 0
+        runs += (kv - 1) // PAGE_SIZE + 1 - first // (2 * PAGE_SIZE) * 2
+    return runs
+
+
+def latent_gather(pool: torch.Tensor, page_table: torch.Tensor, step, window: int, num_runs: int):
+    """The cached rows that a step's tokens see, sequence after sequence: rows [num_runs * PAGE_SIZE, width], the runs that the
+    pages became [sequences, max pages] and the tables' row of every sequence.  pool: [pages, 1, PAGE_SIZE, width] bf16."""
+    _need(pool, "pool", torch.bfloat16); _need(page_table, "page_table", torch.int32)
+    B, width = len(step.q_lens), pool.shape[3]
+    rows = torch.empty((num_runs * PAGE_SIZE, width), dtype=pool.dtype, device=pool.device)
+    table = torch.empty((B, page_table.shape[1]), dtype=torch.int32, device=pool.device)
+    table_rows = torch.empty(B, dtype=torch.int32, device=pool.device)
+    _check(library().rl_latent_gather(pool.data_ptr(), width, step.cu_seqlens.data_ptr(), step.seq_slots.data_ptr(), step.kv_lens.data_ptr(), B,
+                                      page_table.data_ptr(), page_table.shape[1], int(window), num_runs, rows.data_ptr(), table.data_ptr(),
+                                      table_rows.data_ptr(), _stream()), "rl_latent_gather")
+    _count()
+    return rows, table, table_rows
+
+
+def attention_prefill_shared_part(q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, shared: torch.Tensor, shared_col: int,
+                                  table: torch.Tensor, table_rows: torch.Tensor, step, out: torch.Tensor, num_heads: int, scale: float,
+                                  window: int = 0, gate: Optional[torch.Tensor] = None, gate_per_head: bool = False) -> None:
+    """Attention of a prompt step's tokens over keys and values that lie beside the cache, bf16 on the tensor cores: q [M, H * 192]; a head's key
+    is its 128 columns of ``keys`` [rows, H * 128] and columns ``shared_col`` .. + 64 of ``shared`` [rows, .], its value 128 columns of
+    ``values``.  Positions lie in runs of PAGE_SIZE rows; ``table``, ``table_rows``: as from ``latent_gather``."""
+    for t, name in ((q, "q"), (shared, "shared")):
+        _need(t, name, torch.bfloat16, contiguous=False)
+    for t, name in ((keys, "keys"), (values, "values"), (out, "out")):
+        _need(t, name, torch.bfloat16)
+    M, B = q.shape[0], len(step.q_lens)
+    assert q.shape[1] == num_heads * 192 and q.stride(1) == 1 and keys.shape == values.shape == (shared.shape[0], num_heads * 128)
+    assert out.shape == (M, num_heads * 128) and shared.shape[0] % PAGE_SIZE == 0 and shared.stride(1) == 1 and M == sum(step.q_lens)
+    tiles = sum(-(-n // PREFILL_TC_QTILE) for n in step.q_lens)
+    order = None
+    if B > 1:
+        order = step.derived.get("prefill_tile_order")
+        if order is None:
+            order = step.derived["prefill_tile_order"] = prefill_tile_order(step.q_lens, step.kv_lens_host, q.device)
+    gptr, ldg = _gate_args(gate, M, num_heads, 2) if gate_per_head else _gate_args(gate, M, num_heads * 128, 16)
+    _check(library().rl_attention_prefill_tc_shared_part(
+        q.data_ptr(), q.stride(0), keys.data_ptr(), values.data_ptr(), shared.data_ptr(), shared.stride(0), int(shared_col),
+        shared.shape[0] // PAGE_SIZE, table.data_ptr(), table.shape[1], step.cu_seqlens.data_ptr(), table_rows.data_ptr(), step.kv_lens.data_ptr(),
+        B, tiles, M, out.data_ptr(), out.stride(0), num_heads, float(scale), int(window), _tc_error_word(q.device).data_ptr(), _ptr(order),
+        gptr, ldg, int(bool(gate_per_head and gate is not None)), _stream()), "rl_attention_prefill_tc_shared_part")
     _count()
 
 

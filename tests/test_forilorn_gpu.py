@@ -774,3 +774,96 @@ def test_heads_over_one_cached_row_with_unequal_sequences_in_one_step(H, r, rd, 
     for b in range(len(lens)):
         ref = plain_latent_scan(H, r, rd, window, scale, ql[b], rows[b], gate[b])
         torch.testing.assert_close(torch.cat(got[b]), ref, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("H,r,per_head", [(2, 64, True), (5, 128, False), (16, 512, True), (3, 24, None)])
+@pytest.mark.parametrize("window", [None, 130, 64])
+def test_keys_and_values_made_of_the_latents_a_step_sees(H, r, per_head, window):
+    """Five sequences of unequal lengths, then more of each behind what is cached: what a window leaves out is not gathered and may have
+    been given back, sequences end inside a page and inside a tile of two; scores over 128 dimensions of the head's own and 64 of all
+    heads.  Against float64 attention over the made keys and values rounded to bfloat16; a gate a head, an element, none."""
+    from rustyllm_b200 import kernels as K
+    from rustyllm_b200.cache.sequence_cache import KVNeed, SequenceCache
+    from rustyllm_b200.engine.step import StepState
+    from rustyllm_b200.parts.linear import OUT_SAME, linear
+    steps = [[200, 37, 1, 129, 64], [150, 70, 260, 1, 5]]
+    torch.manual_seed(H + r)
+    bf, scale, total = torch.bfloat16, 2.0 / math.sqrt(192), [a + b for a, b in zip(*steps)]
+    q = [rounded(torch.randn(n, H * 192, dtype=F64), "bfloat16") for n in total]
+    rows = [rounded(torch.randn(n, r + 64, dtype=F64), "bfloat16") for n in total]
+    width = H if per_head else H * 128
+    gate = [rounded(2.0 * torch.randn(n, width, dtype=F64), "bfloat16") for n in total] if per_head is not None else None
+    wk, wv = (rounded(torch.randn(H * 128, r, dtype=F64) / math.sqrt(r), "bfloat16") for _ in range(2))
+    cache = SequenceCache([KVNeed(1, r + 64, window, 0)], [None], 64 * 24, bf, DEV, max_slots=6)
+    cache.alloc_slot()
+    slots = [cache.alloc_slot() for _ in total]
+    group, layer = cache.kv_entry(0)
+    at, got = [0] * 5, [[] for _ in total]
+    for cnts in steps:
+        cache.prepare(slots, cnts)
+        pool = group.k_pool(layer)
+        for b, (sl, a, c) in enumerate(zip(slots, at, cnts)):
+            pages = group.page_table[sl].tolist()
+            for i in range(a, a + c):
+                pool[pages[i // 64], 0, i % 64] = rows[b][i].to(bf).to(DEV)
+        kv, cu = [a + c for a, c in zip(at, cnts)], [0]
+        for c in cnts:
+            cu.append(cu[-1] + c)
+        st = StepState(cu[-1], 5, i32([0] * cu[-1]), i32([i for a, c in zip(at, cnts) for i in range(a, a + c)]),
+                       i32([sl for sl, c in zip(slots, cnts) for _ in range(c)]), i32(cu), i32(slots), i32(kv), i32([]), list(cnts), kv,
+                       max(cnts), max(kv), False)
+        pick = lambda x: torch.cat([x[b][a:a + c] for b, (a, c) in enumerate(zip(at, cnts))]).to(bf).to(DEV).contiguous()
+        lat, table, table_rows = K.latent_gather(pool, group.page_table, st, window or 0, K.latent_runs(cnts, kv, window or 0))
+        keys, values = (torch.empty(lat.shape[0], H * 128, dtype=bf, device=DEV) for _ in range(2))
+        linear(lat[:, :r], wk.to(bf).to(DEV), keys, OUT_SAME)
+        linear(lat[:, :r], wv.to(bf).to(DEV), values, OUT_SAME)
+        out = torch.empty((cu[-1], H * 128), dtype=bf, device=DEV)
+        K.attention_prefill_shared_part(pick(q), keys, values, lat, r, table, table_rows, st, out, H, scale, window or 0,
+                                        gate=pick(gate) if gate else None, gate_per_head=bool(per_head))
+        for b, c in enumerate(cnts):
+            got[b].append(out[cu[b]:cu[b] + c].double().cpu())
+        cache.commit(slots, cnts)
+        at = kv
+    K.check_device_errors()
+    for b, n in enumerate(total):
+        kr = rounded(rows[b][:, :r] @ wk.T, "bfloat16").view(n, H, 128)
+        vr = rounded(rows[b][:, :r] @ wv.T, "bfloat16").view(n, H, 128)
+        kr = torch.cat([kr, rows[b][:, None, r:].expand(-1, H, -1)], dim=-1)
+        sc = torch.einsum("ihd,jhd->hij", q[b].view(n, H, 192), kr) * scale
+        i, j = torch.arange(n)[:, None], torch.arange(n)[None]
+        sc = sc.masked_fill(~((j <= i) & (i - j < (window or n))), -math.inf)
+        ref = torch.einsum("hij,jhd->ihd", torch.softmax(sc, -1), vr)
+        if gate:
+            ref = ref * torch.sigmoid(gate[b]).view(n, H, -1)
+        torch.testing.assert_close(torch.cat(got[b]).view(n, H, 128), ref, rtol=2e-2, atol=2e-2)
+
+
+def test_made_keys_and_widened_queries_agree():
+    """A model whose latent layers have the widths that keys and values are made for: a prompt whole, in portions (behind what is cached) and
+    beside another, against the route that widens the queries."""
+    from rustyllm_b200 import Runner
+    from rustyllm_b200.bench_designs import forilorn_config
+    from rustyllm_b200.parts.latent import LatentAttention
+    cfg = forilorn_config(dict(width=256, heads=2, kv_heads=1, dim=128, ff=512, layers=3, vocab=512), window=150)
+    r = Runner.from_config(cfg, seed=3, dtype="bfloat16", device=DEV, norm_noise=True, max_batch=4, max_cache_tokens=64 * 40)
+    a, b = random_tokens(512, 400, 5), random_tokens(512, 261, 6)
+
+    def run():
+        out = []
+        s, t = r.engine.alloc_slot(), r.engine.alloc_slot()
+        out.append(r.engine.step([s, t], [a, b], "all"))
+        r.engine.free_slot(s); r.engine.free_slot(t)
+        s = r.engine.alloc_slot()
+        out += [r.engine.step([s], [a[i:i + 200]], "all") for i in (0, 200)]
+        r.engine.free_slot(s)
+        return torch.cat(out).double().cpu()
+    layer = next(l.mixer for l in r.model.blocks if isinstance(l.mixer, LatentAttention))
+    assert layer.wuk_rows is not None
+    made, most = run(), LatentAttention.MADE_FROM
+    try:
+        LatentAttention.MADE_FROM = 1 << 30
+        widened = run()
+    finally:
+        LatentAttention.MADE_FROM = most
+    close(made, widened, "bfloat16", cfg, "keys made of the latents")
+    assert not torch.equal(made, widened)
