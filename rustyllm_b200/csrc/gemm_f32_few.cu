@@ -32,8 +32,10 @@ __device__ __forceinline__ void few_copy16(float* dst, const float* src, bool li
 // used, every step waited for them (2,048 rows of 8,192, four tokens: 30 us instead of 19).
 constexpr int FEW_STEPS = 4, FEW_STAGES = 3;
 
-// R rows of W a warp, MT >= M tokens, U steps of 128 values of k on their way
-template <int R, int MT, int U>
+// R rows of W a warp, MT >= M tokens, U steps of 128 values of k on their way.  GATED: W is N / 2 gate rows and N / 2 up rows behind them; a
+// warp takes R / 2 of each, and out [M, N / 2] is silu(gate) * up - the sums, and the activation on them, bit for bit those of the
+// product and the activation's own kernel.
+template <int R, int MT, int U, bool GATED>
 __global__ void __launch_bounds__(FEW_WARPS * 32)
 gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out_,
                     int add, int M, int N, int K, int lda, int ldo) {
@@ -43,8 +45,11 @@ gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, c
   const int n0 = ((int)blockIdx.x * FEW_WARPS + (int)(threadIdx.x >> 5)) * R;
   rl_pdl_trigger();
   const float* w[R];
+  const int half = N / 2;
+  // the weight row of this warp's row r (a row beyond the last reads the last: not stored)
+  auto row_of = [&](int r) { return GATED ? (r & 1) * half + min(n0 / 2 + r / 2, half - 1) : min(n0 + r, N - 1); };
 #pragma unroll
-  for (int r = 0; r < R; ++r) w[r] = W + (size_t)min(n0 + r, N - 1) * K + lane * 4;       // a row beyond the last reads the last: not stored
+  for (int r = 0; r < R; ++r) w[r] = W + (size_t)row_of(r) * K + lane * 4;
   const int steps = (K + 127) / 128, mine = (K - lane * 4 + 127) / 128;                    // K is a multiple of 4: a lane's piece is whole or beyond the end
   const int stages = (steps + FEW_STEPS - 1) / FEW_STEPS;
   float4 x[R][U];
@@ -124,6 +129,15 @@ gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, c
       acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
     }
   }
+  if constexpr (GATED) {
+    // the gate's sum and its up's lie in lanes that the row's lowest bit parts: the second of the distances above with four rows, the first with two
+    static_assert(COUNT <= 32, "a lane holds one sum");
+    const int r = first / MT, m = first % MT, i = n0 / 2 + r / 2;
+    const float v = acc[0] + (bias ? bias[row_of(r)] : 0.f);
+    const float up = __shfl_xor_sync(0xffffffffu, v, R == 4 ? 8 : 16);
+    if (lane % (32 / COUNT) == 0 && (r & 1) == 0 && i < half && m < M) out[(size_t)m * ldo + i] = v / (1.0f + expf(-v)) * up;
+    return;
+  }
   constexpr int HELD = COUNT > 32 ? COUNT / 32 : 1, COPIES = COUNT < 32 ? 32 / COUNT : 1;      // a sum's copies lie in neighbouring lanes
   if (lane % COPIES) return;
 #pragma unroll
@@ -136,16 +150,16 @@ gemm_f32_few_kernel(const float* __restrict__ A_, const float* __restrict__ W, c
   }
 }
 
-template <int R, int MT>
+template <int R, int MT, bool GATED>
 int few_launch(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo, int early,
                cudaStream_t stream) {
   const int rows = R * FEW_WARPS;
   const dim3 grid((N + rows - 1) / rows), block(FEW_WARPS * 32);
   cudaError_t e;
   if (early) {
-    e = rl_launch_pdl(gemm_f32_few_kernel<R, MT, 16 / R>, grid, block, 0, stream, A, W, bias, out, add, M, N, K, lda, ldo);
+    e = rl_launch_pdl(gemm_f32_few_kernel<R, MT, 16 / R, GATED>, grid, block, 0, stream, A, W, bias, out, add, M, N, K, lda, ldo);
   } else {           // launched the ordinary way the kernel begins when all in front of it have ended
-    gemm_f32_few_kernel<R, MT, 16 / R><<<grid, block, 0, stream>>>(A, W, bias, out, add, M, N, K, lda, ldo);
+    gemm_f32_few_kernel<R, MT, 16 / R, GATED><<<grid, block, 0, stream>>>(A, W, bias, out, add, M, N, K, lda, ldo);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
@@ -164,19 +178,35 @@ extern "C" int rl_gemm_f32_few_supported(const void* A, const void* W, int M, in
   return M > 0 && M <= 8 && N > 0 && K >= 256 && K % 4 == 0 && lda % 4 == 0 && lda >= K && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
 }
 
+template <bool GATED>
+static int few_run(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo, int early,
+                   cudaStream_t stream) {
+  // Four rows a warp halve the tokens' loads a weight row; two leave more warps to stream where rows are few.  Four tokens, two / four rows:
+  // 2,048 rows of 8,192 19.4 / 22.3 us, 3,072 of 2,048 7.2 / 8.3, 16,384 of 2,048 30.6 / 26.3, 128,256 of 2,048 189 / 162.
+  const bool four = N >= 32 * rl_num_sms();
+#define FEW_GO(MT)                                                                                                      \
+  (four ? few_launch<4, MT, GATED>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream)                              \
+        : few_launch<2, MT, GATED>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream))
+  if (M == 1) return FEW_GO(1);
+  if (M == 2) return FEW_GO(2);
+  if (M <= 4) return FEW_GO(4);
+  return FEW_GO(8);
+#undef FEW_GO
+}
+
 // A: float [M, K], row stride lda; W: float [N, K] contiguous; out: float [M, N], row stride ldo; add != 0: added into out.
 // early != 0: W is a weight, which no kernel that may still run writes, so it may be read before the kernels in front have ended.
 extern "C" int rl_gemm_f32_few(const float* A, const float* W, const float* bias, float* out, int add, int M, int N, int K, int lda, int ldo,
                                int early, cudaStream_t stream) {
   RL_REQUIRE(rl_gemm_f32_few_supported(A, W, M, N, K, lda) && ldo >= N, "rl_gemm_f32_few: operands not supported (M=%d N=%d K=%d lda=%d ldo=%d)", M, N,
              K, lda, ldo);
-  // Four rows a warp halve the tokens' loads a weight row; two leave more warps to stream where rows are few.  Four tokens, two / four rows:
-  // 2,048 rows of 8,192 19.4 / 22.3 us, 3,072 of 2,048 7.2 / 8.3, 16,384 of 2,048 30.6 / 26.3, 128,256 of 2,048 189 / 162.
-  const bool four = N >= 32 * rl_num_sms();
-#define FEW_GO(MT) (four ? few_launch<4, MT>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream) : few_launch<2, MT>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream))
-  if (M == 1) return FEW_GO(1);
-  if (M == 2) return FEW_GO(2);
-  if (M <= 4) return FEW_GO(4);
-  return FEW_GO(8);
-#undef FEW_GO
+  return few_run<false>(A, W, bias, out, add, M, N, K, lda, ldo, early, stream);
+}
+
+// W: float [2 I, K], gate rows first (as its bias [2 I], may be null), a weight; out: float [M, I] = silu(gate) * up.
+extern "C" int rl_gemm_f32_few_swiglu(const float* A, const float* W, const float* bias, float* out, int M, int I, int K, int lda, int ldo,
+                                      cudaStream_t stream) {
+  RL_REQUIRE(I > 0 && I <= 1073741823 && rl_gemm_f32_few_supported(A, W, M, 2 * I, K, lda) && ldo >= I,
+             "rl_gemm_f32_few_swiglu: operands not supported (M=%d I=%d K=%d lda=%d ldo=%d)", M, I, K, lda, ldo);
+  return few_run<true>(A, W, bias, out, 0, M, 2 * I, K, lda, ldo, 1, stream);
 }

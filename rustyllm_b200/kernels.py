@@ -159,6 +159,7 @@ _SIGNATURES = {
     "rl_attention_prefill_tc_shared_part": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int,
                                             _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
                                             _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p],
+    "rl_gemm_f32_few_swiglu": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "rl_repeat_penalty": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p],
     "rl_argmax": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p],
     "rl_sample_temperature": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -616,6 +617,32 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int
         return
     _check(library().rl_gemm_simt(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), _dt(a), out_mode,
                                   M, N, K, lda, ldo, _stream()), "rl_gemm_simt")
+    _count()
+
+
+def gemm_f32_few_swiglu_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether ``gemm_f32_few_swiglu`` takes these operands: the products of up to 8 float tokens that the kernel for few takes."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or not w.is_contiguous() or a.stride(1) != 1:
+        return False
+    M, K = a.shape
+    lda = a.stride(0) if M > 1 else K
+    lib = library()
+    return bool(lib.rl_gemm_f32_few_supported(a.data_ptr(), w.data_ptr(), M, w.shape[0], K, lda)
+                and not lib.rl_gemm_f32_split_supported(a.data_ptr(), w.data_ptr(), M, w.shape[0], K, lda))
+
+
+def gemm_f32_few_swiglu(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None) -> None:
+    """out [M, I] = silu(gate) * up of the product of ``a`` [M, K] with a weight ``w`` [2 I, K] whose gate rows come first; float32, the bits
+    of the product followed by ``swiglu``."""
+    _need(a, "a", torch.float32, contiguous=False); _need(w, "w", torch.float32); _need(out, "out", torch.float32, contiguous=False)
+    M, K = a.shape
+    I = w.shape[0] // 2
+    assert w.shape == (2 * I, K) and out.shape == (M, I) and a.stride(1) == 1 and out.stride(1) == 1
+    if bias is not None:
+        _need(bias, "bias", torch.float32)
+        assert bias.numel() == 2 * I
+    _check(library().rl_gemm_f32_few_swiglu(a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, I, K, a.stride(0) if M > 1 else K,
+                                            out.stride(0) if M > 1 else I, _stream()), "rl_gemm_f32_few_swiglu")
     _count()
 
 

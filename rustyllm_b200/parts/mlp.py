@@ -72,6 +72,8 @@ class GatedMLP(FeedForward):
         if self.interleaved and self.wgu.dtype == torch.bfloat16 and K.gemm_tc_supported(x, self.wgu, None):
             kw = dict(row_sumsq=xn.sumsq, row_eps=xn.eps) if isinstance(xn, NormedInput) else {}
             K.gemm_tc(x, self.wgu, h, K.OUT_GEGLU if gelu else K.OUT_SWIGLU, self.bgu, **kw)
+        elif not gelu and not self.interleaved and K.gemm_f32_few_swiglu_supported(xn, self.wgu):
+            K.gemm_f32_few_swiglu(xn, self.wgu, h, self.bgu)       # few tokens in 32-bit: the activation rides along there too
         else:
             gu = torch.empty((M, 2 * self.I), dtype=xn.dtype, device=xn.device)
             linear(xn, self.wgu, gu, OUT_SAME, self.bgu)

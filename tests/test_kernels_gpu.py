@@ -1468,6 +1468,24 @@ def test_gemm_f32_split_keeps_what_is_no_finite_number_and_the_largest_floats():
     torch.testing.assert_close(out[fine], plain[fine], rtol=1e-5, atol=1e-4)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 7, 8])
+@pytest.mark.parametrize("I,K_", [(1, 256), (131, 260), (2048, 512), (2401, 1028)])
+def test_gemm_f32_few_with_swiglu_has_the_bits_of_product_and_activation(M, I, K_):
+    """Two and four weight rows a warp (half of them gates), ends of both, rows of a wider output."""
+    k = K()
+    a, w, bias = _rand(M, K_, seed=1), _rand(2 * I, K_, seed=2), _rand(2 * I, seed=3)
+    for b in (None, bias):
+        gu, ref = torch.empty(M, 2 * I, device=DEV), torch.empty(M, I, device=DEV)
+        k.gemm_simt(a, w, gu, k.OUT_SAME, b, is_weight=True)
+        k.swiglu(gu, ref, interleaved=False)
+        wide = _rand(M, I + 3, seed=4)
+        out = wide.clone()
+        assert k.gemm_f32_few_swiglu_supported(a, w)
+        k.gemm_f32_few_swiglu(a, w, out[:, :I], b)
+        assert torch.equal(out[:, :I], ref) and torch.equal(out[:, I:], wide[:, I:])
+    assert not k.gemm_f32_few_swiglu_supported(_rand(9, K_, seed=5), w)
+
+
 def test_products_of_many_float_rows_take_the_split_kernel():
     k = K()
     lib = k.library()
