@@ -27,11 +27,12 @@
 //   O += P V    tcgen05.mma with P in tensor memory as A and the value tile as an
 //               MN-major B operand (values are stored [position][head_dim]); O stays in
 //               tensor memory over all key tiles
-// Heads of 64 (keys and values): one buffer of S and of P, 256 columns of tensor memory, 96 KB of shared memory and 80 registers a
+// Heads of 64 (keys and values) in steps of many CTAs: one buffer of S and of P, 256 columns of tensor memory, 96 KB of shared memory and 80 registers a
 // thread, so that two CTAs share an SM, and two threads a row, one for each half of a tile's keys, who exchange the halves'
 // maxima through shared memory; the running maximum stays in their registers.  With one CTA an SM its eight warps issued in 35 % of the
 // slots and the special-function unit ran 45 % of the time: two warps a scheduler do not cover one another's waits, and nothing
-// ran under a CTA's start and end.  Sixteen warps do better: 32 heads over 8, 8,192 tokens 504 -> 442 us, 4,096 141 -> 130.
+// ran under a CTA's start and end.  Sixteen warps do better: 32 heads over 8, 8,192 tokens 504 -> 442 us, 4,096 141 -> 130
+// (each form with the code for masks in its loop, see PLAIN).
 // Tensor memory: the S buffers, O behind them, P behind O (512 columns at head size 128).
 // A key tile is two cache pages (128 positions).  Warp 0 feeds TMA, warps 1 and 2 issue the two
 // products (a thread each: issuing blocks while the tensor pipe is full, and one thread's waits
@@ -58,14 +59,15 @@ constexpr int FA_PV_WARP = 2;
 constexpr uint32_t FA_WAIT_LIMIT = 1u << 22;
 constexpr int HALF_BYTES = 128 * 64 * 2;               // [128 rows x 64 bf16], 16 KB
 // sizes that depend on the widths of a key head HD (64, 128 or 192) and of a value head VD (64 or 128): halves of 64 dimensions
-template <int HD, int VD> struct FaSizes {
+template <int HD, int VD, bool PAIRED = false> struct FaSizes {
   static constexpr int HALVES = HD / 64, V_HALVES = VD / 64;
   static constexpr int Q_BYTES = HALVES * HALF_BYTES;          // 16 or 32 KB
   static constexpr int TILE_BYTES = HALVES * HALF_BYTES;       // a key tile: 16 or 32 KB
   static constexpr int V_TILE_BYTES = V_HALVES * HALF_BYTES;   // a value tile
   // keys are asked for a tile further ahead than values: the scores of a tile are computed as soon as the
   // buffer is free, a whole tile before its P V
-  static constexpr bool TWO = HD == 64 && VD == 64;            // two CTAs an SM: what they hold fits twice (see above)
+  static constexpr bool TWO = PAIRED;                          // two CTAs an SM: what they hold fits twice (see above)
+  static_assert(!PAIRED || (HD == 64 && VD == 64), "two CTAs fit an SM with heads of 64");
   // heads of 192: 128 key dimensions of their own and 64 that all heads share (see rl_attention_prefill_tc_shared_part)
   static constexpr bool SHARED_PART = HD == 192;
   static constexpr int K_STAGES = SHARED_PART ? 2 : TWO ? 3 : HD == 64 ? 4 : 3;
@@ -203,8 +205,10 @@ __host__ __device__ constexpr uint32_t fa_idesc(int m, int n, int b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-template <int HD, int VD>
-__global__ void __launch_bounds__(FA_THREADS, FaSizes<HD, VD>::CTAS)
+// PLAIN: every position up to the query's own is visible and scores are not capped; the code for windows, blocks, kept first tokens and soft caps is then
+// left out of the loop, which is bound by what its warps issue (heads of 64, 8,192 tokens 439 -> 429 us; heads of 128, 4,096 tokens 155 -> 145, 1,000 21.6 -> 20.6).
+template <int HD, int VD, bool PLAIN, bool PAIRED>
+__global__ void __launch_bounds__(FA_THREADS, FaSizes<HD, VD, PAIRED>::CTAS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ page_table, int max_pages,
                             const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slots,
@@ -213,10 +217,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int* __restrict__ tile_order, int sink, const __nv_bfloat16* __restrict__ gate, int ldg,
                             float cap_in, float cap_out, int keep_first, int chunk, int gate_per_head, const float* __restrict__ sinks,
                             const __grid_constant__ CUtensorMap map_shared, int shared_col) {
+  if constexpr (PLAIN) { window = 0; chunk = 0; keep_first = 0; cap_in = 0.f; }
   extern __shared__ uint8_t fa_smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)fa_smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* q_tile = smem;                                   // [2 halves][128 x 64]
-  using SZ = FaSizes<HD, VD>;
+  using SZ = FaSizes<HD, VD, PAIRED>;
   constexpr int HALVES = SZ::HALVES, V_HALVES = SZ::V_HALVES, Q_BYTES = SZ::Q_BYTES, TILE_BYTES = SZ::TILE_BYTES, V_TILE_BYTES = SZ::V_TILE_BYTES;
   constexpr int K_STAGES = SZ::K_STAGES, V_STAGES = SZ::V_STAGES, BUFS = SZ::BUFS, SPLIT = SZ::SPLIT, GROUPS = SZ::GROUPS;
   uint8_t* k_ring = smem + Q_BYTES;                         // [stage][halves]
@@ -651,7 +656,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   }
   fa_fence_before();
   __syncthreads();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FaSizes<HD, VD>::TMEM_COLS) : "memory");
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)FaSizes<HD, VD, PAIRED>::TMEM_COLS) : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -686,20 +691,31 @@ int fa_make_map(CUtensorMap* map, const void* base, long long rows, int cols, lo
   return RL_OK;
 }
 
-template <int HD, int VD, typename... Args>
-int fa_launch(dim3 grid, cudaStream_t stream, Args... args) {
+template <int HD, int VD, bool PLAIN, bool PAIRED, typename... Args>
+int fa_launch_as(dim3 grid, cudaStream_t stream, Args... args) {
+  constexpr int SMEM = FaSizes<HD, VD, PAIRED>::SMEM;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, VD>, cudaFuncAttributeMaxDynamicSharedMemorySize, FaSizes<HD, VD>::SMEM);
-    RL_REQUIRE(e == cudaSuccess, "rl_attention_prefill_tc: cannot reserve %d bytes of shared memory: %s", FaSizes<HD, VD>::SMEM, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, VD, PLAIN, PAIRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    RL_REQUIRE(e == cudaSuccess, "rl_attention_prefill_tc: cannot reserve %d bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
     configured = true;
   }
-  cudaError_t e = rl_launch_pdl(attention_prefill_tc_kernel<HD, VD>, grid, dim3(FA_THREADS), (size_t)FaSizes<HD, VD>::SMEM, stream, args...);
+  cudaError_t e = rl_launch_pdl(attention_prefill_tc_kernel<HD, VD, PLAIN, PAIRED>, grid, dim3(FA_THREADS), (size_t)SMEM, stream, args...);
   if (e != cudaSuccess) {
     rl_set_error("rl_attention_prefill_tc: launch failed: %s", cudaGetErrorString(e));
     return RL_ERR_CUDA;
   }
   return RL_OK;
+}
+template <int HD, int VD, typename... Args>
+int fa_launch(bool plain, dim3 grid, cudaStream_t stream, Args... args) {
+  if constexpr (HD == 64 && VD == 64) {
+    // Two CTAs an SM from where they are more than fit the GPU so at once.  Up to there a CTA with an SM of its own is done sooner: 32 heads,
+    // 1,000 tokens (256 CTAs) 17.6 us alone, 20.4 two an SM; 1,300 (352) 28.7 and 25.2, 2,000 47.1 and 38.9
+    if ((long long)grid.x * grid.y > 2LL * rl_num_sms())
+      return plain ? fa_launch_as<HD, VD, true, true>(grid, stream, args...) : fa_launch_as<HD, VD, false, true>(grid, stream, args...);
+  }
+  return plain ? fa_launch_as<HD, VD, true, false>(grid, stream, args...) : fa_launch_as<HD, VD, false, false>(grid, stream, args...);
 }
 
 }  // namespace
@@ -760,8 +776,9 @@ extern "C" int rl_attention_prefill_tc_wide(const void* q, int ldq, const void* 
   if (rc != RL_OK) return rc;
   rc = fa_make_map(&mv, v_pool, pool_rows, value_dim, value_dim, RL_PAGE);
   if (rc != RL_OK) return rc;
+  const bool plain = window == 0 && chunk == 0 && softcap == 0.f;
 #define FA_GO(HD, VD)                                                                                                          \
-  fa_launch<HD, VD>(dim3(num_heads, num_tiles), stream, mq, mk, mv, page_table, max_pages, cu_seqlens, seq_slots, kv_lens,     \
+  fa_launch<HD, VD>(plain, dim3(num_heads, num_tiles), stream, mq, mk, mv, page_table, max_pages, cu_seqlens, seq_slots, kv_lens,     \
                     num_seqs, (__nv_bfloat16*)out, ldo, num_heads, num_kv_heads, scale * 1.4426950408889634f, window, err,      \
                     tile_order, sink, (const __nv_bfloat16*)gate, ldg, cap_in, cap_out, keep_first, chunk, gate_per_head, sinks, mk, 0)
   if (head_dim == 64) return value_dim == 64 ? FA_GO(64, 64) : FA_GO(64, 128);
@@ -801,7 +818,7 @@ extern "C" int rl_attention_prefill_tc_shared_part(const void* q, int ldq, const
   if (rc != RL_OK) return rc;
   rc = fa_make_map(&ms, shared, rows, ld_shared, ld_shared, RL_PAGE);
   if (rc != RL_OK) return rc;
-  return fa_launch<192, 128>(dim3(num_heads, num_tiles), stream, mq, mk, mv, run_table, max_runs, cu_seqlens, table_rows, kv_lens, num_seqs,
+  return fa_launch<192, 128>(window == 0, dim3(num_heads, num_tiles), stream, mq, mk, mv, run_table, max_runs, cu_seqlens, table_rows, kv_lens, num_seqs,
                              (__nv_bfloat16*)out, ldo, num_heads, num_heads, scale * 1.4426950408889634f, window, err, tile_order, 0,
                              (const __nv_bfloat16*)gate, ldg, 0.f, 0.f, 0, 0, gate_per_head, (const float*)nullptr, ms, shared_col);
 }
