@@ -1208,13 +1208,19 @@ extern "C" int rl_gemm_tc_heads(const void* A, const void* W, void* out, int M, 
 
 // 1 if rl_gemm_tc_qkv_rope takes the shape: head size 128 or 64, the whole head rotated, a step
 // of up to 64 tokens whose product is split over K (a function of the shapes only).
-extern "C" int rl_gemm_tc_qkv_rope_supported(int M, int num_heads, int num_kv_heads, int head_dim, int rotary_dim, int K) {
-  if ((head_dim != 128 && head_dim != 64) || rotary_dim != head_dim || M <= 0 || M > 64 || K % 8 != 0) return 0;
-  const int N = (num_heads + 2 * num_kv_heads) * head_dim;
+// rl_gemm_tc_qkv_beside_supported: `beside` more output columns (a multiple of 4) behind the heads, and heads that are not rotated
+// at all (rotary_dim 0) too.
+extern "C" int rl_gemm_tc_qkv_beside_supported(int M, int num_heads, int num_kv_heads, int head_dim, int rotary_dim, int beside, int K) {
+  if ((head_dim != 128 && head_dim != 64) || (rotary_dim != head_dim && rotary_dim != 0) || beside < 0 || beside % 4 != 0 || M <= 0 || M > 64 || K % 8 != 0)
+    return 0;
+  const int N = (num_heads + 2 * num_kv_heads) * head_dim + beside;
   const int total_kb = (K + BLOCK_K - 1) / BLOCK_K;
   int splits = rl_gemm_tc_splits(M, N, K);
   while (splits > 1 && (splits - 1) * ((total_kb + splits - 1) / splits) >= total_kb) splits /= 2;
   return splits > 1;
+}
+extern "C" int rl_gemm_tc_qkv_rope_supported(int M, int num_heads, int num_kv_heads, int head_dim, int rotary_dim, int K) {
+  return rotary_dim == head_dim && rl_gemm_tc_qkv_beside_supported(M, num_heads, num_kv_heads, head_dim, rotary_dim, 0, K);
 }
 
 // The QKV product of an attention layer with rotary encoding and cache write in its
@@ -1223,20 +1229,22 @@ extern "C" int rl_gemm_tc_qkv_rope_supported(int M, int num_heads, int num_kv_he
 // values go to k_pool / v_pool [pages, G, RL_PAGE, head_dim] at each token's position (null
 // pools: they are not stored at all).  positions, slot_of_token: [M]; inv_freq: [head_dim / 2]
 // float.  scale_*: as in rl_gemm_tc.  Refused unless rl_gemm_tc_qkv_rope_supported(...).
-extern "C" int rl_gemm_tc_qkv_rope(const void* A, const void* W, const float* bias, void* out, int M, int K, int lda, int ldo,
-                                   int* err, const float* scale_partials, int scale_count, float scale_eps,
-                                   const int* positions, const int* slot_of_token, const int* page_table, int max_pages,
-                                   const float* inv_freq, int interleaved, int num_heads, int num_kv_heads, int head_dim,
-                                   void* k_pool, void* v_pool, cudaStream_t stream) {
-  RL_REQUIRE(num_heads > 0 && num_kv_heads > 0 && positions != nullptr && inv_freq != nullptr,
-             "rl_gemm_tc_qkv_rope: bad head counts or null positions / frequencies");
+// rl_gemm_tc_qkv_beside: W has `beside` more rows (say, an output gate's), whose products lie behind the heads in `out` as they are; a null
+// inv_freq rotates nothing (the keys' and values' copy into the cache is then no kernel of its own).
+extern "C" int rl_gemm_tc_qkv_beside(const void* A, const void* W, const float* bias, void* out, int M, int K, int lda, int ldo,
+                                     int* err, const float* scale_partials, int scale_count, float scale_eps,
+                                     const int* positions, const int* slot_of_token, const int* page_table, int max_pages,
+                                     const float* inv_freq, int interleaved, int num_heads, int num_kv_heads, int head_dim,
+                                     void* k_pool, void* v_pool, int beside, cudaStream_t stream) {
+  RL_REQUIRE(num_heads > 0 && num_kv_heads > 0 && positions != nullptr && beside >= 0 && beside % 4 == 0,
+             "rl_gemm_tc_qkv_rope: bad head counts, null positions or columns beside the heads that are no multiple of 4");
   RL_REQUIRE(head_dim == 128 || head_dim == 64, "rl_gemm_tc_qkv_rope: head size %d; 128 and 64 are taken", head_dim);
   RL_REQUIRE((k_pool == nullptr) == (v_pool == nullptr), "rl_gemm_tc_qkv_rope: give both pools or neither");
   RL_REQUIRE(k_pool == nullptr || (slot_of_token != nullptr && page_table != nullptr && max_pages > 0),
              "rl_gemm_tc_qkv_rope: the cache write needs slots and the page table");
   RL_REQUIRE(((uintptr_t)out & 7) == 0 && ldo % 4 == 0 && ((uintptr_t)k_pool & 7) == 0 && ((uintptr_t)v_pool & 7) == 0,
              "rl_gemm_tc_qkv_rope: output and pools must be 8-byte aligned, ldo a multiple of 4");
-  const int N = (num_heads + 2 * num_kv_heads) * head_dim;
+  const int N = (num_heads + 2 * num_kv_heads) * head_dim + beside;
   TcFuse fuse = {};
   fuse.head_dim = head_dim;
   fuse.scale_partials = scale_partials; fuse.scale_count = scale_count; fuse.scale_eps = scale_eps;
@@ -1244,4 +1252,14 @@ extern "C" int rl_gemm_tc_qkv_rope(const void* A, const void* W, const float* bi
   fuse.inv_freq = inv_freq; fuse.interleaved = interleaved; fuse.num_heads = num_heads; fuse.num_kv_heads = num_kv_heads;
   fuse.k_pool = (__nv_bfloat16*)k_pool; fuse.v_pool = (__nv_bfloat16*)v_pool;
   return gemm_tc_run(A, W, bias, out, TC_OUT_ROPE_KV, M, N, K, lda, ldo, err, 0, fuse, stream);
+}
+
+extern "C" int rl_gemm_tc_qkv_rope(const void* A, const void* W, const float* bias, void* out, int M, int K, int lda, int ldo,
+                                   int* err, const float* scale_partials, int scale_count, float scale_eps,
+                                   const int* positions, const int* slot_of_token, const int* page_table, int max_pages,
+                                   const float* inv_freq, int interleaved, int num_heads, int num_kv_heads, int head_dim,
+                                   void* k_pool, void* v_pool, cudaStream_t stream) {
+  RL_REQUIRE(inv_freq != nullptr, "rl_gemm_tc_qkv_rope: null frequencies");
+  return rl_gemm_tc_qkv_beside(A, W, bias, out, M, K, lda, ldo, err, scale_partials, scale_count, scale_eps, positions, slot_of_token, page_table,
+                               max_pages, inv_freq, interleaved, num_heads, num_kv_heads, head_dim, k_pool, v_pool, 0, stream);
 }

@@ -52,7 +52,7 @@ struct TcFuse {
   const int* slot_of_token;     // [M]
   const int* page_table;        // [slots, max_pages]
   int max_pages;
-  const float* inv_freq;        // [head_dim / 2]
+  const float* inv_freq;        // [head_dim / 2]; null: nothing is rotated
   int interleaved;              // pairs (2i, 2i+1) instead of (i, i + head_dim / 2)
   int num_heads, num_kv_heads;
   int head_dim;                 // 128 (a tile of 128 output columns is one head) or 64 (two heads)
@@ -256,7 +256,7 @@ __device__ __forceinline__ void tc_finish_column(float4 v, int j, int r4, int la
           float e[4] = {v.x, v.y, v.z, v.w};
           // (all lanes take part in the exchange below, also those of a head beyond the last)
           if (head < H + G || hd < BLOCK_N_OUT) {
-            const bool rotate = head < H + G;
+            const bool rotate = head < H + G && fuse.inv_freq != nullptr;
             const float pos = (float)tok_pos[j];
             if (fuse.interleaved) {             // pairs (d, d + 1) and (d + 2, d + 3), frequencies d / 2 and d / 2 + 1
               if (rotate) {
@@ -285,9 +285,9 @@ __device__ __forceinline__ void tc_finish_column(float4 v, int j, int r4, int la
           }
           __nv_bfloat162 lo = __floats2bfloat162_rn(e[0], e[1]), hi = __floats2bfloat162_rn(e[2], e[3]);
           const uint2 pk = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-          if (head < H) {
-            *reinterpret_cast<uint2*>((__nv_bfloat16*)out + (size_t)(m0 + j) * ldo + nn) = pk;
-          } else if (fuse.k_pool != nullptr && head < H + 2 * G) {
+          if (head < H || head >= H + 2 * G) {        // queries, and what lies beside the heads (a gate) as it is
+            if (nn < N) *reinterpret_cast<uint2*>((__nv_bfloat16*)out + (size_t)(m0 + j) * ldo + nn) = pk;
+          } else if (fuse.k_pool != nullptr) {
             const bool is_v = head >= H + G;
             const int g = head - (is_v ? H + G : H);
             __nv_bfloat16* pool = is_v ? fuse.v_pool : fuse.k_pool;

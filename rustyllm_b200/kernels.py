@@ -225,6 +225,10 @@ _SIGNATURES = {
     "rl_gemm_tc_qkv_rope": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                             _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
                             _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
+    "rl_gemm_tc_qkv_beside": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
+                            _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
+                            _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p],
+    "rl_gemm_tc_qkv_beside_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int],
 }
 
 
@@ -1623,33 +1627,37 @@ def gemm_tc(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, out_mode: int,
 
 
 def gemm_tc_qkv_rope_supported(a: torch.Tensor, w: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int,
-                               rotary_dim: int) -> bool:
+                               rotary_dim: int, beside: int = 0) -> bool:
     """Whether the QKV product of these operands can carry the rotary encoding and the cache
-    write in its epilogue (head size 128 or 64 rotated whole, up to 64 tokens, a product that
-    is split over K)."""
-    if not gemm_tc_supported(a, w, None) or w.shape[0] != (num_heads + 2 * num_kv_heads) * head_dim:
+    write in its epilogue (head size 128 or 64 rotated whole or not at all, up to 64 tokens, a product that
+    is split over K).  ``beside``: output columns behind the heads, stored as they are."""
+    if not gemm_tc_supported(a, w, None) or w.shape[0] != (num_heads + 2 * num_kv_heads) * head_dim + beside:
         return False
-    return bool(library().rl_gemm_tc_qkv_rope_supported(a.shape[0], num_heads, num_kv_heads, head_dim, rotary_dim, a.shape[1]))
+    return bool(library().rl_gemm_tc_qkv_beside_supported(a.shape[0], num_heads, num_kv_heads, head_dim, rotary_dim, beside, a.shape[1]))
 
 
 def gemm_tc_qkv_rope(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor],
                      positions: torch.Tensor, slot_of_token: torch.Tensor, page_table: torch.Tensor,
-                     inv_freq: torch.Tensor, interleaved: bool, num_heads: int, num_kv_heads: int,
+                     inv_freq: Optional[torch.Tensor], interleaved: bool, num_heads: int, num_kv_heads: int,
                      k_pool: Optional[torch.Tensor], v_pool: Optional[torch.Tensor],
-                     row_sumsq: Optional[torch.Tensor] = None, row_eps: float = 0.0) -> None:
+                     row_sumsq: Optional[torch.Tensor] = None, row_eps: float = 0.0, beside: int = 0) -> None:
     """qkv = a @ w.T (+ bias) with rotary encoding of the query and key heads and the write of
     keys and values into the paged cache, all in the product's epilogue.  Of ``out``
     [M, (H + 2G) * head_dim] bf16 only the query heads are written; keys and values go to the
-    pools (``None``: nowhere).  The head size (128 or 64) follows from ``w``'s rows.
+    pools (``None``: nowhere).  The head size (128 or 64) follows from ``w``'s rows.  ``inv_freq`` ``None``: nothing is rotated.
+    ``beside`` rows of ``w`` behind the heads' (an output gate): their columns of ``out`` are written as they are.
     ``row_sumsq`` / ``row_eps``: as in ``gemm_tc``."""
     _need(a, "a", torch.bfloat16, contiguous=False); _need(w, "w", torch.bfloat16); _need(out, "out", torch.bfloat16, contiguous=False)
     _need(positions, "positions", torch.int32); _need(slot_of_token, "slot_of_token", torch.int32)
-    _need(page_table, "page_table", torch.int32); _need(inv_freq, "inv_freq", torch.float32)
+    _need(page_table, "page_table", torch.int32)
     M, K = a.shape
-    hd = w.shape[0] // (num_heads + 2 * num_kv_heads)
-    assert hd in (64, 128) and w.shape == ((num_heads + 2 * num_kv_heads) * hd, K)
+    hd = (w.shape[0] - beside) // (num_heads + 2 * num_kv_heads)
+    assert hd in (64, 128) and w.shape == ((num_heads + 2 * num_kv_heads) * hd + beside, K)
     assert out.shape == (M, w.shape[0]) and out.stride(1) == 1
-    assert positions.numel() == M and slot_of_token.numel() == M and inv_freq.numel() == hd // 2
+    assert positions.numel() == M and slot_of_token.numel() == M
+    if inv_freq is not None:
+        _need(inv_freq, "inv_freq", torch.float32)
+        assert inv_freq.numel() == hd // 2
     if bias is not None:
         _need(bias, "bias", torch.float32)
         assert bias.numel() == w.shape[0]
@@ -1663,11 +1671,11 @@ def gemm_tc_qkv_rope(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: 
         pieces = row_sumsq.shape[1]
     lda = a.stride(0) if M > 1 else K
     ldo = out.stride(0) if M > 1 else out.shape[1]
-    _check(library().rl_gemm_tc_qkv_rope(
+    _check(library().rl_gemm_tc_qkv_beside(
         a.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), M, K, lda, ldo, _tc_error_word(a.device).data_ptr(),
         _ptr(row_sumsq), pieces, float(row_eps), positions.data_ptr(), slot_of_token.data_ptr(), page_table.data_ptr(),
-        page_table.shape[1], inv_freq.data_ptr(), 1 if interleaved else 0, num_heads, num_kv_heads, hd,
-        _ptr(k_pool), _ptr(v_pool), _stream()), "rl_gemm_tc_qkv_rope")
+        page_table.shape[1], _ptr(inv_freq), 1 if interleaved else 0, num_heads, num_kv_heads, hd,
+        _ptr(k_pool), _ptr(v_pool), int(beside), _stream()), "rl_gemm_tc_qkv_rope")
     _count()
 
 

@@ -229,13 +229,14 @@ class GQAttention(Mixer):
                           k_pool if cache.writes else None, v_pool if cache.writes else None)
             if self.conv_taps > 1 and cache.writes:
                 K.short_conv_state(qkv, self.conv_taps, step.cu_seqlens, step.seq_slots, cache.state)
-        elif (v_other is None and dt == torch.bfloat16 and vd == hd and not self.gated and self.wqkv.dtype == torch.bfloat16 and k_pool.dtype == torch.bfloat16
-                and K.gemm_tc_qkv_rope_supported(x, self.wqkv, H, G, hd, pos.rotary_dim)):
-            # few tokens: rotation and cache write ride in the product's epilogue
+        elif (v_other is None and dt == torch.bfloat16 and vd == hd and self.wqkv.dtype == torch.bfloat16 and k_pool.dtype == torch.bfloat16
+                and self.value_mix is None        # (the epilogue leaves no values in the row)
+                and K.gemm_tc_qkv_rope_supported(x, self.wqkv, H, G, hd, pos.rotary_dim, self.gate_rows)):
+            # few tokens: rotation and cache write ride in the product's epilogue, the gate's columns beside them
             kw = dict(row_sumsq=xn.sumsq, row_eps=xn.eps) if isinstance(xn, NormedInput) else {}
             K.gemm_tc_qkv_rope(x, self.wqkv, qkv, self.bqkv, step.positions, step.slot_of_token, group.page_table,
-                               pos.inv_freq, pos.interleaved, H, G,
-                               k_pool if cache.writes else None, v_pool if cache.writes else None, **kw)
+                               pos.inv_freq if pos.rotary_dim else None, pos.interleaved, H, G,
+                               k_pool if cache.writes else None, v_pool if cache.writes else None, beside=self.gate_rows, **kw)
         else:
             linear(xn, self.wqkv, qkv, OUT_SAME, self.bqkv)
             K.rope_kv_write(qkv, step.positions, step.slot_of_token, group.page_table, pos.inv_freq, H, G, hd,

@@ -450,6 +450,39 @@ def test_rope_kv_write_at_positions_in_the_thousands(dtype, H, G, hd, factor, in
         assert torch.equal(v_pool[page, :, off].double().cpu(), v[m])
 
 
+@pytest.mark.parametrize("hd,rot", [(128, 0), (64, 0), (128, 128), (64, 64)])
+@pytest.mark.parametrize("M,H,G,K_,beside,store", [(1, 3, 1, 1024, 4, True), (17, 5, 1, 512, 60, True), (48, 16, 4, 2048, 2048, True), (64, 4, 2, 1024, 132, False),
+                                                  (5, 2, 2, 1024, 0, True)])
+def test_gemm_tc_qkv_with_columns_beside_the_heads_and_without_rotation(M, H, G, K_, beside, store, hd, rot):
+    """Against the product and the kernel behind it (rotation, cache write): where nothing is rotated the same bits - queries, what lies beside
+    the heads, keys and values in their pages, the rest of the pools as it was - with rotation to bf16's rounding (the separate kernel
+    rounds twice)."""
+    k = K()
+    N = (H + 2 * G) * hd + beside
+    a, w, bias = _rand(M, K_, dtype=torch.bfloat16, seed=51), _rand(N, K_, dtype=torch.bfloat16, seed=53, scale=0.05), _rand(N, seed=54, scale=0.5)
+    assert k.gemm_tc_qkv_rope_supported(a, w, H, G, hd, rot, beside)
+    assert not k.gemm_tc_qkv_rope_supported(a, w, H, G, hd, hd // 2, beside)
+    positions = torch.arange(M, dtype=torch.int32, device=DEV) * 3 % 200
+    slot_of_token = torch.arange(M, dtype=torch.int32, device=DEV) % 4
+    page_table = torch.randperm(16).to(torch.int32).view(4, 4).to(DEV)
+    inv = torch.tensor([1.0 / (10000.0 ** (2 * i / hd)) for i in range(hd // 2)], device=DEV)
+    k0, v0 = _paged(G, hd, 16, torch.bfloat16)
+    pools = [(k0.clone(), v0.clone()) for _ in range(2)]
+    ref, out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV), torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    k.gemm_tc(a, w, ref, k.OUT_SAME, bias)
+    k.rope_kv_write(ref, positions, slot_of_token, page_table, inv, H, G, hd, rot, False, *(pools[0] if store else (None, None)))
+    k.gemm_tc_qkv_rope(a, w, out, bias, positions, slot_of_token, page_table, inv if rot else None, False, H, G,
+                       *(pools[1] if store else (None, None)), beside=beside)
+    k.check_device_errors()
+    same = (lambda x, y: torch.testing.assert_close(x.float(), y.float(), rtol=2e-2, atol=2e-2)) if rot else (lambda x, y: torch.testing.assert_close(x, y, rtol=0, atol=0))
+    heads = (H + 2 * G) * hd
+    same(out[:, :H * hd], ref[:, :H * hd])
+    assert torch.equal(out[:, heads:], ref[:, heads:])
+    assert (out[:, H * hd:heads] == 7.0).all()
+    same(pools[1][0], pools[0][0])
+    assert torch.equal(pools[1][1], pools[0][1])
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 def test_gemm_tc_qkv_rope_at_positions_in_the_thousands(interleaved):
     k = K()
