@@ -265,9 +265,6 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv
     if (e.x < 0) return;                                 // spare chunk
     b = e.x; split = e.y & 0xffff; num_splits = e.y >> 16; len = e.z; cache_slot = e.w;
   }
-  // a sequence that is one chunk (always so without splits; with a plan, the short ones beside
-  // long ones) is finished here: no scratch, nothing for the combining kernel to do
-  const bool direct = num_splits == 1;
   const int start = dec_start(len, window);
   const int* pages = page_table + (size_t)cache_slot * max_pages;
 
@@ -284,6 +281,20 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv
   const int kept_blk = min((fin.keep_first + DEC_BLOCK - 1) / DEC_BLOCK, first_blk);
   const int num_blk = (len + DEC_BLOCK - 1) / DEC_BLOCK - first_blk + kept_blk;
   const int rounds = (num_blk + DEC_WARPS - 1) / DEC_WARPS;
+  // A short sequence of a cluster is one chunk after all (the launch does not know the lengths): the first CTA takes it whole, the
+  // others leave; no barriers, no trip through the cluster's memory.  One sequence, in eight chunks / whole: heads of 64, 64 tokens 4.3 / 2.6 us, 192
+  // 4.5 / 3.4, 320 4.4 / 4.2, 448 4.6 / 5.2; heads of 128, 100 tokens 4.9 / 4.0, 131 5.0 / 4.5, 256 5.1 / 5.4; four sequences, four chunks, 64 tokens
+  // 5.1 / 3.6, 131 5.1 / 5.1
+  constexpr int SHORT_ROUNDS = HD + VD <= 128 ? 3 : 2;
+  bool combines = clustered;
+  if (clustered && rounds <= SHORT_ROUNDS) {
+    if (split > 0) return;
+    num_splits = 1;
+    combines = false;
+  }
+  // a sequence that is one chunk (always so without splits; with a plan, the short ones beside
+  // long ones) is finished here: no scratch, nothing for the combining kernel to do
+  const bool direct = num_splits == 1;
   const int per_split = (rounds + num_splits - 1) / num_splits * DEC_WARPS;   // whole rounds: every warp gets a block of each
   const int blk_lo = split * per_split;                                      // places
   const int blk_hi = min(blk_lo + per_split, num_blk);
@@ -451,7 +462,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv
     const int h = gkv * m + r;
     if (direct) {
       out[(size_t)b * ldo + (size_t)h * VD + d] = __float2bfloat16_rn(dec_finish(O, L, M, fin, b, h * VD + d));
-    } else if (clustered) {
+    } else if (combines) {
       float* c_o = reinterpret_cast<float*>(dec_smem + SM::MERGE_BYTES);
       c_o[r * VD + d] = O;
       if (d == 0) { c_o[16 * VD + r] = M; c_o[16 * VD + 16 + r] = L; }
@@ -461,7 +472,7 @@ attention_decode_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv
       if (d == 0) { part_ml[2 * p] = M; part_ml[2 * p + 1] = L; }
     }
   }
-  if (clustered) {
+  if (combines) {
     // every chunk of the sequence has its result in shared memory; this CTA finishes its share
     // of the m x VD outputs, adding the chunks in their order
     dec_cluster_sync();

@@ -1335,6 +1335,26 @@ def test_gemm_tc_heads_is_a_product_a_head(M, H, N, K_, gap):
     k.check_device_errors()
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("lens", [[1], [16, 17], [64], [128], [129], [192], [193], [1, 128, 129, 700], [191, 5, 257, 193]])
+def test_attention_decode_clusters_with_short_sequences(hd, window, lens):
+    """Sequences about the length up to which the first CTA of a cluster takes a sequence whole, alone and beside long ones, against chunks
+    combined through global memory (the softmax's sums in another order: bf16 rounding)."""
+    k = K()
+    H, G, B = 8, 2, len(lens)
+    pools = torch.randn(2, 16 * B, G, 64, hd, device=DEV).to(torch.bfloat16)
+    pt = torch.randperm(16 * B).to(torch.int32).view(B, 16).to(DEV)
+    q = torch.randn(B, (H + 2 * G) * hd, device=DEV).to(torch.bfloat16)
+    slots, kv = torch.arange(B, dtype=torch.int32, device=DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+    for splits in (2, 4, 8):
+        out, ref = (torch.zeros(B, H * hd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        args = (q, pools[0], pools[1], pt, slots, kv)
+        k.attention_decode(*args, out, H, G, hd, hd ** -0.5, window, num_splits=splits, cluster=True)
+        k.attention_decode(*args, ref, H, G, hd, hd ** -0.5, window, num_splits=splits)
+        torch.testing.assert_close(out.float(), ref.float(), rtol=1e-2, atol=2e-3)
+
+
 # ----------------------------------------------------------------------------- 32-bit attention by tiles of rows
 @pytest.mark.parametrize("H,G,hd", [(4, 4, 64), (8, 2, 64), (15, 3, 64), (16, 1, 64), (3, 3, 128), (6, 1, 128), (28, 2, 128)])
 def test_attention_f32_tiles_are_exact_and_do_not_depend_on_the_cut(H, G, hd):
