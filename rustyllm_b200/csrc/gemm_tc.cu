@@ -681,7 +681,9 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
 static constexpr int PAIR_ROWS = 2 * BLOCK_N_OUT;
 static constexpr int PAIR_MAX_STAGES = 10;
 static constexpr int PAIR_RING_BYTES = 6 * (BLOCK_N_OUT + 128) * BLOCK_K * 2;      // six stages of tiles of 256 tokens
-static constexpr int PAIR_SMEM_BYTES = PAIR_RING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+static constexpr int PAIR_CHUNK = 32;              // an epilogue warp's piece of the output: 32 tokens x its 32 features
+static constexpr int PAIR_STAGING_BYTES = 8 * PAIR_CHUNK * 32 * 4;
+static constexpr int PAIR_SMEM_BYTES = PAIR_RING_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + PAIR_STAGING_BYTES;
 static constexpr int PAIR_ACC_COLS = 256;
 
 __device__ __forceinline__ void pair_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {
@@ -707,11 +709,53 @@ __device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
+// An epilogue warp's 32 features of `cols` tokens (from accumulator column 0 of tmem_acc), by pieces of 32 tokens through its staging area: the copy engine
+// stores a piece (bf16, float) or adds it to the output in L2 (float residual), so the warp waits for no load of the residual and its stores are whole
+// rows of a piece.  With loads and stores by the warps, 4 bytes a lane, products of K = 2,048 took as long by pairs as by CTAs alone: 5,514 tokens, us, alone /
+// pairs: 2,048 -> 3,072 63.4 / 63.2, 2,048 -> 2,048 into the residual 54.2 / 53.9, 8,192 -> 2,048 179 / 167; by the copy engine (another call) 54.5 / 50.3,
+// 44.8 / 38.3, 167 / 151; 3,000 tokens 33.5 / 27.7, 33.2 / 26.5, 106 / 88.  The tensor map ends at the output's last row and column.  (An addition in L2
+// is the float addition of the warps, but for subnormal numbers, which count as zero.)
+template <bool BF16>
+__device__ __forceinline__ void pair_epilogue_bulk(uint32_t tmem_acc, int quarter, int lane, int n0, int m0, int cols, int M, int N,
+                                                   const float* __restrict__ bias, const CUtensorMap* map_out, bool add, uint8_t* staging) {
+  const int n_first = n0 + quarter * 32;
+  const float b = (bias != nullptr && n_first + lane < N) ? bias[n_first + lane] : 0.f;
+#pragma unroll 1
+  for (int c = 0; c < cols; c += PAIR_CHUNK) {
+    uint32_t r[PAIR_CHUNK];
+    const uint32_t t = tmem_acc + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c;
+    tmem_ld16(t, *reinterpret_cast<uint32_t(*)[16]>(r));
+    tmem_ld16(t + 16, *reinterpret_cast<uint32_t(*)[16]>(r + 16));
+    tmem_ld_wait();
+    // the copy of the piece before has read the staging area
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < PAIR_CHUNK; ++j) {
+      const float v = __uint_as_float(r[j]) + b;
+      if constexpr (BF16) reinterpret_cast<__nv_bfloat16*>(staging)[j * 32 + lane] = __float2bfloat16_rn(v);
+      else reinterpret_cast<float*>(staging)[j * 32 + lane] = v;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0 && n_first < N && m0 + c < M) {
+      if (add)
+        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+                     ::"l"(map_out), "r"(smem_u32(staging)), "r"(n_first), "r"(m0 + c) : "memory");
+      else
+        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                     ::"l"(map_out), "r"(smem_u32(staging)), "r"(n_first), "r"(m0 + c) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_PERSISTENT_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                     const __grid_constant__ CUtensorMap map_a_tail, const float* __restrict__ bias,
                     void* __restrict__ out, int out_mode, int M, int N, int K, int ldo, int* __restrict__ err,
-                    int tile_m, int tiles_m, int num_tiles, int stages, const TcTail tail, float act_limit, float act_alpha) {
+                    int tile_m, int tiles_m, int num_tiles, int stages, const TcTail tail, float act_limit, float act_alpha,
+                    const __grid_constant__ CUtensorMap map_out, int bulk) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = smem;
@@ -827,6 +871,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // ---------------- epilogue warps: this CTA's 128 weight rows ----------------
     rl_pdl_wait();
     const int quarter = warp & 3, second = (warp - 2) >> 2;      // as in the kernel above
+    uint8_t* staging = smem + PAIR_RING_BYTES + 256 + (warp - 2) * (PAIR_STAGING_BYTES / 8);
     int t = 0;
     for (int tile = pair; tile < num_tiles; tile += pairs) {
       const TcTileAt at = tc_tile_at(tile, tiles_m, tile_m, tail);
@@ -841,19 +886,28 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       fuse.act_limit = act_limit;
       fuse.act_alpha = act_alpha;
       const int cols = min(at.bt, M - at.m0), half = min(cols, (at.bt / 2 + 31) & ~31), c0 = second ? half : 0;
-      tile_epilogue<256>(tmem_base + (uint32_t)(buf * PAIR_ACC_COLS + c0), quarter, lane, at.n0 * 2 + rank * BLOCK_N_OUT, at.m0 + c0,
-                         second ? cols - half : half, M, N, ldo, bias, out, out_mode, fuse, nullptr);
+      const uint32_t tmem_tile = tmem_base + (uint32_t)(buf * PAIR_ACC_COLS + c0);
+      const int n0 = at.n0 * 2 + rank * BLOCK_N_OUT, warp_cols = second ? cols - half : half;
+      if (bulk && out_mode == TC_OUT_BF16)
+        pair_epilogue_bulk<true>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, bias, &map_out, false, staging);
+      else if (bulk)
+        pair_epilogue_bulk<false>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, bias, &map_out, out_mode == TC_OUT_ADD_F32, staging);
+      else
+                           tile_epilogue<256>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, ldo, bias, out, out_mode, fuse, nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive(dsmem_addr(smem_u32(&acc_empty[buf]), 0));    // this warp has read the accumulator
       ++t;
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");       // this warp's pieces are in the output
   }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();        // nobody leaves while the other still signals it or reads its operands
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * PAIR_ACC_COLS) : "memory");
 }
+
+static int tc_make_out_map(CUtensorMap* map, void* out, int rows, int cols, int ld, bool bf16);
 
 // The height of equal tiles that cover M tokens with as few of them as tiles of 256 do, in steps of 32 (the instruction's two halves
 // in steps of 16).
@@ -903,12 +957,20 @@ static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const f
     rc = tc_make_map(&ma_tail, A, M, K, lda, tail.bt / 2);
     if (rc != RL_OK) return rc;
   }
+  // the output by the copy engine where its rows are whole 16-byte pieces
+  const bool bf16 = out_mode == TC_OUT_BF16;
+  const int bulk = (bf16 || out_mode == TC_OUT_F32 || out_mode == TC_OUT_ADD_F32) && ldo % (bf16 ? 8 : 4) == 0 && ((uintptr_t)out & 15) == 0;
+  CUtensorMap mo = mw;
+  if (bulk) {
+    rc = tc_make_out_map(&mo, out, M, N, ldo, bf16);
+    if (rc != RL_OK) return rc;
+  }
   const int stage_bytes = (BLOCK_N_OUT + tile_m / 2) * BLOCK_K * 2;
   const int stages = PAIR_RING_BYTES / stage_bytes < PAIR_MAX_STAGES ? PAIR_RING_BYTES / stage_bytes : PAIR_MAX_STAGES;
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
   cudaError_t e = rl_launch_pdl(gemm_tc_pair_kernel, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)PAIR_SMEM_BYTES, stream, mw, ma, ma_tail,
                                 bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, stages, tail,
-                                fuse.act_limit, fuse.act_alpha);
+                                fuse.act_limit, fuse.act_alpha, mo, bulk);
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_tc: launch of the kernel by pairs failed: %s", cudaGetErrorString(e));
     return RL_ERR_CUDA;
@@ -948,6 +1010,19 @@ int tc_make_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, 
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   RL_REQUIRE(r == CUDA_SUCCESS, "rl_gemm_tc: cuTensorMapEncodeTiled failed with %d (rows=%d cols=%d ld=%d box_rows=%d)",
              (int)r, rows, cols, ld, box_rows);
+  return RL_OK;
+}
+
+// The output [rows, cols] with row stride ld (elements) in boxes of 32 rows x 32 columns, as the pairs' epilogue warps store it.
+static int tc_make_out_map(CUtensorMap* map, void* out, int rows, int cols, int ld, bool bf16) {
+  EncodeTiledFn enc = get_encode_fn();
+  RL_REQUIRE(enc != nullptr, "rl_gemm_tc: the driver does not provide cuTensorMapEncodeTiled");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * (bf16 ? 2 : 4)};
+  cuuint32_t box[2] = {32, (cuuint32_t)PAIR_CHUNK}, estr[2] = {1, 1};
+  CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  RL_REQUIRE(r == CUDA_SUCCESS, "rl_gemm_tc: cuTensorMapEncodeTiled failed with %d for the output (rows=%d cols=%d ld=%d)", (int)r, rows, cols, ld);
   return RL_OK;
 }
 
