@@ -916,11 +916,14 @@ static int pair_tile(int M) {
   return (each + 31) / 32 * 32;
 }
 
-// Whether the pairs take a product of more than 128 tokens that is not split over K: where its tiles are more than one wave of them.
-// In one wave nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster barriers): us, CTAs
-// alone / pairs, 2,048 tokens 2,048 -> 3,072 34.2 / 36.2, 2,048 -> 2,048 26.9 / 29.5; 1,500 tokens 18.1 / 18.7, 18.5 / 19.5.
-static bool pairs_pay(int M, int N) {
-  return (M + 255) / 256 * ((N + PAIR_ROWS - 1) / PAIR_ROWS) > rl_num_sms() / 2;
+// Whether the pairs take a product of more than 128 tokens that is not split over K: where its tiles are more than one wave of them, or
+// three fifths of a wave and K is long.  In one wave nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster
+// barriers).  us, CTAs alone / pairs: 1,500 tokens 2,048 -> 2,048 16.4 / 17.1, 1,000 tokens 18.3 / 20.3, 293 tokens 4,096 -> 6,144 24.2 / 27.7, 800 tokens
+// 4,096 -> 4,096 29.4 / 29.7; 1,500 tokens 8,192 -> 2,048 (48 tiles of 74) 49.2 / 46.6, 2,048 tokens (64) 59.1 / 52.0, 1,000 tokens (32) 35.5 / 36.6,
+// 14,336 -> 4,096 (64) 98.4 / 88.2.
+static bool pairs_pay(int M, int N, int K) {
+  const int tiles = (M + 255) / 256 * ((N + PAIR_ROWS - 1) / PAIR_ROWS), pairs = rl_num_sms() / 2;
+  return tiles > pairs || (K >= 8192 && tiles * 5 >= pairs * 3);
 }
 
 static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const float* bias, void* out, int out_mode, int M, int N, int K,
@@ -1176,7 +1179,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   CUtensorMap mw, ma;
   int rc = tc_make_map(&mw, W, N, K, K, BLOCK_N_OUT);
   if (rc != RL_OK) return rc;
-  if (bt > 128 && splits == 1 && pairs_pay(M, N)) return launch_tc_pair(mw, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
+  if (bt > 128 && splits == 1 && pairs_pay(M, N, K)) return launch_tc_pair(mw, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
   fuse.tile_m = bt > 64 ? balanced_tile(M, bt) : bt;
   rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
   if (rc != RL_OK) return rc;

@@ -1298,22 +1298,31 @@ def test_gemm_tc_persistent_tiles_of_full_height(M):
     k.check_device_errors()
 
 
-@pytest.mark.parametrize("M,N,K_", [(129, 150 * 128 + 2, 8), (300, 75 * 256 - 130, 1032), (256, 75 * 256, 640), (777, 26 * 256 + 2, 2056)])
+@pytest.mark.parametrize("M,N,K_", [(129, 150 * 128 + 2, 8), (300, 75 * 256 - 130, 1032), (301, 75 * 256 - 136, 264), (256, 75 * 256, 640), (777, 26 * 256 + 8, 2056),
+                                    (1025, 2303, 8200)])
 def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
-    """More tiles of 256 x 256 than pairs of SMs, so pairs of CTAs take them: a K shorter than a block, rings that go round several times
-    with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave.  Float sums of K products."""
+    """More tiles of 256 x 256 than pairs of SMs, or more than three fifths and a long K, so pairs of CTAs take them: a K shorter than a block, rings
+    that go round several times with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave;
+    outputs stored by the copy engine (rows of whole 16-byte pieces) that end inside its pieces of 32 x 32, and by the warps.  Float sums of K
+    products; rows behind the last stay as they are."""
     k = K()
     assert k.gemm_tc_splits(M, N, K_) == 1
-    a, w = _rand(M, K_, dtype=torch.bfloat16, seed=1), _rand(N, K_, dtype=torch.bfloat16, seed=2)
+    a, w, bias = _rand(M, K_, dtype=torch.bfloat16, seed=1), _rand(N, K_, dtype=torch.bfloat16, seed=2), _rand(N, seed=3)
     ref = a.double() @ w.double().T
     res = _rand(M + 3, N, seed=4)
-    out = res.clone()
-    k.gemm_tc(a, w, out[:M], k.OUT_ADD_F32)
-    torch.testing.assert_close(out[:M].double(), ref + res[:M].double(), rtol=1e-4, atol=8e-5 * math.sqrt(K_))
-    assert torch.equal(out[M:], res[M:])
-    again = res.clone()
-    k.gemm_tc(a, w, again[:M], k.OUT_ADD_F32)
-    assert torch.equal(out, again)
+    f32 = dict(rtol=1e-4, atol=8e-5 * math.sqrt(K_))
+    for b in (None, bias):
+        full = ref + (b.double() if b is not None else 0.0)
+        out, again, flt, same = res.clone(), res.clone(), res.clone(), res.to(torch.bfloat16)
+        k.gemm_tc(a, w, out[:M], k.OUT_ADD_F32, b)
+        torch.testing.assert_close(out[:M].double(), full + res[:M].double(), **f32)
+        k.gemm_tc(a, w, again[:M], k.OUT_ADD_F32, b)
+        assert torch.equal(out, again)
+        k.gemm_tc(a, w, flt[:M], k.OUT_F32, b)
+        torch.testing.assert_close(flt[:M].double(), full, **f32)
+        k.gemm_tc(a, w, same[:M], k.OUT_SAME, b)
+        torch.testing.assert_close(same[:M].double(), full, rtol=1e-2, atol=1e-2 * math.sqrt(K_))
+        assert torch.equal(out[M:], res[M:]) and torch.equal(flt[M:], res[M:]) and torch.equal(same[M:], res[M:].to(torch.bfloat16))
     k.check_device_errors()
 
 
