@@ -1134,14 +1134,17 @@ def latent_prepare(u: torch.Tensor, q_rank: int, kv_rank: int, rot_dim: int, q_w
 def latent_query(q: torch.Tensor, out: torch.Tensor, num_heads: int, head_dim: int, rot_dim: int, latent_dim: int,
                  positions: torch.Tensor, inv_freq: torch.Tensor, rotary_dim: int, interleaved: bool, magnitude: float = 1.0) -> None:
     """q [M, H * (hd + rd)] (a head: [plain | rotary]); the turned rotary parts go behind the ``latent_dim`` columns of
-    each head of ``out`` [M, H * (latent_dim + rd)].  ``magnitude``: a factor on every cosine and sine."""
-    _need(q, "q", contiguous=False); _need(out, "out", q.dtype); _need(positions, "positions", torch.int32)
+    each head of ``out`` [M, H * (latent_dim + rd)].  ``out`` may be ``q`` itself, columns of a wider row or not.
+    ``magnitude``: a factor on every cosine and sine."""
+    _need(q, "q", contiguous=False); _need(out, "out", q.dtype, contiguous=False); _need(positions, "positions", torch.int32)
     _need(inv_freq, "inv_freq", torch.float32)
     M = q.shape[0]
-    assert q.stride(1) == 1 and q.shape[1] == num_heads * (head_dim + rot_dim) and out.shape == (M, num_heads * (latent_dim + rot_dim))
+    assert q.stride(1) == 1 and q.shape[1] == num_heads * (head_dim + rot_dim)
+    assert out.stride(1) == 1 and out.shape == (M, num_heads * (latent_dim + rot_dim))
     ldq = q.stride(0) if M > 1 else q.shape[1]
+    ldo = out.stride(0) if M > 1 else out.shape[1]
     _check(library().rl_latent_query(q.data_ptr(), ldq, _dt(q), num_heads, head_dim, rot_dim, positions.data_ptr(),
-                                     inv_freq.data_ptr(), int(rotary_dim), int(bool(interleaved)), float(magnitude), out.data_ptr(), out.stride(0),
+                                     inv_freq.data_ptr(), int(rotary_dim), int(bool(interleaved)), float(magnitude), out.data_ptr(), ldo,
                                      latent_dim, M, _stream()), "rl_latent_query")
     _count()
 

@@ -705,6 +705,33 @@ def test_configurations_drawn_at_random(tmp_path, seed, dtype):
     close(torch.cat(rows_b), plain_logits(d, b, ch.of(s[1])), dtype, cfg, f"random {seed} {dtype} b")
 
 
+def test_prompts_whose_keys_and_values_are_made_of_the_latents(tmp_path, monkeypatch):
+    """Latent layers without a query latent (the queries are columns of the first product's rows), with a gate an element, of the widths that
+    keys and values are made for: a prompt whole, in portions behind what is cached and beside another, against the plain
+    implementation."""
+    from rustyllm_b200 import kernels as K
+    cfg = {"architecture": "Buketar", "vocab": 97, "width": 136, "norm": {"eps": 1e-5}, "streams": 2, "logit_softcap": 20.0,
+           "layers": [C.latent(5, 128, 64, 128, 256, 0.07, None, base=1.0e4, scaling=(8.0, 64, 8.0, 1.0)),
+                      C.latent(2, 128, 64, 128, 264, 0.07, None, base=1.0e5)]}
+    d = C.write_model(str(tmp_path / "made"), cfg)
+    made = []
+    plain = K.attention_prefill_shared_part
+    monkeypatch.setattr(K, "attention_prefill_shared_part", lambda *a, **kw: (made.append(a[0].shape[0]), plain(*a, **kw)))
+    r = runner(d, "bfloat16")
+    a, b = random_tokens(cfg["vocab"], 400, 91), random_tokens(cfg["vocab"], 261, 92)
+    s, t = r.engine.alloc_slot(), r.engine.alloc_slot()
+    both = r.engine.step([s, t], [a, b], "all")
+    r.engine.free_slot(s); r.engine.free_slot(t)
+    s = r.engine.alloc_slot()
+    cut = torch.cat([r.engine.step([s], [a[i:i + 200]], "all") for i in (0, 200)])
+    r.engine.free_slot(s)
+    K.check_device_errors()
+    assert made == [661] * 2 + [200] * 4
+    close(both[:400], plain_logits(d, a), "bfloat16", cfg, "beside another")
+    close(both[400:], plain_logits(d, b), "bfloat16", cfg, "the other")
+    close(cut, plain_logits(d, a), "bfloat16", cfg, "in portions")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", NAMES)
 def test_greedy_generation_through_the_runner(dirs, name, dtype):
