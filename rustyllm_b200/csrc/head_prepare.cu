@@ -402,10 +402,12 @@ latent_query_kernel(const T* __restrict__ q, int ldq, int H, int hd, int rd, con
   }
 }
 
+// The same by pairs: a thread reads both elements of a pair before it writes either and no other thread touches them, so out may be q
+// itself (lat = hd, one row stride).
 template <typename T>
 __global__ void __launch_bounds__(HP_THREADS)
-latent_query_pairs_kernel(const T* __restrict__ q, int ldq, int H, int hd, int rd, const int* __restrict__ positions,
-                          const float* __restrict__ inv_freq, int rot, int interleaved, float magnitude, T* __restrict__ out, int ldo, int lat) {
+latent_query_pairs_kernel(const T* q, int ldq, int H, int hd, int rd, const int* __restrict__ positions,
+                          const float* __restrict__ inv_freq, int rot, int interleaved, float magnitude, T* out, int ldo, int lat) {
   rl_pdl_trigger();
   rl_pdl_wait();
   const int m = blockIdx.x;
@@ -418,7 +420,8 @@ latent_query_pairs_kernel(const T* __restrict__ q, int ldq, int H, int hd, int r
   }
 }
 
-// q [M, ldq]: H heads of [hd | rd]; out [M, ldo]: H heads of [lat | rd], of which this fills the rd columns.
+// q [M, ldq]: H heads of [hd | rd]; out [M, ldo]: H heads of [lat | rd], of which this fills the rd columns.  out may be q itself where the kernel by
+// pairs takes the call (even widths and strides, both elements of a pair in one aligned piece), else they must not overlap.
 extern "C" int rl_latent_query(const void* q, int ldq, int dtype, int num_heads, int head_dim, int rot_dim, const int* positions,
                                const float* inv_freq, int rotary_dim, int interleaved, float magnitude, void* out, int ldo, int latent_dim,
                                int num_tokens, cudaStream_t stream) {
@@ -430,6 +433,8 @@ extern "C" int rl_latent_query(const void* q, int ldq, int dtype, int num_heads,
   const uintptr_t two = dtype == RL_F32 ? 8 : 4;
   const bool pairs = head_dim % 2 == 0 && rot_dim % 2 == 0 && latent_dim % 2 == 0 && ldq % 2 == 0 &&
                      ldo % 2 == 0 && (uintptr_t)q % two == 0 && (uintptr_t)out % two == 0;
+  RL_REQUIRE(out != q || (pairs && latent_dim == head_dim && ldo == ldq),
+             "rl_latent_query: turned in place, heads must stay where they are and widths, strides and bases be those of whole pairs");
   if (pairs && dtype == RL_F32)
     rl_launch_pdl(latent_query_pairs_kernel<float>, num_tokens, HP_THREADS, 0, stream, (const float*)q, ldq, num_heads, head_dim, rot_dim,
                   positions, inv_freq, rotary_dim, interleaved, magnitude, (float*)out, ldo, latent_dim);

@@ -113,3 +113,19 @@ def test_plain_masks():
     w = P.window_mask(10, 3)
     assert w[5].tolist() == [False] * 3 + [True] * 3 + [False] * 4
     assert P.chunk_mask(4, None).tolist() == P.window_mask(4, None).tolist() == torch.ones(4, 4).tril().bool().tolist()
+
+
+@pytest.mark.parametrize("what", ["odd base", "odd stride", "odd width", "another width"])
+def test_a_rotation_in_place_that_could_overwrite_a_partner_is_refused(what):
+    """In place only the kernel that owns whole pairs is safe; a call that it cannot take is refused before anything is launched (the
+    buffer is host memory: no kernel could read it)."""
+    from rustyllm_b200 import kernels
+    H, hd, rd, lat = 2, 7 if what == "odd width" else 8, 4, 10 if what == "another width" else 8
+    lat = hd if what == "odd width" else lat
+    ld = H * (lat + rd) + (1 if what == "odd stride" else 0)
+    buf = torch.zeros(3 * ld + 1, dtype=torch.bfloat16)
+    base = buf.data_ptr() + (2 if what == "odd base" else 0)
+    positions, freq = torch.zeros(3, dtype=torch.int32), torch.ones(2)
+    lib = kernels.library()
+    rc = lib.rl_latent_query(base, ld, 1, H, hd, rd, positions.data_ptr(), freq.data_ptr(), 4, 0, 1.0, base, ld, lat, 3, None)
+    assert rc == -1 and b"in place" in lib.rl_last_error()
