@@ -456,8 +456,8 @@ extern "C" int rl_latent_query(const void* q, int ldq, int dtype, int num_heads,
 // ------------------------------------------------------------------ the cached rows that a step sees, out of their pages
 // A block a page: out [runs * RL_PAGE, width] takes the pages of sequence after sequence, from the pair of pages (the attention's tile)
 // that holds the first position any of the step's rows sees; table [num_seqs, max_pages] says which run of RL_PAGE rows a page became,
-// and table_rows = 0, 1, ...  Rows behind a sequence's end come as they are in its last page.  Bound by one read and one write of
-// the rows.
+// and table_rows = 0, 1, ...  Rows behind a sequence's end, and of a pair's first page that the window has left (it may have been given to
+// another sequence), come as zeros: the attention multiplies what is there by a probability of 0.  Bound by one read and one write of the rows.
 __global__ void __launch_bounds__(HP_THREADS)
 latent_gather_kernel(const uint4* __restrict__ pool, int pieces, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_slots,
                      const int* __restrict__ kv_lens, int num_seqs, const int* __restrict__ page_table, int max_pages, int window,
@@ -475,9 +475,10 @@ latent_gather_kernel(const uint4* __restrict__ pool, int pieces, const int* __re
       table[(size_t)b * max_pages + p0 + run] = blockIdx.x;
       if (run == 0) table_rows[b] = b;
     }
+    const int p = p0 + run, own = p < first / RL_PAGE ? 0 : min(RL_PAGE, kv - p * RL_PAGE);     // rows that are the sequence's
     const uint4* src = rl_behind_wait(pool) + (size_t)page * RL_PAGE * pieces;
     uint4* dst = out + (size_t)blockIdx.x * RL_PAGE * pieces;
-    for (int i = threadIdx.x; i < RL_PAGE * pieces; i += HP_THREADS) dst[i] = src[i];
+    for (int i = threadIdx.x; i < RL_PAGE * pieces; i += HP_THREADS) dst[i] = i < own * pieces ? src[i] : make_uint4(0u, 0u, 0u, 0u);
     return;
   }
 }

@@ -838,6 +838,38 @@ def test_keys_and_values_made_of_the_latents_a_step_sees(H, r, per_head, window)
         torch.testing.assert_close(torch.cat(got[b]).view(n, H, 128), ref, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("window", [None, 130])
+def test_gathered_latents_hold_nothing_of_other_sequences(window):
+    """A page that the window has left and that another sequence owns by now, and rows behind the sequence's end that were used before, hold
+    what is no number: the gathered rows there are zeros, the sequence's own are as cached."""
+    from rustyllm_b200 import kernels as K
+    from rustyllm_b200.cache.sequence_cache import KVNeed, SequenceCache
+    torch.manual_seed(5)
+    r, bf = 64, torch.bfloat16
+    cache = SequenceCache([KVNeed(1, r + 64, window, 0)], [None], 64 * 8, bf, DEV, max_slots=2)
+    slot = cache.alloc_slot()
+    group, layer = cache.kv_entry(0)
+    pool = group.k_pool(layer)
+    pool.fill_(math.nan)
+    rows = torch.randn(350, r + 64, device=DEV).to(bf)
+    for at, cnt in ((0, 200), (200, 150)):
+        cache.prepare([slot], [cnt])
+        pages = group.page_table[slot].tolist()
+        if window and at:
+            pool[pages[0]].fill_(math.nan)                   # given back behind the first step
+            assert group.slot_pages[slot][0] == -1
+        for i in range(at, at + cnt):
+            pool[pages[i // 64], 0, i % 64] = rows[i]
+        st = step_state(slot, at, cnt)
+        runs = K.latent_runs(st.q_lens, st.kv_lens_host, window or 0)
+        lat, table, table_rows = K.latent_gather(pool, group.page_table, st, window or 0, runs)
+        seen = 64 if window and at else 0                    # position 71 is the first that the second step's tokens see
+        assert runs == -(-(at + cnt) // 64) and table_rows.tolist() == [0] and table[0, :runs].tolist() == list(range(runs))
+        assert (lat[:seen] == 0).all() and torch.equal(lat[seen:at + cnt], rows[seen:at + cnt]) and (lat[at + cnt:] == 0).all()
+        cache.commit([slot], [cnt])
+    K.check_device_errors()
+
+
 def test_made_keys_and_widened_queries_agree():
     """A model whose latent layers have the widths that keys and values are made for: a prompt whole, in portions (behind what is cached) and
     beside another, against the route that widens the queries."""
