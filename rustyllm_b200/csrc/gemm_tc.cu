@@ -893,7 +893,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       else if (bulk)
         pair_epilogue_bulk<false>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, bias, &map_out, out_mode == TC_OUT_ADD_F32, staging);
       else
-                           tile_epilogue<256>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, ldo, bias, out, out_mode, fuse, nullptr);
+        tile_epilogue<256>(tmem_tile, quarter, lane, n0, at.m0 + c0, warp_cols, M, N, ldo, bias, out, out_mode, fuse, nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive(dsmem_addr(smem_u32(&acc_empty[buf]), 0));    // this warp has read the accumulator
@@ -916,18 +916,30 @@ static int pair_tile(int M) {
   return (each + 31) / 32 * 32;
 }
 
-// Whether the pairs take a product of more than 128 tokens that is not split over K: where its tiles are more than one wave of them, or
-// three fifths of a wave and K is long.  In one wave nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster
-// barriers).  us, CTAs alone / pairs: 1,500 tokens 2,048 -> 2,048 16.4 / 17.1, 1,000 tokens 18.3 / 20.3, 293 tokens 4,096 -> 6,144 24.2 / 27.7, 800 tokens
-// 4,096 -> 4,096 29.4 / 29.7; 1,500 tokens 8,192 -> 2,048 (48 tiles of 74) 49.2 / 46.6, 2,048 tokens (64) 59.1 / 52.0, 1,000 tokens (32) 35.5 / 36.6,
-// 14,336 -> 4,096 (64) 98.4 / 88.2.
-static bool pairs_pay(int M, int N, int K) {
-  const int tiles = (M + 255) / 256 * ((N + PAIR_ROWS - 1) / PAIR_ROWS), pairs = rl_num_sms() / 2;
-  return tiles > pairs || (K >= 8192 && tiles * 5 >= pairs * 3);
+// Whether the pairs' outputs go by the copy engine: float and bf16 outputs whose rows are whole 16-byte pieces.
+static bool pair_bulk(const void* out, int out_mode, int ldo) {
+  const bool bf16 = out_mode == TC_OUT_BF16;
+  return (bf16 || out_mode == TC_OUT_F32 || out_mode == TC_OUT_ADD_F32) && ldo % (bf16 ? 8 : 4) == 0 && ((uintptr_t)out & 15) == 0;
+}
+
+// Whether the pairs take a product of more than 128 tokens that is not split over K.  us, CTAs alone / pairs:
+// Not where they need more waves (an odd number of 128-row weight tiles leaves the last pair half empty): bf16 outputs, 20,480 tokens 2,048 -> 64
+// 20.1 / 26.3 (one wave / two), 10,240 tokens 2,048 -> 384 20.1 / 25.2, 12,000 tokens 4,096 -> 260 35.4 / 47.5, 8,192 tokens 2,048 -> 1,152 33.7 / 36.2 (two / three);
+// as many waves: 5,000 tokens -> 1,152 27.3 / 26.0, 8,192 tokens -> 520 27.8 / 25.6, 20,480 tokens -> 200 31.1 / 27.0.
+// More than one wave of tiles: from K = 512 on (float outputs 1,024, outputs by the warps 2,048); below, a tile's time is its
+// epilogue and its start.  bf16, 20,480 tokens -> 200, K = 512 13.2 / 11.0; 2,048 tokens -> 8,192, gated, K = 1,024 42.0 / 43.1, 2,048 56.5 / 54.2; bf16 rows of 8,188,
+// K = 512 25.0 / 31.3, 2,048 56.6 / 53.3; float, 5,000 tokens -> 4,096, K = 512 30.7 / 32.2, 1,024 42.2 / 38.8.
+// One wave, where nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster barriers): three fifths of it and K from 8,192 on.
+static bool pairs_pay(int M, int N, int K, int out_mode, bool bulk) {
+  const int tiles_m = (M + 255) / 256, tiles = tiles_m * ((N + PAIR_ROWS - 1) / PAIR_ROWS), sms = rl_num_sms(), pairs = sms / 2;
+  const int alone = tiles_m * ((N + BLOCK_N_OUT - 1) / BLOCK_N_OUT);
+  if ((tiles + pairs - 1) / pairs > (alone + sms - 1) / sms) return false;
+  const int least = !bulk ? 2048 : out_mode == TC_OUT_F32 ? 1024 : 512;
+  return tiles > pairs ? K >= least : K >= 8192 && tiles * 5 >= pairs * 3;
 }
 
 static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const float* bias, void* out, int out_mode, int M, int N, int K,
-                          int ldo, int* err, cudaStream_t stream, const TcFuse& fuse) {
+                          int ldo, int* err, cudaStream_t stream, const TcFuse& fuse, bool bulk) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
@@ -960,12 +972,9 @@ static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const f
     rc = tc_make_map(&ma_tail, A, M, K, lda, tail.bt / 2);
     if (rc != RL_OK) return rc;
   }
-  // the output by the copy engine where its rows are whole 16-byte pieces
-  const bool bf16 = out_mode == TC_OUT_BF16;
-  const int bulk = (bf16 || out_mode == TC_OUT_F32 || out_mode == TC_OUT_ADD_F32) && ldo % (bf16 ? 8 : 4) == 0 && ((uintptr_t)out & 15) == 0;
   CUtensorMap mo = mw;
   if (bulk) {
-    rc = tc_make_out_map(&mo, out, M, N, ldo, bf16);
+    rc = tc_make_out_map(&mo, out, M, N, ldo, out_mode == TC_OUT_BF16);
     if (rc != RL_OK) return rc;
   }
   const int stage_bytes = (BLOCK_N_OUT + tile_m / 2) * BLOCK_K * 2;
@@ -973,7 +982,7 @@ static int launch_tc_pair(const CUtensorMap& mw, const void* A, int lda, const f
   const int grid = 2 * (num_tiles < pairs ? num_tiles : pairs);
   cudaError_t e = rl_launch_pdl(gemm_tc_pair_kernel, dim3(grid), dim3(TC_PERSISTENT_THREADS), (size_t)PAIR_SMEM_BYTES, stream, mw, ma, ma_tail,
                                 bias, out, out_mode, M, N, K, ldo, err, tile_m, tiles_m, num_tiles, stages, tail,
-                                fuse.act_limit, fuse.act_alpha, mo, bulk);
+                                fuse.act_limit, fuse.act_alpha, mo, bulk ? 1 : 0);
   if (e != cudaSuccess) {
     rl_set_error("rl_gemm_tc: launch of the kernel by pairs failed: %s", cudaGetErrorString(e));
     return RL_ERR_CUDA;
@@ -1179,7 +1188,10 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   CUtensorMap mw, ma;
   int rc = tc_make_map(&mw, W, N, K, K, BLOCK_N_OUT);
   if (rc != RL_OK) return rc;
-  if (bt > 128 && splits == 1 && pairs_pay(M, N, K)) return launch_tc_pair(mw, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
+  if (bt > 128 && splits == 1) {
+    const bool bulk = pair_bulk(out, out_mode, ldo);
+    if (pairs_pay(M, N, K, out_mode, bulk)) return launch_tc_pair(mw, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse, bulk);
+  }
   fuse.tile_m = bt > 64 ? balanced_tile(M, bt) : bt;
   rc = tc_make_map(&ma, A, M, K, lda, fuse.tile_m);
   if (rc != RL_OK) return rc;
@@ -1195,6 +1207,11 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   }
   if (bt == 128) return launch_tc_persistent<128>(mw, ma, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
   return launch_tc_persistent<256>(mw, ma, A, lda, bias, out, out_mode, M, N, K, ldo, err, stream, fuse);
+}
+
+// 1 if rl_gemm_tc runs a product with this output by pairs of CTAs (the number of K parts not forced).
+extern "C" int rl_gemm_tc_by_pairs(const void* out, int out_mode, int M, int N, int K, int ldo) {
+  return token_tile(M) > 128 && rl_gemm_tc_splits(M, N, K) == 1 && pairs_pay(M, N, K, out_mode, pair_bulk(out, out_mode, ldo));
 }
 
 // act_limit, act_alpha: the constants of out_mode 7 (else unused)

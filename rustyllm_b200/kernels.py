@@ -221,6 +221,7 @@ _SIGNATURES = {
                        _c_void_p, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_float, _c_float,
                        _c_void_p],
     "rl_gemm_tc_splits": [_c_int, _c_int, _c_int],
+    "rl_gemm_tc_by_pairs": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int],
     "rl_gemm_tc_qkv_rope_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int],
     "rl_gemm_tc_qkv_rope": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                             _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
@@ -1546,6 +1547,11 @@ def _tc_error_word(device: torch.device) -> torch.Tensor:
 def gemm_tc_splits(M: int, N: int, K: int) -> int:
     """Parts (cluster size) the kernel cuts the K range into for these shapes."""
     return int(library().rl_gemm_tc_splits(M, N, K))
+
+
+def gemm_tc_by_pairs(out: torch.Tensor, out_mode: int, M: int, N: int, K: int) -> bool:
+    """Whether ``gemm_tc`` runs a product with this output by pairs of CTAs."""
+    return bool(library().rl_gemm_tc_by_pairs(out.data_ptr(), out_mode, M, N, K, out.stride(0) if M > 1 else out.shape[1]))
 
 
 def check_device_errors() -> None:

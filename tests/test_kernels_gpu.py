@@ -1298,11 +1298,14 @@ def test_gemm_tc_persistent_tiles_of_full_height(M):
     k.check_device_errors()
 
 
-@pytest.mark.parametrize("M,N,K_", [(129, 150 * 128 + 2, 8), (300, 75 * 256 - 130, 1032), (301, 75 * 256 - 136, 264), (256, 75 * 256, 640), (777, 26 * 256 + 8, 2056),
-                                    (1025, 2303, 8200)])
-def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
-    """More tiles of 256 x 256 than pairs of SMs, or more than three fifths and a long K, so pairs of CTAs take them: a K shorter than a block, rings
-    that go round several times with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave;
+@pytest.mark.parametrize("M,N,K_,by_pairs", [(129, 150 * 128 + 2, 8, ""), (300, 75 * 256 - 130, 1032, ""), (301, 75 * 256 - 136, 264, ""), (256, 75 * 256, 640, "as"),
+                                             (777, 26 * 256 + 8, 2056, "afsg"), (1025, 2303, 8200, "afs"), (300, 75 * 256 - 130, 2056, "afsg"),
+                                             (301, 74 * 256 + 64, 1024, "afs"), (301, 74 * 256 + 72, 2184, "afsg"), (129, 75 * 256, 512, "as"), (2000, 2048, 520, ""),
+                                             (20000, 248, 520, "as"), (20000, 128, 2048, ""), (5200, 640, 2048, "")])
+def test_gemm_tc_pairs_rings_and_edges(M, N, K_, by_pairs):
+    """More tiles of 256 x 256 than pairs of SMs, or more than three fifths and a long K, so pairs of CTAs take them (``by_pairs``: additions into the
+    residual, float, bf16 and gated outputs; the others and those of short K or of more waves by pairs than by CTAs alone go there): the shortest
+    K, rings that go round several times with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave;
     outputs stored by the copy engine (rows of whole 16-byte pieces) that end inside its pieces of 32 x 32, and by the warps.  Float sums of K
     products; rows behind the last stay as they are."""
     k = K()
@@ -1311,6 +1314,9 @@ def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
     ref = a.double() @ w.double().T
     res = _rand(M + 3, N, seed=4)
     f32 = dict(rtol=1e-4, atol=8e-5 * math.sqrt(K_))
+    act = _rand(M + 3, N // 2, dtype=torch.bfloat16, seed=5)
+    outs = {"a": (k.OUT_ADD_F32, res), "f": (k.OUT_F32, res), "s": (k.OUT_SAME, res.to(torch.bfloat16)), "g": (k.OUT_SWIGLU, act)}
+    assert "".join(c for c, (mode, o) in outs.items() if (c != "g" or N % 2 == 0) and k.gemm_tc_by_pairs(o, mode, M, N, K_)) == by_pairs
     for b in (None, bias):
         full = ref + (b.double() if b is not None else 0.0)
         out, again, flt, same = res.clone(), res.clone(), res.clone(), res.to(torch.bfloat16)
@@ -1323,6 +1329,13 @@ def test_gemm_tc_pairs_rings_and_edges(M, N, K_):
         k.gemm_tc(a, w, same[:M], k.OUT_SAME, b)
         torch.testing.assert_close(same[:M].double(), full, rtol=1e-2, atol=1e-2 * math.sqrt(K_))
         assert torch.equal(out[M:], res[M:]) and torch.equal(flt[M:], res[M:]) and torch.equal(same[M:], res[M:].to(torch.bfloat16))
+    if N % 2 == 0:
+        scale = 2.0 ** -round(math.log2(math.sqrt(K_)))            # gates of about 1; a power of two: the weights stay bf16
+        gated = act.clone()
+        k.gemm_tc(a, w * scale, gated[:M], k.OUT_SWIGLU)
+        small = ref * scale
+        torch.testing.assert_close(gated[:M].double(), torch.nn.functional.silu(small[:, 0::2]) * small[:, 1::2], rtol=2e-2, atol=2e-2)
+        assert torch.equal(gated[M:], act[M:])
     k.check_device_errors()
 
 
