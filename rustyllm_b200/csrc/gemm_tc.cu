@@ -389,8 +389,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
           for (int u = 0; u < U; ++u) { v[u].x += t[u].x; v[u].y += t[u].y; v[u].z += t[u].z; v[u].w += t[u].w; }
         }
-        // (warp-uniform) the last of this warp's reads: the other parts need not wait for its stores (64 tokens: 1,525 us a step so, 1,512 without)
-        if (BT != 64 && j0 + step * U >= cols) {
+        // (warp-uniform) the last of this warp's reads: the other parts need not wait for its stores.  Up to 32 tokens only; us, without / so: 8 tokens
+        // 2,048 -> 2,048 5.28 / 5.15, 4,096 -> 6,144 11.5 / 11.5; 48 tokens 2,048 -> 2,048 6.97 / 7.33, 8,192 -> 2,048 13.5 / 13.9; 128 tokens 2,048 -> 2,048
+        // 16.3 / 16.0, 4,096 -> 4,096 13.9 / 14.3; 256 tokens 2,048 -> 2,048 25.3 / 27.0, 8,192 -> 2,048 38.0 / 38.8, 4,096 -> 4,096 20.9 / 21.2
+        if (BT < 64 && j0 + step * U >= cols) {
           __syncwarp();
           cluster_arrive();
           arrived = true;
