@@ -716,7 +716,7 @@ __device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) {
 // rows of a piece.  With loads and stores by the warps, 4 bytes a lane, products of K = 2,048 took as long by pairs as by CTAs alone: 5,514 tokens, us, alone /
 // pairs: 2,048 -> 3,072 63.4 / 63.2, 2,048 -> 2,048 into the residual 54.2 / 53.9, 8,192 -> 2,048 179 / 167; by the copy engine (another call) 54.5 / 50.3,
 // 44.8 / 38.3, 167 / 151; 3,000 tokens 33.5 / 27.7, 33.2 / 26.5, 106 / 88.  The tensor map ends at the output's last row and column.  (An addition in L2
-// is the float addition of the warps, but for subnormal numbers, which count as zero.)
+// is the float addition of the warps, subnormal numbers too.)
 template <bool BF16>
 __device__ __forceinline__ void pair_epilogue_bulk(uint32_t tmem_acc, int quarter, int lane, int n0, int m0, int cols, int M, int N,
                                                    const float* __restrict__ bias, const CUtensorMap* map_out, bool add, uint8_t* staging) {

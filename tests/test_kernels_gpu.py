@@ -1339,6 +1339,27 @@ def test_gemm_tc_pairs_rings_and_edges(M, N, K_, by_pairs):
     k.check_device_errors()
 
 
+@pytest.mark.parametrize("M,N,K_,pad", [(300, 75 * 256 - 130, 520, 2), (300, 75 * 256 - 130, 2056, 1), (1025, 2303, 8200, 1), (129, 2048, 64, 0)])
+def test_gemm_tc_additions_into_the_residual_keep_subnormal_numbers(M, N, K_, pad):
+    """By pairs (added by the copy engine, and by the warps where rows are no whole 16-byte pieces) and by CTAs alone: residuals below the smallest
+    normal float, products that are, and normal ones whose sum is.  A product is one number, so each sum rounds once: the float nearest to
+    it, bit for bit."""
+    k = K()
+    tiny = torch.finfo(torch.float32).tiny
+    a, w = torch.zeros(M, K_, device=DEV, dtype=torch.bfloat16), torch.zeros(N, K_, device=DEV, dtype=torch.bfloat16)
+    w[:, 0] = (-16.0 * tiny * (1 + torch.arange(N) % 4)).to(DEV)
+    a[:, 0] = torch.tensor([0.0, 2.0 ** -4, 2.0 ** -9])[torch.arange(M) % 3].to(DEV)         # nothing, a normal and a subnormal number to add
+    small = torch.randint(1, 1 << 22, (M, N + pad), dtype=torch.int32).view(torch.float32)    # bit patterns of subnormal numbers
+    res = torch.where(torch.rand(M, N + pad) < 0.5, small, 2.5 * tiny * torch.rand(M, N + pad)).to(DEV)
+    out = res.clone()
+    assert k.gemm_tc_by_pairs(out[:, :N], k.OUT_ADD_F32, M, N, K_) == (M != 129)
+    k.gemm_tc(a, w, out[:, :N], k.OUT_ADD_F32)
+    ref = (res[:, :N].double() + a[:, :1].double() * w[:, 0].double()).float()
+    k.check_device_errors()
+    assert ((ref != 0) & (ref.abs() < tiny)).any()
+    assert torch.equal(out[:, :N], ref) and torch.equal(out[:, N:], res[:, N:])
+
+
 @pytest.mark.parametrize("M,H,N,K_,gap", [(65, 3, 40, 64, 8), (129, 16, 512, 128, 64), (300, 5, 130, 192, 0), (1000, 2, 128, 512, 24)])
 def test_gemm_tc_heads_is_a_product_a_head(M, H, N, K_, gap):
     """Heads that lie apart in wider rows on both sides; what lies between them stays as it is.  Float sums, one rounding to bf16."""
