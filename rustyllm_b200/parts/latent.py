@@ -6,7 +6,7 @@ rd and a value width vd, a query latent of q_rank and a key/value latent of kv_r
 
     cq = n(Wdq h) wq;   q = Wuq cq, a head laid out [plain (hd) | rotary (rd)]
     [c | kr] = Wdkv h;  c <- n(c) wkv (kv_rank);  kr (rd) is turned by the position and serves every head
-    k_a = Wuk_a c,  v_a = Wuv_a c                                   (head a; neither is ever materialised)
+    k_a = Wuk_a c,  v_a = Wuv_a c                                   (head a; materialised for prompt steps alone)
     s_ij = (q_plain_i . k_a,j + rot(q_rot_i) . rot(kr_j)) * scale,  0 <= i - j < window;  softmax
     out = Wo concat_a(sigmoid((Wg h)_a) * sum_j p_ij v_a,j)         (one gate number a head)
 
@@ -19,10 +19,11 @@ What runs is the same sum reordered so that the cache is read as it is stored: q
 meets the cached rows [c | rot(kr)] directly - attention of H query heads over ONE key head whose values are the
 first kv_rank elements of the key rows; sum_j p_ij v_a,j = Wuv_a (sum_j p_ij c_j) brings a head's result back
 from the latent, and the head's gate, a number, is applied to the latent sum (an element's gate behind Wuv).  Steps of many tokens
-turn it round where that takes fewer operations: the latents that the step's tokens see are gathered once, k_a and v_a are made of them
+turn it round (bfloat16, widths of 128 + 64 and 128): the latents that the step's tokens see are gathered once, k_a and v_a are made of them
 (two products over the latents), and the heads meet keys of hd + rd and values of vd instead of rows of kv_rank + rd
-and kv_rank (128 + 64 and 128 against 576 and 512: 3.4 times fewer).  A position's result does not depend on how its sequence was cut beyond
-bfloat16 rounding of what stands between the products.
+and kv_rank: at kv_rank 512 3.4 times fewer operations a pair of positions, and at any rank on tcgen05 instead of mma.sync.  Which way a position's
+step goes depends on how many tokens the step has and how many they see, so how its sequence was cut and what else is in the step
+reach its result by bfloat16 rounding of what stands between the products.
 
 The cache holds kv_rank + rd numbers a token and layer (``KVNeed(1, kv_rank + rd, window, value_dim=0)``: no value
 pool).  Wdq (or Wq), Wdkv and Wg are one matrix so that one product serves the three.  Wuk is kept head by head transposed
@@ -71,10 +72,15 @@ class LatentAttention(Mixer):
         self.w_in = self.wuq = self.wuk = self.wuk_rows = self.wuv = self.wo = self.q_norm_w = self.kv_norm_w = None
 
     FEW_TOKENS = 64        # up to here a step's per-head products run on the CUDA cores as one launch
-    # From MADE_FROM tokens on keys and values are made of the latents a step sees, if those are at most ROWS_PER_TOKEN times as many as its
-    # tokens (making them is then worth it, and takes no more memory than the widened queries and sums).
-    # 8 layers of width 2,048, two of them latent with 16 heads, prompts of 600 and 1,400 tokens: 2.61 -> 2.11 ms.
-    MADE_FROM, ROWS_PER_TOKEN = 128, 3
+    # Keys and values are made of the latents a step sees from MADE_FROM tokens on (SMALL_RANK_FROM where kv_rank is below 256), if those are at most
+    # ROWS_PER_TOKEN times as many as its tokens.  A layer's forward, us, queries widened / keys made, 16 heads of width 2,048 over as many rows as tokens:
+    # kv_rank 512, 128 tokens 62 / 70, 144 72 / 70, 256 88 / 79, 1,024 255 / 114; 256, 128 tokens 56 / 62, 144 66 / 67, 192 69 / 69, 256 79 / 74;
+    # 64, 128 tokens 52 / 57, 192 65 / 67, 256 73 / 70, 2,048 221 / 126.  5 heads: kv_rank 256, 160 tokens 48 / 52, 64, 192 tokens 45 / 50, 256 tokens
+    # 52 / 53.  Over three times as many rows the gain is larger throughout (512, 1,024 tokens 752 / 131), and so it would be over more: the limit
+    # is for memory.  Made keys and values take up to 3 * 256 numbers a token and head, the widened queries and sums 2 * kv_rank + 64: no more than those from
+    # kv_rank 352 on, up to four times those at 64.  8 layers of width 2,048, two of them latent with 16 heads, prompts of 600 and 1,400 tokens:
+    # 2.61 -> 2.11 ms.
+    MADE_FROM, SMALL_RANK_FROM, ROWS_PER_TOKEN = 144, 256, 3
 
     def param_specs(self) -> Dict[str, ParamSpec]:
         d, H, hd, rd, vd, n = self.d, self.H, self.hd, self.rd, self.vd, self.names
@@ -100,7 +106,8 @@ class LatentAttention(Mixer):
         if w is not None and w.dim() == 2:
             # [H * hd, kv_rank] -> [H, kv_rank, hd]: head a's rows are the weight of the product q_plain_a -> latent
             tensors = dict(tensors, wuk=w.view(self.H, self.hd, self.kv_rank).transpose(1, 2).contiguous())
-            # the widths that the prompt attention with a shared part takes
+            # the widths that the prompt attention with a shared part takes.  (Wuk is then held twice, transposed for the widened queries and as it
+            # is for the keys: 2 H hd kv_rank bytes more a layer, 2 MB with 16 heads over a latent of 512)
             if w.dtype == torch.bfloat16 and (self.hd, self.rd, self.vd) == (128, 64, 128) and self.kv_rank % 8 == 0:
                 self.wuk_rows = w
         super().bind(tensors)
@@ -116,7 +123,9 @@ class LatentAttention(Mixer):
     def _runs(self, q: torch.Tensor, gates: torch.Tensor, step) -> int:
         """Runs of PAGE_SIZE latents that the step's tokens see, if keys and values are to be made of them; else 0."""
         M = q.shape[0]
-        if self.wuk_rows is None or self.wuv.dtype != torch.bfloat16 or q.dtype != torch.bfloat16 or M < self.MADE_FROM or step.is_decode:
+        if self.wuk_rows is None or self.wuv.dtype != torch.bfloat16 or q.dtype != torch.bfloat16 or step.is_decode:
+            return 0
+        if M < self.MADE_FROM or (self.kv_rank < 256 and M < self.SMALL_RANK_FROM):
             return 0
         if q.stride(0) % 8 or q.data_ptr() % 16 or (self.element_gate and (gates.stride(0) % 8 or gates.data_ptr() % 16)):
             return 0

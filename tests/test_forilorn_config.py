@@ -129,3 +129,20 @@ def test_a_rotation_in_place_that_could_overwrite_a_partner_is_refused(what):
     lib = kernels.library()
     rc = lib.rl_latent_query(base, ld, 1, H, hd, rd, positions.data_ptr(), freq.data_ptr(), 4, 0, 1.0, base, ld, lat, 3, None)
     assert rc == -1 and b"in place" in lib.rl_last_error()
+
+
+@pytest.mark.parametrize("rank,tokens,rows,made", [(512, 143, 143, False), (512, 144, 144, True), (256, 144, 384, True), (256, 128, 384, False), (248, 144, 432, False),
+                                                   (64, 255, 510, False), (64, 256, 256, True), (512, 640, 1920, True), (512, 640, 1921, False), (260, 1024, 1024, False)])
+def test_when_keys_and_values_are_made_of_the_latents(rank, tokens, rows, made):
+    """By the step's tokens, what they see, and the latent's width (a width that the products cannot address: never)."""
+    from types import SimpleNamespace
+    from rustyllm_b200 import kernels as K
+    from rustyllm_b200.config.spec import PartSpec
+    from rustyllm_b200.parts.latent import LatentAttention
+    names = {n: n for n in ("dq", "dq_norm", "uq", "dkv", "dkv_norm", "uk", "uv", "o", "g")}
+    layer = LatentAttention(Runtime(torch.device("cpu"), torch.bfloat16), 64, 2, 128, 64, 128, 32, rank, 0.07, 1e-5, PartSpec("none", {"head_dim": 64}), names)
+    layer.bind({n: torch.zeros([sum(x) for x in zip(*[s.shape for s in p.sources])][:1] + list(p.sources[0].shape[1:]), dtype=torch.bfloat16)
+                for n, p in layer.param_specs().items()})
+    step = SimpleNamespace(is_decode=False, q_lens=[tokens], kv_lens_host=[rows])
+    runs = layer._runs(torch.zeros(tokens, 384, dtype=torch.bfloat16), torch.zeros(tokens, 2, dtype=torch.bfloat16), step)
+    assert runs == (K.latent_runs([tokens], [rows], 0) if made else 0)
