@@ -250,7 +250,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  rl_pdl_trigger();
   if (threadIdx.x == 0) {
     fa_mbar_init(fa_smem_u32(q_full), 1);
     for (int i = 0; i < K_STAGES; ++i) { fa_mbar_init(fa_smem_u32(&k_full[i]), 1); fa_mbar_init(fa_smem_u32(&k_empty[i]), 1); }
@@ -273,6 +272,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_smem_u32(tmem_slot)), "r"((uint32_t)SZ::TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // The next kernel may start once this CTA holds its tensor memory: started before, a product's CTA could take columns on this SM, wait
+  // for this grid to end, and keep it from its own
+  __syncthreads();
+  rl_pdl_trigger();
   rl_pdl_wait();       // everything below reads what earlier kernels of the step wrote
   // ---- which sequence and which of its 128-row query tiles.  The grid is (heads, tiles) and
   // blocks start in the order of the grid: with the caller's table the tiles come by falling
