@@ -222,10 +222,6 @@ _SIGNATURES = {
                        _c_void_p],
     "rl_gemm_tc_splits": [_c_int, _c_int, _c_int],
     "rl_gemm_tc_by_pairs": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int],
-    "rl_gemm_tc_qkv_rope_supported": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int],
-    "rl_gemm_tc_qkv_rope": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
-                            _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
-                            _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
     "rl_gemm_tc_qkv_beside": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                             _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
                             _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p],
