@@ -873,6 +873,96 @@ def test_attention_prefill_tc_finds_one_far_key_and_rescales(far, hd):
     assert (ref[far + 1:] - want).abs().max() < 1e-3
 
 
+# ----------------------------------------------------------------------------- prefill attention (tcgen05), two CTAs an SM
+def _plain_attention_f64(q, kp, vp, pt, slots, lens_q, lens_kv, H, G, hd, scale, window=0, keep_first=0, chunk=0, softcap=0.0, sink=False, sinks=None,
+                         gate=None, gate_per_head=False):
+    """Float64 attention of a prompt step over the paged cache, with every option of the tensor-core prompt kernel."""
+    outs, at = [], 0
+    for b, (nq, n) in enumerate(zip(lens_q, lens_kv)):
+        pages = pt[int(slots[b]), :-(-n // PAGE)].long()
+        kb, vb = ((x[pages].transpose(1, 2).reshape(-1, G, hd)[:n].double().repeat_interleave(H // G, dim=1)) for x in (kp, vp))
+        s = torch.einsum("ihd,jhd->hij", q[at:at + nq].view(nq, H, hd).double(), kb) * scale
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        i, j = torch.arange(n - nq, n, device=q.device)[:, None], torch.arange(n, device=q.device)[None]
+        seen = j <= i
+        if window:
+            seen &= (i - j < window) | (j < keep_first)
+        if chunk:
+            seen &= j >= i - i % chunk
+        s = s.masked_fill(~seen, -math.inf)
+        if sink:
+            extra = torch.zeros(H, dtype=torch.float64, device=q.device) if sinks is None else sinks.double()
+            s = torch.cat([s, extra[:, None, None].expand(H, nq, 1)], dim=-1)
+        p = torch.softmax(s, dim=-1)[..., :n]
+        outs.append(torch.einsum("hij,jhd->ihd", p, vb))
+        at += nq
+    out = torch.cat(outs)
+    if gate is not None:
+        out = out * torch.sigmoid(gate.double()).view(out.shape[0], H, -1)
+    return out.reshape(out.shape[0], H * hd)
+
+
+def _more_ctas_than_two_an_sm(H, lens_q):
+    return H * sum(-(-n // K().PREFILL_TC_QTILE) for n in lens_q) > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.parametrize("opts", [{}, {"window": 4096}, {"chunk": 4096}], ids=["plain", "window", "chunk"])
+@pytest.mark.parametrize("far", [0, 63, 64, 127, 128, 191, 192, 300, "stairs"])
+def test_attention_prefill_tc_by_halves_of_a_row_rescales(far, opts):
+    """Heads of 64 in more CTAs than fit the GPU two an SM at once: the form with two threads a row.  A key in either half of a 128-key tile far
+    above the running maximum of all before it, so that both halves' threads must learn of it and rescale their part of the accumulator; "stairs":
+    a higher one in every half tile.  With and without the code for masks (a window and a chunk that hide nothing)."""
+    k = K()
+    H, G, hd, n = 104, 8, 64, 451
+
+    def craft(b, qb, kb, vb):
+        direction = torch.ones(hd) / math.sqrt(hd)
+        qb[:] = (direction * 20.0).to(qb.dtype)
+        kb[:] = (kb.float() * 0.05).to(kb.dtype)
+        for i, pos in enumerate(range(5, n, 64) if far == "stairs" else [far]):
+            kb[pos] = (direction * (3.0 * (i + 1) if far == "stairs" else 14.0)).to(kb.dtype)       # a step: 60 / 8 in the score, 2^10.8
+    case = _attention_case(torch.bfloat16, H, G, hd, [n], [n], seed=6, craft=craft)
+    q, kp, vp, pt, cu, slots, kv_lens, ref = _prefill_inputs(case, [n], [n])
+    assert _more_ctas_than_two_an_sm(H, [n])
+    out = torch.full((n, H * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    k.attention_prefill_tc(q, kp, vp, pt, cu, slots, kv_lens, [n], out, H, G, hd, 1.0 / math.sqrt(hd), **opts)
+    k.check_device_errors()
+    torch.testing.assert_close(out.double().cpu(), ref, **_tol(torch.bfloat16))
+    if far != "stairs":
+        page = int(pt[1, far // PAGE]); v_far = vp[page, :, far % PAGE].double().cpu()
+        assert (ref[far + 1:] - v_far.repeat_interleave(H // G, dim=0).reshape(1, H * hd)).abs().max() < 1e-3
+
+
+@pytest.mark.parametrize("opts", [{}, {"window": 100}, {"window": 200, "keep_first": 70}, {"window": 65, "keep_first": 3, "sink": True}, {"chunk": 96}, {"chunk": 256},
+                                  {"softcap": 5.0}, {"softcap": 20.0, "window": 150, "sink": True}, {"sink": True, "gate": "element"},
+                                  {"sinks": True, "sink": True, "gate": "head"}, {"gate": "head", "window": 129}, {"chunk": 200, "gate": "element"}],
+                         ids=lambda o: "-".join(f"{a}{b}" for a, b in o.items()) or "plain")
+@pytest.mark.parametrize("lens_q,lens_kv", [([200, 37, 300, 1], [200, 130, 700, 260]), ([1400], [1400])])
+def test_attention_prefill_tc_by_halves_of_a_row_with_every_option(lens_q, lens_kv, opts):
+    """The same form with masks, kept first tokens, caps, sinks and gates, against float64: sequences behind what is cached, query tiles that
+    are not whole, rows whose window begins inside a tile's first or second half."""
+    k = K()
+    H, G, hd = 48, 6, 64
+    assert _more_ctas_than_two_an_sm(H, lens_q)
+
+    def craft(b, qb, kb, vb):
+        qb *= 2                              # scores of standard deviation 2: the running maximum moves
+    case = _attention_case(torch.bfloat16, H, G, hd, lens_q, lens_kv, seed=len(lens_q), craft=craft)
+    q, kp, vp, pt, cu, slots, kv_lens, _ = _prefill_inputs(case, lens_q, lens_kv)
+    kw = dict(opts)
+    if kw.get("sinks"):
+        kw["sinks"] = _rand(H, seed=8, scale=2.0)
+    if kw.get("gate"):
+        kw["gate_per_head"] = kw["gate"] == "head"
+        kw["gate"] = _rand(q.shape[0], H if kw["gate_per_head"] else H * hd, dtype=torch.bfloat16, seed=9)
+    out = torch.full((q.shape[0], H * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    k.attention_prefill_tc(q, kp, vp, pt, cu, slots, kv_lens, lens_q, out, H, G, hd, 1.0 / math.sqrt(hd), **kw)
+    k.check_device_errors()
+    ref = _plain_attention_f64(q, kp, vp, pt, slots, lens_q, lens_kv, H, G, hd, 1.0 / math.sqrt(hd), **kw)
+    torch.testing.assert_close(out.double(), ref, **_tol(torch.bfloat16))
+
+
 # ----------------------------------------------------------------------------- attention over thousands of keys
 def _far_key_craft(far, hd, gain=16.0):
     def craft(b, qb, kb, vb):
