@@ -925,18 +925,23 @@ static bool pair_bulk(const void* out, int out_mode, int ldo) {
 }
 
 // Whether the pairs take a product of more than 128 tokens that is not split over K.  us, CTAs alone / pairs:
+// More than one wave of tiles: outputs by the copy engine at any K (2,048 tokens -> 8,192, bf16, K = 256 23.4 / 18.7, 1,024 31.9 / 28.9; into the residual
+// 43.4 / 34.6, 47.0 / 39.9), but float ones, twice the bytes of bf16, from K = 1,024 on (5,000 tokens -> 4,096, K = 512 30.3 / 30.5, 1,024 43.0 / 38.7), and outputs by the
+// warps from 2,048 on (2,048 tokens -> 8,192, gated, K = 1,024 42.0 / 43.1, 2,048 56.5 / 54.2; into rows of 8,191 48.1 / 51.8, 71.3 / 67.0): below, a tile's time is its epilogue's.
 // Not where they need more waves (an odd number of 128-row weight tiles leaves the last pair half empty): bf16 outputs, 20,480 tokens 2,048 -> 64
 // 20.1 / 26.3 (one wave / two), 10,240 tokens 2,048 -> 384 20.1 / 25.2, 12,000 tokens 4,096 -> 260 35.4 / 47.5, 8,192 tokens 2,048 -> 1,152 33.7 / 36.2 (two / three);
-// as many waves: 5,000 tokens -> 1,152 27.3 / 26.0, 8,192 tokens -> 520 27.8 / 25.6, 20,480 tokens -> 200 31.1 / 27.0.
-// More than one wave of tiles: from K = 512 on (float outputs 1,024, outputs by the warps 2,048); below, a tile's time is its
-// epilogue and its start.  bf16, 20,480 tokens -> 200, K = 512 13.2 / 11.0; 2,048 tokens -> 8,192, gated, K = 1,024 42.0 / 43.1, 2,048 56.5 / 54.2; bf16 rows of 8,188,
-// K = 512 25.0 / 31.3, 2,048 56.6 / 53.3; float, 5,000 tokens -> 4,096, K = 512 30.7 / 32.2, 1,024 42.2 / 38.8.
-// One wave, where nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster barriers): three fifths of it and K from 8,192 on.
+// as many waves: 5,000 tokens -> 1,152 27.3 / 26.0, 8,192 tokens -> 520 27.8 / 25.6, 20,480 tokens -> 200 31.1 / 27.0.  With a short K the copy engine's
+// stores outweigh that (K = 512, 13,653 tokens -> 640 17.4 / 15.2, 10,240 tokens into 300 of the residual 18.2 / 14.8).
+// One wave, where nothing hides a tile's start and epilogue, and the pair's start is the longer (two cluster barriers): from K = 8,192 and three fifths of it on,
+// where every form gains (1,500 tokens -> 2,048, residual 50.0 / 46.0, bf16 47.4 / 44.5, gated 50.0 / 48.5; 32 of 74 pairs, 512 tokens -> 4,096 38.9 / 38.8).  Below, forms
+// differ: 1,500 tokens 2,048 -> 2,048, residual 19.1 / 17.3, bf16 16.8 / 16.3, gated 19.8 / 20.4, float 16.2 / 17.2; 300 tokens 4,096 -> 6,144 26.9 / 27.1, 25.8 / 26.2,
+// 27.7 / 28.7, 25.5 / 26.3.
 static bool pairs_pay(int M, int N, int K, int out_mode, bool bulk) {
   const int tiles_m = (M + 255) / 256, tiles = tiles_m * ((N + PAIR_ROWS - 1) / PAIR_ROWS), sms = rl_num_sms(), pairs = sms / 2;
   const int alone = tiles_m * ((N + BLOCK_N_OUT - 1) / BLOCK_N_OUT);
-  if ((tiles + pairs - 1) / pairs > (alone + sms - 1) / sms) return false;
-  const int least = !bulk ? 2048 : out_mode == TC_OUT_F32 ? 1024 : 512;
+  const bool more_waves = (tiles + pairs - 1) / pairs > (alone + sms - 1) / sms;
+  if (more_waves && (!bulk || K >= 1024)) return false;
+  const int least = !bulk ? 2048 : out_mode == TC_OUT_F32 ? 1024 : 0;
   return tiles > pairs ? K >= least : K >= 8192 && tiles * 5 >= pairs * 3;
 }
 

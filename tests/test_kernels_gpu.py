@@ -1388,14 +1388,14 @@ def test_gemm_tc_persistent_tiles_of_full_height(M):
     k.check_device_errors()
 
 
-@pytest.mark.parametrize("M,N,K_,by_pairs", [(129, 150 * 128 + 2, 8, ""), (300, 75 * 256 - 130, 1032, ""), (301, 75 * 256 - 136, 264, ""), (256, 75 * 256, 640, "as"),
+@pytest.mark.parametrize("M,N,K_,by_pairs", [(129, 150 * 128 + 2, 8, ""), (300, 75 * 256 - 130, 1032, ""), (301, 75 * 256 - 136, 264, "as"), (256, 75 * 256, 640, "as"),
                                              (777, 26 * 256 + 8, 2056, "afsg"), (1025, 2303, 8200, "afs"), (300, 75 * 256 - 130, 2056, "afsg"),
-                                             (301, 74 * 256 + 64, 1024, "afs"), (301, 74 * 256 + 72, 2184, "afsg"), (129, 75 * 256, 512, "as"), (2000, 2048, 520, ""),
-                                             (20000, 248, 520, "as"), (20000, 128, 2048, ""), (5200, 640, 2048, "")])
+                                             (301, 74 * 256 + 64, 1024, "afs"), (301, 74 * 256 + 72, 2184, "afsg"), (129, 75 * 256, 8, "as"), (2000, 2048, 520, ""),
+                                             (20000, 248, 520, "as"), (20000, 128, 2048, ""), (20000, 128, 520, "as"), (5200, 640, 2048, "")])
 def test_gemm_tc_pairs_rings_and_edges(M, N, K_, by_pairs):
     """More tiles of 256 x 256 than pairs of SMs, or more than three fifths and a long K, so pairs of CTAs take them (``by_pairs``: additions into the
-    residual, float, bf16 and gated outputs; the others and those of short K or of more waves by pairs than by CTAs alone go there): the shortest
-    K, rings that go round several times with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave;
+    residual, float, bf16 and gated outputs; the others and those of short K or of more waves by pairs than by CTAs alone go there): a K shorter
+    than a block, rings that go round several times with a ragged last block, weight tiles whose second CTA has no rows or some, narrow tiles of the last wave;
     outputs stored by the copy engine (rows of whole 16-byte pieces) that end inside its pieces of 32 x 32, and by the warps.  Float sums of K
     products; rows behind the last stay as they are."""
     k = K()
