@@ -32,7 +32,7 @@
 // maxima through shared memory; the running maximum stays in their registers.  With one CTA an SM its eight warps issued in 35 % of the
 // slots and the special-function unit ran 45 % of the time: two warps a scheduler do not cover one another's waits, and nothing
 // ran under a CTA's start and end.  Sixteen warps do better: 32 heads over 8, 8,192 tokens 504 -> 442 us, 4,096 141 -> 130
-// (each form with the code for masks in its loop, see PLAIN).
+// (each form with the code for masks in its loop, see PLAIN; where each form runs: see fa_two_an_sm).
 // Tensor memory: the S buffers, O behind them, P behind O (512 columns at head size 128).
 // A key tile is two cache pages (128 positions).  Warp 0 feeds TMA, warps 1 and 2 issue the two
 // products (a thread each: issuing blocks while the tensor pipe is full, and one thread's waits
@@ -206,7 +206,7 @@ __host__ __device__ constexpr uint32_t fa_idesc(int m, int n, int b_mn) {
 }
 
 // PLAIN: every position up to the query's own is visible and scores are not capped; the code for windows, blocks, kept first tokens and soft caps is then
-// left out of the loop, which is bound by what its warps issue (heads of 64, 8,192 tokens 439 -> 429 us; heads of 128, 4,096 tokens 155 -> 145, 1,000 21.6 -> 20.6).
+// left out of the loop (heads of 64, 8,192 tokens 439 -> 429 us; heads of 128, 4,096 tokens 155 -> 145, 1,000 21.6 -> 20.6).
 template <int HD, int VD, bool PLAIN, bool PAIRED>
 __global__ void __launch_bounds__(FA_THREADS, FaSizes<HD, VD, PAIRED>::CTAS)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -710,13 +710,25 @@ int fa_launch_as(dim3 grid, cudaStream_t stream, Args... args) {
   }
   return RL_OK;
 }
+// Whether a step's attention at heads of 64 runs two CTAs an SM.  us, a CTA an SM / two, 32 heads:
+// Only where they are more than fit the GPU so at once; up to there a CTA with an SM of its own is done sooner: 1,000 tokens (256 CTAs) 17.6 / 20.4, 1,400 (352)
+// 29.3 / 26.1, 2,048 47.7 / 39.1.
+// With a cap from three and a quarter CTAs for every SM on (1,400 tokens 47.4 / 51.7, four prompts of 30 to 900 (448) 47.7 / 56.7, 2,048 tokens (512) 83.5 / 74.8), or
+// where every sequence is one query tile (12 of 100 tokens 22.4 / 16.7): a cap's operations keep a CTA's warps busy by themselves.
+// With a window or a chunk a thread of the pair runs the code for masks over half as many scores a tile with 104 registers, and loses: 4,096 tokens, window of
+// 512 79.5 / 115.9, chunk of 256 50.3 / 52.4, 16 prompts of 200 49.8 / 49.6, 12 of 100 20.1 / 20.9; but not where most rows of a tile are none, which
+// a CTA's start and end are most of (64 prompts of 40 tokens 85.6 / 69.1).
+bool fa_two_an_sm(int num_heads, int num_tiles, int num_seqs, int num_tokens, bool masked, bool capped) {
+  const long long ctas = (long long)num_heads * num_tiles, sms = rl_num_sms();
+  if (ctas <= 2 * sms) return false;
+  if (masked) return num_tokens <= 64LL * num_tiles;
+  return !capped || 4 * ctas > 13 * sms || num_tiles == num_seqs;
+}
+
 template <int HD, int VD, typename... Args>
-int fa_launch(bool plain, dim3 grid, cudaStream_t stream, Args... args) {
+int fa_launch(bool plain, bool two, dim3 grid, cudaStream_t stream, Args... args) {
   if constexpr (HD == 64 && VD == 64) {
-    // Two CTAs an SM from where they are more than fit the GPU so at once.  Up to there a CTA with an SM of its own is done sooner: 32 heads,
-    // 1,000 tokens (256 CTAs) 17.6 us alone, 20.4 two an SM; 1,300 (352) 28.7 and 25.2, 2,000 47.1 and 38.9
-    if ((long long)grid.x * grid.y > 2LL * rl_num_sms())
-      return plain ? fa_launch_as<HD, VD, true, true>(grid, stream, args...) : fa_launch_as<HD, VD, false, true>(grid, stream, args...);
+    if (two) return plain ? fa_launch_as<HD, VD, true, true>(grid, stream, args...) : fa_launch_as<HD, VD, false, true>(grid, stream, args...);
   }
   return plain ? fa_launch_as<HD, VD, true, false>(grid, stream, args...) : fa_launch_as<HD, VD, false, false>(grid, stream, args...);
 }
@@ -730,6 +742,10 @@ extern "C" int rl_attention_prefill_tc_supported_shaped(int num_heads, int num_k
 }
 extern "C" int rl_attention_prefill_tc_supported(int num_heads, int num_kv_heads, int head_dim) {
   return rl_attention_prefill_tc_supported_shaped(num_heads, num_kv_heads, head_dim, head_dim);
+}
+// 1 if a step of num_tokens tokens in num_tiles query tiles of num_seqs sequences runs two CTAs an SM (key and value heads of 64).
+extern "C" int rl_attention_prefill_tc_two_an_sm(int num_heads, int num_tiles, int num_seqs, int num_tokens, int window, int chunk, float softcap) {
+  return fa_two_an_sm(num_heads, num_tiles, num_seqs, num_tokens, window > 0 || chunk > 0, softcap != 0.f);
 }
 
 // Same interface as rl_attention_prefill, with num_tiles = sum over sequences of
@@ -779,9 +795,10 @@ extern "C" int rl_attention_prefill_tc_wide(const void* q, int ldq, const void* 
   if (rc != RL_OK) return rc;
   rc = fa_make_map(&mv, v_pool, pool_rows, value_dim, value_dim, RL_PAGE);
   if (rc != RL_OK) return rc;
-  const bool plain = window == 0 && chunk == 0 && softcap == 0.f;
+  const bool masked = window > 0 || chunk > 0, capped = softcap != 0.f, plain = !masked && !capped;
+  const bool two = fa_two_an_sm(num_heads, num_tiles, num_seqs, num_tokens, masked, capped);
 #define FA_GO(HD, VD)                                                                                                          \
-  fa_launch<HD, VD>(plain, dim3(num_heads, num_tiles), stream, mq, mk, mv, page_table, max_pages, cu_seqlens, seq_slots, kv_lens,     \
+  fa_launch<HD, VD>(plain, two, dim3(num_heads, num_tiles), stream, mq, mk, mv, page_table, max_pages, cu_seqlens, seq_slots, kv_lens,     \
                     num_seqs, (__nv_bfloat16*)out, ldo, num_heads, num_kv_heads, scale * 1.4426950408889634f, window, err,      \
                     tile_order, sink, (const __nv_bfloat16*)gate, ldg, cap_in, cap_out, keep_first, chunk, gate_per_head, sinks, mk, 0)
   if (head_dim == 64) return value_dim == 64 ? FA_GO(64, 64) : FA_GO(64, 128);
@@ -821,7 +838,7 @@ extern "C" int rl_attention_prefill_tc_shared_part(const void* q, int ldq, const
   if (rc != RL_OK) return rc;
   rc = fa_make_map(&ms, shared, rows, ld_shared, ld_shared, RL_PAGE);
   if (rc != RL_OK) return rc;
-  return fa_launch<192, 128>(window == 0, dim3(num_heads, num_tiles), stream, mq, mk, mv, run_table, max_runs, cu_seqlens, table_rows, kv_lens, num_seqs,
+  return fa_launch<192, 128>(window == 0, false, dim3(num_heads, num_tiles), stream, mq, mk, mv, run_table, max_runs, cu_seqlens, table_rows, kv_lens, num_seqs,
                              (__nv_bfloat16*)out, ldo, num_heads, num_heads, scale * 1.4426950408889634f, window, err, tile_order, 0,
                              (const __nv_bfloat16*)gate, ldg, 0.f, 0.f, 0, 0, gate_per_head, (const float*)nullptr, ms, shared_col);
 }

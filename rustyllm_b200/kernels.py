@@ -221,6 +221,7 @@ _SIGNATURES = {
                        _c_void_p, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_float, _c_float,
                        _c_void_p],
     "rl_gemm_tc_splits": [_c_int, _c_int, _c_int],
+    "rl_attention_prefill_tc_two_an_sm": [_c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float],
     "rl_gemm_tc_by_pairs": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int],
     "rl_gemm_tc_qkv_beside": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
                             _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
@@ -1953,6 +1954,12 @@ def attention_prefill_tc_supported(dtype: torch.dtype, num_heads: int, num_kv_he
                                    value_dim: Optional[int] = None) -> bool:
     return dtype == torch.bfloat16 and bool(library().rl_attention_prefill_tc_supported_shaped(num_heads, num_kv_heads, head_dim,
                                                                                                head_dim if value_dim is None else value_dim))
+
+
+def attention_prefill_tc_two_an_sm(q_lens, num_heads: int, window: int = 0, chunk: int = 0, softcap: float = 0.0) -> bool:
+    """Whether ``attention_prefill_tc`` runs this step with two CTAs an SM (key and value heads of 64)."""
+    tiles = sum(-(-n // PREFILL_TC_QTILE) for n in q_lens)
+    return bool(library().rl_attention_prefill_tc_two_an_sm(num_heads, tiles, len(q_lens), sum(q_lens), int(window), int(chunk), float(softcap)))
 
 
 def attention_prefill_tc(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, page_table: torch.Tensor,

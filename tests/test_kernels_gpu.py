@@ -903,18 +903,23 @@ def _plain_attention_f64(q, kp, vp, pt, slots, lens_q, lens_kv, H, G, hd, scale,
     return out.reshape(out.shape[0], H * hd)
 
 
-def _more_ctas_than_two_an_sm(H, lens_q):
-    return H * sum(-(-n // K().PREFILL_TC_QTILE) for n in lens_q) > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+def test_attention_prefill_tc_two_an_sm_where_it_pays():
+    """By the CTAs, masks, caps and the rows of a tile."""
+    two = K().attention_prefill_tc_two_an_sm
+    assert [two([n], 32) for n in (1000, 1152, 1153, 4096)] == [False, False, True, True]
+    assert [two([n], 32, softcap=30.0) for n in (1400, 1920, 1921)] == [False, False, True] and two([100] * 12, 32, softcap=30.0)
+    for mask in ({"window": 512}, {"chunk": 256}, {"window": 9, "softcap": 5.0}):
+        assert not two([8192], 32, **mask) and not two([100] * 12, 32, **mask) and two([40] * 64, 32, **mask) and not two([40] * 9, 32, **mask)
 
 
-@pytest.mark.parametrize("opts", [{}, {"window": 4096}, {"chunk": 4096}], ids=["plain", "window", "chunk"])
+@pytest.mark.parametrize("opts", [{}, {"softcap": 1000.0}], ids=["plain", "cap"])
 @pytest.mark.parametrize("far", [0, 63, 64, 127, 128, 191, 192, 300, "stairs"])
 def test_attention_prefill_tc_by_halves_of_a_row_rescales(far, opts):
     """Heads of 64 in more CTAs than fit the GPU two an SM at once: the form with two threads a row.  A key in either half of a 128-key tile far
     above the running maximum of all before it, so that both halves' threads must learn of it and rescale their part of the accumulator; "stairs":
-    a higher one in every half tile.  With and without the code for masks (a window and a chunk that hide nothing)."""
+    a higher one in every half tile.  With and without the code for masks and caps (a cap that moves a score of 35 by 1.4e-2)."""
     k = K()
-    H, G, hd, n = 104, 8, 64, 451
+    H, G, hd, n = 128, 8, 64, 451
 
     def craft(b, qb, kb, vb):
         direction = torch.ones(hd) / math.sqrt(hd)
@@ -924,33 +929,42 @@ def test_attention_prefill_tc_by_halves_of_a_row_rescales(far, opts):
             kb[pos] = (direction * (3.0 * (i + 1) if far == "stairs" else 14.0)).to(kb.dtype)       # a step: 60 / 8 in the score, 2^10.8
     case = _attention_case(torch.bfloat16, H, G, hd, [n], [n], seed=6, craft=craft)
     q, kp, vp, pt, cu, slots, kv_lens, ref = _prefill_inputs(case, [n], [n])
-    assert _more_ctas_than_two_an_sm(H, [n])
+    assert k.attention_prefill_tc_two_an_sm([n], H, **opts)
     out = torch.full((n, H * hd), float("nan"), dtype=torch.bfloat16, device=DEV)
     k.attention_prefill_tc(q, kp, vp, pt, cu, slots, kv_lens, [n], out, H, G, hd, 1.0 / math.sqrt(hd), **opts)
     k.check_device_errors()
+    if opts:
+        ref = _plain_attention_f64(q, kp, vp, pt, slots, [n], [n], H, G, hd, 1.0 / math.sqrt(hd), **opts).cpu()
     torch.testing.assert_close(out.double().cpu(), ref, **_tol(torch.bfloat16))
     if far != "stairs":
         page = int(pt[1, far // PAGE]); v_far = vp[page, :, far % PAGE].double().cpu()
         assert (ref[far + 1:] - v_far.repeat_interleave(H // G, dim=0).reshape(1, H * hd)).abs().max() < 1e-3
 
 
+_SHORT_Q = [1, 64, 33, 17, 2, 48, 63, 50, 128, 1, 40, 5]
+
+
 @pytest.mark.parametrize("opts", [{}, {"window": 100}, {"window": 200, "keep_first": 70}, {"window": 65, "keep_first": 3, "sink": True}, {"chunk": 96}, {"chunk": 256},
                                   {"softcap": 5.0}, {"softcap": 20.0, "window": 150, "sink": True}, {"sink": True, "gate": "element"},
                                   {"sinks": True, "sink": True, "gate": "head"}, {"gate": "head", "window": 129}, {"chunk": 200, "gate": "element"}],
                          ids=lambda o: "-".join(f"{a}{b}" for a, b in o.items()) or "plain")
-@pytest.mark.parametrize("lens_q,lens_kv", [([200, 37, 300, 1], [200, 130, 700, 260]), ([1400], [1400])])
+@pytest.mark.parametrize("lens_q,lens_kv", [([200, 37, 300, 1], [200, 130, 700, 260]), ([1400], [1400]),
+                                            (_SHORT_Q, [n + p for n, p in zip(_SHORT_Q, (700, 0, 95, 300, 128, 64, 1, 500, 260, 63, 127, 191))])],
+                         ids=["portions", "prompt", "short"])
 def test_attention_prefill_tc_by_halves_of_a_row_with_every_option(lens_q, lens_kv, opts):
-    """The same form with masks, kept first tokens, caps, sinks and gates, against float64: sequences behind what is cached, query tiles that
-    are not whole, rows whose window begins inside a tile's first or second half."""
+    """The same form with caps, sinks and gates, and, where its tiles have few rows, with masks and kept first tokens (longer ones: the form with a thread a
+    row, in as many CTAs), against float64: sequences behind what is cached, query tiles that are not whole, rows whose window begins inside a
+    tile's first or second half."""
     k = K()
-    H, G, hd = 48, 6, 64
-    assert _more_ctas_than_two_an_sm(H, lens_q)
+    H, G, hd = 72, 6, 64
 
     def craft(b, qb, kb, vb):
         qb *= 2                              # scores of standard deviation 2: the running maximum moves
     case = _attention_case(torch.bfloat16, H, G, hd, lens_q, lens_kv, seed=len(lens_q), craft=craft)
     q, kp, vp, pt, cu, slots, kv_lens, _ = _prefill_inputs(case, lens_q, lens_kv)
     kw = dict(opts)
+    masked = "window" in kw or "chunk" in kw
+    assert k.attention_prefill_tc_two_an_sm(lens_q, H, **{a: v for a, v in kw.items() if a in ("window", "chunk", "softcap")}) == (not masked or len(lens_q) > 4)
     if kw.get("sinks"):
         kw["sinks"] = _rand(H, seed=8, scale=2.0)
     if kw.get("gate"):
