@@ -714,10 +714,9 @@ int fa_launch_as(dim3 grid, cudaStream_t stream, Args... args) {
 // Only where they are more than fit the GPU so at once; up to there a CTA with an SM of its own is done sooner: 1,000 tokens (256 CTAs) 17.6 / 20.4, 1,400 (352)
 // 29.3 / 26.1, 2,048 47.7 / 39.1.
 // With a cap from three and a quarter CTAs for every SM on (1,400 tokens 47.4 / 51.7, four prompts of 30 to 900 (448) 47.7 / 56.7, 2,048 tokens (512) 83.5 / 74.8), or
-// where every sequence is one query tile (12 of 100 tokens 22.4 / 16.7): a cap's operations keep a CTA's warps busy by themselves.
-// With a window or a chunk a thread of the pair runs the code for masks over half as many scores a tile with 104 registers, and loses: 4,096 tokens, window of
-// 512 79.5 / 115.9, chunk of 256 50.3 / 52.4, 16 prompts of 200 49.8 / 49.6, 12 of 100 20.1 / 20.9; but not where most rows of a tile are none, which
-// a CTA's start and end are most of (64 prompts of 40 tokens 85.6 / 69.1).
+// where every sequence is one query tile (12 of 100 tokens 22.4 / 16.7).
+// With a window or a chunk they lose: 4,096 tokens, window of 512 79.5 / 115.9, chunk of 256 50.3 / 52.4, 16 prompts of 200 49.8 / 49.6, 12 of 100 20.1 / 20.9;
+// but not in tiles with few rows, whose CTAs are mostly start and end (64 prompts of 40 tokens 85.6 / 69.1).
 bool fa_two_an_sm(int num_heads, int num_tiles, int num_seqs, int num_tokens, bool masked, bool capped) {
   const long long ctas = (long long)num_heads * num_tiles, sms = rl_num_sms();
   if (ctas <= 2 * sms) return false;

@@ -674,11 +674,10 @@ static int launch_tc_persistent(const CUtensorMap& mw, const CUtensorMap& ma, co
 // ------------------------------------------------------------------ persistent variant by pairs of CTAs
 // Two CTAs on neighbouring SMs (a cluster of two) hold one tile of 256 weight rows: tcgen05.mma with cta_group::2, M = 256,
 // each CTA staging its own 128 weight rows and half of the tile's tokens, each with its 128 rows of the accumulator in its own
-// tensor memory.  What bounds the kernel above is what its SMs pull out of L2 and what the tensor cores read out of shared memory: a CTA
-// alone fetches 48 KB for a block of K of 128 x 256 outputs, a CTA of a pair 32 KB.  One B200, us, CTAs alone / pairs: 2,048 tokens,
-// 4,096 -> 28,672 with SwiGLU 358 / 346 (1.39 PFLOP/s, the power cap), 4,096 -> 6,144 82 / 76, 4,096 -> 4,096 added into the residual
-// 67.7 / 57.0, 14,336 -> 4,096 204 / 190; 5,514 tokens, 2,048 -> 16,384 285 / 276, 8,192 -> 2,048 179 / 167; 293 tokens, 4,096 -> 28,672
-// 90.9 / 86.2.  Roles, the two accumulators and the narrow tiles of the last wave are as above; the leader's (rank 0)
+// tensor memory.  A CTA alone fetches 48 KB for a block of K of 128 x 256 outputs and its tensor cores read as much out of shared memory, a CTA of a pair
+// 32 KB.  One B200, us, CTAs alone / pairs: 2,048 tokens, 4,096 -> 28,672 with SwiGLU 349 / 332 (1.45 PFLOP/s, the power cap), 4,096 -> 6,144 81.2 / 75.4,
+// 4,096 -> 4,096 added into the residual 62.5 / 54.1, 14,336 -> 4,096 191 / 172; 5,514 tokens, 8,192 -> 2,048 175 / 158.  Which products go here: see
+// pairs_pay.  Roles, the two accumulators and the narrow tiles of the last wave are as above; the leader's (rank 0)
 // issuing thread works for both CTAs, both producers' loads arrive at the leader's barriers, and a commit arrives in both CTAs.
 static constexpr int PAIR_ROWS = 2 * BLOCK_N_OUT;
 static constexpr int PAIR_MAX_STAGES = 10;
